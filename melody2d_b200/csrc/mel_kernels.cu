@@ -325,6 +325,105 @@ __device__ __forceinline__ void warp_scatter(const mel_dev& d, int n0, int node,
     }
 }
 
+// scatter of up to 32 (node, force) pairs, one per lane, in lane order: pair by pair over the node's
+// supports, four pairs' support loads in flight at once.  A pair whose force is zero is passed over:
+// its terms are +-0, and an accumulator that started at +0 is never -0, so adding them changes nothing
+// (open contact elements, and the two outer master nodes of linear borders, are such pairs).
+__device__ __forceinline__ void scatter_pairs(const mel_dev& d, int n0, int node, double fx, double fy, double2* acc, int lane)
+{
+    const bool on = !(fx == 0. && fy == 0.);
+    int a = 0, cnt = 0;
+    if (on) { a = d.sup_ptr[n0 + node]; cnt = d.sup_ptr[n0 + node + 1] - a; }
+    unsigned m = __ballot_sync(0xffffffffu, on);
+    while (m) {
+        int pa[4], pc[4], t[4];
+        double px[4], py[4], N[4];
+#pragma unroll
+        for (int u = 0; u < 4; u++) {
+            const int s = m ? __ffs(m) - 1 : 0;
+            const int c = __shfl_sync(0xffffffffu, cnt, s);
+            pc[u] = m ? c : 0;
+            pa[u] = __shfl_sync(0xffffffffu, a, s);
+            px[u] = __shfl_sync(0xffffffffu, fx, s);
+            py[u] = __shfl_sync(0xffffffffu, fy, s);
+            m &= m - 1;
+            t[u] = 0; N[u] = 0.;
+            if (lane < pc[u]) { t[u] = d.sup_idx[pa[u] + lane]; N[u] = d.sup_N[pa[u] + lane]; }
+        }
+#pragma unroll
+        for (int u = 0; u < 4; u++) {
+            if (lane < pc[u]) {
+                double2 f = acc[t[u]];
+                f.x = f.x + px[u] * N[u];
+                f.y = f.y + py[u] * N[u];
+                acc[t[u]] = f;
+            }
+            for (int j = lane + 32; j < pc[u]; j += 32) {
+                const double Nj = d.sup_N[pa[u] + j];
+                const int tj = d.sup_idx[pa[u] + j];
+                double2 f = acc[tj];
+                f.x = f.x + px[u] * Nj;
+                f.y = f.y + py[u] * Nj;
+                acc[tj] = f;
+            }
+            __syncwarp();
+        }
+    }
+}
+
+// contact forces of deformable body b (Body::Update_contact_forces and Send_contact_forces,
+// Code/Body.h:1642-1967): its own contacts in list order, then those of its incoming ranges in send
+// order, by one warp.  A serial walk is bound by its chain of dependent loads (contact, support
+// range, supports: about 2 us a pair, and a body in a compressed sample has 20 contacts of its own
+// and as many incoming ones with four master nodes each, so that this warp outlasted the
+// Gauss-point pass).  Here the lanes read 32 pairs at a time and only the pairs that carry
+// force are walked.
+__device__ void contact_scatter(const mel_dev& d, int b, int n0, double2* acc, int lane)
+{
+    const int mb = d.b_mat[b];
+    const int c1 = d.b_cont0[b + 1];
+    for (int base = d.b_cont0[b]; base < c1; base += 32) {
+        int node = 0;
+        double fx = 0., fy = 0.;
+        if (base + lane < c1) {
+            const mel_contact* ct = d.cont + base + lane;
+            if (d.table[mb * d.nmat + d.b_mat[ct->bodyM]] > -1) { node = ct->nodeS; fx = ct->fx; fy = ct->fy; }
+        }
+        scatter_pairs(d, n0, node, fx, fy, acc, lane);
+    }
+    const int r1 = d.b_inc0[b + 1];
+    for (int r = d.b_inc0[b]; r < r1; r += 32) {
+        // 32 ranges as one concatenated list, eight contacts (32 master nodes) of it at a time
+        const int2 rg = r + lane < r1 ? d.inc_rng[r + lane] : make_int2(0, 0);
+        const int len = rg.y - rg.x;
+        int incl = len;
+        for (int o = 1; o < 32; o <<= 1) {
+            const int t = __shfl_up_sync(0xffffffffu, incl, o);
+            if (lane >= o) incl += t;
+        }
+        const int total = __shfl_sync(0xffffffffu, incl, 31);
+        for (int tb = 0; tb < total; tb += 8) {
+            const int t = tb + (lane >> 2), k = lane & 3;
+            int lo = 0;                        // the range that holds item t: the first with incl > t
+            for (int step = 16; step > 0; step >>= 1)
+                if (__shfl_sync(0xffffffffu, incl, lo + step - 1) <= t) lo += step;
+            const int c = __shfl_sync(0xffffffffu, rg.y - incl, lo & 31) + t;
+            int node = 0;
+            double fx = 0., fy = 0.;
+            if (t < total) {
+                const mel_contact* ct = d.cont + c;
+                if (d.table[d.b_mat[ct->bodyS] * d.nmat + mb] > -1) {
+                    const double sk = ct->shapeM[k];
+                    node = ct->nodeM[k];
+                    fx = -ct->fx * sk;
+                    fy = -ct->fy * sk;
+                }
+            }
+            scatter_pairs(d, n0, node, fx, fy, acc, lane);
+        }
+    }
+}
+
 // ---- bulk copies into shared memory and their mbarriers (PTX: mbarrier.*, cp.async.bulk) --
 __device__ __forceinline__ unsigned smem_u32(const void* p) { return (unsigned)__cvta_generic_to_shared(p); }
 __device__ __forceinline__ void mbar_init(uint64_t* bar, unsigned count)
@@ -798,28 +897,8 @@ __device__ void deformable_body(const mel_dev& d, int b, double T, double T0, ch
             if (tid == 0 && *s_abort)   // give the copies still in flight a bounded time to land
                 for (int c = k; c < issued; c++) mbar_wait_bounded(&s_bar[c & 1], (unsigned)((c >> 1) & 1));
         } else {
-            // ---- contact forces (warp 7): slave scatter in list order, then master scatter in send
-            // order (Body::Update_contact_forces, Code/Body.h:1642-1900) ---------------------------
-            for (int c = d.b_cont0[b]; c < d.b_cont0[b + 1]; c++) {
-                const mel_contact* ct = d.cont + c;
-                if (d.table[d.b_mat[b] * d.nmat + d.b_mat[ct->bodyM]] <= -1) continue;
-                double Fsx = ct->fx, Fsy = ct->fy;
-                warp_scatter(d, n0, ct->nodeS, Fsx, Fsy, s_fc, lane);
-                __syncwarp();
-            }
-            for (int r = d.b_inc0[b]; r < d.b_inc0[b + 1]; r++) {
-                int2 rg = d.inc_rng[r];
-                for (int c = rg.x; c < rg.y; c++) {
-                    const mel_contact* ct = d.cont + c;
-                    if (d.table[d.b_mat[ct->bodyS] * d.nmat + d.b_mat[b]] <= -1) continue;
-                    double Fsx = ct->fx, Fsy = ct->fy;
-                    for (int k = 0; k < 4; k++) {
-                        double sk = ct->shapeM[k];
-                        warp_scatter(d, n0, ct->nodeM[k], -Fsx * sk, -Fsy * sk, s_fc, lane);
-                        __syncwarp();
-                    }
-                }
-            }
+            // ---- contact forces (warp 7, meanwhile) --------------------------------------------
+            contact_scatter(d, b, n0, s_fc, lane);
         }
         __syncthreads();
         if (*s_abort) return;
@@ -1280,6 +1359,7 @@ __device__ void deformable_body(const mel_dev& d, int b, double T, double T0, ch
 // body kernel: rigid path
 // ------------------------------------------------------------------------------------------
 #define MEL_RIGID_BATCH 512   // border entries whose terms are staged at once (6 doubles each)
+#define MEL_RIGID_STAGE (2 * MEL_RIGID_BATCH)   // contacts whose terms are staged at once (3 doubles each)
 
 template <bool AD>
 __device__ void rigid_body(const mel_dev& d, int b, double T, double T0, char* smem)
@@ -1334,18 +1414,53 @@ __device__ void rigid_body(const mel_dev& d, int b, double T, double T0, char* s
         }
     }
     // ---- contact forces: own contacts in list order (Code/Body.h:1866-1877), then the incoming
-    // ranges in send order; lanes 8..10 of warp 0 each carry one of the three sums -------------
-    if (tid >= 8 && tid < 11) {
-        const int k = tid - 8;
-        double con = 0.;
-        int c0 = d.b_cont0[b], c1 = d.b_cont0[b + 1];
-        con = ordered_sum(con, d.cont_rt + 6 * (size_t)c0 + k, c1 - c0, 6);
-        for (int r = d.b_inc0[b]; r < d.b_inc0[b + 1]; r++) {
-            int2 rr = d.inc_rng[r];
-            con = ordered_sum(con, d.cont_rt + 6 * (size_t)rr.x + 3 + k, rr.y - rr.x, 6);
+    // ranges in send order.  The CTA stages the terms in that order, MEL_RIGID_STAGE contacts at a
+    // time, and lanes 8..10 of warp 0 each add up one of the three sums: a wall has some fifty
+    // incoming ranges of a few contacts, and a lane that walks them itself pays two dependent
+    // loads from memory for each ---------------------------------------------------------------
+    double con = 0.;
+    const int kcon = tid - 8;
+    {
+        const int c0 = d.b_cont0[b], nown = d.b_cont0[b + 1] - c0;
+        for (int w0 = 0; w0 < nown; w0 += MEL_RIGID_STAGE) {
+            const int m = min(MEL_RIGID_STAGE, nown - w0);
+            for (int i = tid; i < m; i += blockDim.x)
+                for (int k = 0; k < 3; k++) sT[k * MEL_RIGID_STAGE + i] = d.cont_rt[6 * (size_t)(c0 + w0 + i) + k];
+            __syncthreads();
+            if (kcon >= 0 && kcon < 3) con = ordered_sum(con, sT + kcon * MEL_RIGID_STAGE, m, 1);
+            __syncthreads();
         }
-        sh[24 + 6 + k] = con;
+        int* s_wsum = reinterpret_cast<int*>(sh + 40);          // per-warp totals of the range lengths
+        const int lane = tid & 31, warp = tid >> 5;
+        const int r1 = d.b_inc0[b + 1];
+        for (int r = d.b_inc0[b]; r < r1; r += blockDim.x) {
+            const int2 rg = r + tid < r1 ? d.inc_rng[r + tid] : make_int2(0, 0);
+            const int len = rg.y - rg.x;
+            int incl = len;
+            for (int o = 1; o < 32; o <<= 1) {
+                const int t = __shfl_up_sync(0xffffffffu, incl, o);
+                if (lane >= o) incl += t;
+            }
+            if (lane == 31) s_wsum[warp] = incl;
+            __syncthreads();
+            int at = incl - len, total = 0;
+            for (int w = 0; w < MEL_BODY_THREADS / 32; w++) {
+                if (w < warp) at += s_wsum[w];
+                total += s_wsum[w];
+            }
+            for (int w0 = 0; w0 < total; w0 += MEL_RIGID_STAGE) {
+                const int i1 = min(len, w0 + MEL_RIGID_STAGE - at);
+                for (int i = max(0, w0 - at); i < i1; i++)
+                    for (int k = 0; k < 3; k++)
+                        sT[k * MEL_RIGID_STAGE + at + i - w0] = d.cont_rt[6 * (size_t)(rg.x + i) + 3 + k];
+                __syncthreads();
+                if (kcon >= 0 && kcon < 3) con = ordered_sum(con, sT + kcon * MEL_RIGID_STAGE, min(MEL_RIGID_STAGE, total - w0), 1);
+                __syncthreads();
+            }
+            __syncthreads();
+        }
     }
+    if (kcon >= 0 && kcon < 3) sh[24 + 6 + kcon] = con;
     if (tid < 6) sh[24 + tid] = acc;
     __syncthreads();
     if (tid == 0) {
