@@ -1,15 +1,15 @@
-"""Autotuner of the body kernel's chunk size: for each workload class (precision, largest deformable
-body) it times the body kernel at every candidate chunk entry cap on a small sample of that class
-(CUDA events on the solver's stream, mel_get_kernel_times) and writes the fastest cap to a tuning
+"""Autotuner of the body kernel's tile size: for each workload class (precision, largest deformable
+body) it times the body kernel at every candidate number of slots per tile on a small sample of that
+class (CUDA events on the solver's stream, mel_get_kernel_times) and writes the fastest to a tuning
 table that mel_create reads (environment variable MELGPU_TUNE_FILE; melody2d_b200.solver points it at
-melody2d_b200/tuning.txt when that file exists and the variable is unset).
+melody2d_b200/tuning.txt when that file exists and the variable is unset).  A class the table does
+not name takes the largest tile that leaves two CTAs per SM.
 
     python -m melody2d_b200.autotune [--out melody2d_b200/tuning.txt] [--discs 300] [--steps 30]
 
 Classes: the 2000-disc workload's discs (64 border + 340 interior nodes) and the largest grains of
 the batched workload (96 border + 480 interior nodes), each in FP64 and in mixed precision.  The
-chunk cap trades the bytes in flight per SM (larger images) against the number of CTAs that fit an
-SM and the per-chunk pipeline overhead; the table lines are "precision max_body_nodes cap"."""
+tile size trades the points that share a barrier against the number of CTAs that fit an SM."""
 from __future__ import annotations
 
 import argparse
@@ -20,13 +20,13 @@ import time
 
 HERE = os.path.dirname(os.path.abspath(__file__))
 DEFAULT_TABLE = os.path.join(HERE, "tuning.txt")
-CAPS = [2048, 1792, 1536, 1408, 1280, 1152, 1024, 896, 768]
-CAPS_MIXED = [3584, 3328, 3072, 2816, 2560, 2304] + CAPS   # FP32 images: larger chunks fit the same memory
+CAPS = [3840, 3584, 3328, 3072, 2816, 2560, 2304, 2048]
+CAPS_MIXED = [5120, 4608, 4096]           # 4096 slots hold any point; above 5120 only the points count
 CLASSES = [(64, 340), (96, 480)]          # (border nodes, interior nodes) of the class's discs
 
 
 def time_cap(flat, precision: int, cap: int, steps: int, warmup: int = 5) -> float:
-    """Body-kernel milliseconds per step at chunk cap `cap` (CUDA events)."""
+    """Body-kernel milliseconds per step with tiles of `cap` slots (CUDA events)."""
     from melody2d_b200.solver import Solver
     os.environ["MELGPU_CHUNK_CAP"] = str(cap)
     try:
@@ -57,7 +57,7 @@ def tune(out: str, discs: int, steps: int, workers: int) -> dict:
                            "body_ms": {str(k): round(v, 5) for k, v in times.items()}, "generate_s": round(gen_s, 1)})
             print(json.dumps(report[-1]), flush=True)
     with open(out, "w") as fh:
-        fh.write("# chunk entry cap per (precision 0 fp64 / 1 mixed, largest deformable body in nodes), written by\n"
+        fh.write("# slots per tile (precision 0 fp64 / 1 mixed, largest deformable body in nodes), written by\n"
                  "# python -m melody2d_b200.autotune (body-kernel time on a %d-disc sample of each class)\n" % discs)
         for p, n, c in rows:
             fh.write("%d %d %d\n" % (p, n, c))

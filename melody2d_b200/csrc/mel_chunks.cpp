@@ -77,12 +77,7 @@ int table_rows(const int* ns, int n)
 
 }  // namespace
 
-long long mel_body_entries(const mel_model_desc* d, int b)
-{
-    return (long long)d->gp_sup_ptr[d->body_gp_ptr[b + 1]] - d->gp_sup_ptr[d->body_gp_ptr[b]];
-}
-
-mel_status mel_build_chunks(const mel_model_desc* d, int ecap, mel_chunk_set& out, bool mixed, long long pipe_min_entries)
+mel_status mel_build_chunks(const mel_model_desc* d, int ecap, mel_chunk_set& out, bool mixed, long long, int min_nodes)
 {
     const int nb = d->n_bodies;
     out.b_pipe.assign(nb, 0);
@@ -98,15 +93,14 @@ mel_status mel_build_chunks(const mel_model_desc* d, int ecap, mel_chunk_set& ou
         out.b_chunk0[b] = (int)out.chunks.size();
         if (d->body_type[b] != MEL_BODY_DEFORMABLE) continue;
         const int nnb = d->body_node_ptr[b + 1] - d->body_node_ptr[b];
+        if (nnb <= min_nodes) continue;
         if (nnb > MEL_MAX_WIDE_NODES) { mel_set_error("deformable body %d has %d nodes (16-bit node indices: at most %d)", b, nnb, MEL_MAX_WIDE_NODES); return MEL_ERR_UNSUPPORTED; }
         // a body above MEL_MAX_BODY_NODES nodes: its FP64 pull slots name their node in a 16-bit
-        // section (the records hold 12 bits), and it never runs the mixed pipeline
+        // section (the records hold 12 bits)
         const int wide = nnb > MEL_MAX_BODY_NODES ? 1 : 0;
         int g = d->body_gp_ptr[b];
         const int g1 = d->body_gp_ptr[b + 1];
-        const bool pipe = mixed && !wide && mel_body_entries(d, b) >= pipe_min_entries;
-        out.b_pipe[b] = pipe ? 1 : 0;
-        const int gpcap = pipe ? MEL_CHUNK_GP_MX : MEL_CHUNK_GP_FP64;
+        const int gpcap = MEL_CHUNK_GP_FP64;
         while (g < g1) {
             // as many points as fit gpcap slots (one point thread each), ecap entries and the 10-bit
             // row tables
@@ -145,8 +139,8 @@ mel_status mel_build_chunks(const mel_model_desc* d, int ecap, mel_chunk_set& ou
                 }
             }
             std::sort(tp.begin(), tp.end());
-            if (mixed && !pipe) {
-                // pull of the mixed two-buffer loop: the entries in (node, point) order with their
+            if (mixed) {
+                // pull of the mixed form: the entries in (node, point) order with their
                 // stored positions, cut into pieces of at most MEL_PIECE entries of one node, and the
                 // seven pull warps' ranges of pieces cut at node boundaries (every node belongs to
                 // one warp), balanced by entries
@@ -260,8 +254,7 @@ mel_status mel_build_chunks(const mel_model_desc* d, int ecap, mel_chunk_set& ou
                 mel_set_error("chunk row tables too large (%d rows)", nroff);
                 return MEL_ERR_UNSUPPORTED;
             }
-            const int wsec = (wide && !mixed) ? 1 : 0;     // the mixed pipeline is off for wide bodies
-            const mel_chunk_layout L = mel_chunk_sections(ch.ngp, ch.ne, ch.ntn, nroff, mixed ? 8 : 16, wsec);
+            const mel_chunk_layout L = mel_chunk_sections(ch.ngp, ch.ne, ch.ntn, nroff, 16, wide);
             ch.bytes = L.bytes;
             ch.img = (long long)out.img.size();
             out.img.resize(out.img.size() + L.bytes, 0);
@@ -269,7 +262,6 @@ mel_status mel_build_chunks(const mel_model_desc* d, int ecap, mel_chunk_set& ou
             int hdr[4] = { ch.ngp, ch.ne, ch.ntn, nroff };
             memcpy(I, hdr, sizeof hdr);
             double* dN = reinterpret_cast<double*>(I + L.dN);
-            float* dNf = reinterpret_cast<float*>(I + L.dN);
             uint16_t* idx = reinterpret_cast<uint16_t*>(I + L.idx);
             uint16_t* tpos = reinterpret_cast<uint16_t*>(I + L.tpos);
             double* c0 = reinterpret_cast<double*>(I + L.c0);
@@ -284,13 +276,13 @@ mel_status mel_build_chunks(const mel_model_desc* d, int ecap, mel_chunk_set& ou
                 for (int k = 0, j = d->gp_sup_ptr[gg]; k < c; k++, j++) {
                     int e = P.pos(slot, k);
                     idx[e] = (uint16_t)d->gp_sup_idx[j];
-                    if (mixed) { dNf[2 * e] = (float)d->gp_dNdx[j]; dNf[2 * e + 1] = (float)d->gp_dNdy[j]; }
-                    else { dN[2 * e] = d->gp_dNdx[j]; dN[2 * e + 1] = d->gp_dNdy[j]; }
+                    dN[2 * e] = d->gp_dNdx[j];
+                    dN[2 * e + 1] = d->gp_dNdy[j];
                 }
             }
             for (int q = 0; q < P.entries; q++) tpos[q] = tposv[q];
             memcpy(tnr, tn.data(), sizeof(uint32_t) * tn.size());
-            if (wsec) memcpy(I + L.tnode, tnv.data(), sizeof(uint16_t) * tnv.size());
+            if (wide) memcpy(I + L.tnode, tnv.data(), sizeof(uint16_t) * tnv.size());
             for (int r = 0; r < nroff; r++) roff[r] = (uint16_t)(roff_all[r] | (rsw_all[r] << 12));
             out.img_max = std::max(out.img_max, ch.bytes);
             out.n_entries += ch.ne;

@@ -1,4 +1,5 @@
-// Host builder of the Gauss-point chunk images read by the body kernel (layout in mel_internal.h).
+// Host builder of the Gauss-point chunk images that the body kernel reads for bodies above
+// MEL_MAX_BODY_NODES nodes (layout in mel_internal.h; the others have tiles, mel_tiles.h).
 #pragma once
 #include <cstdint>
 #include <vector>
@@ -11,15 +12,12 @@ struct mel_chunk_set {
     int img_max = 16;              // largest image (bytes)
     long long n_entries = 0;       // stored entries, padding included
     long long n_pad = 0;           // padding entries (rounding of each chunk to 8 entries)
-    std::vector<int> b_pipe;       // [n_bodies] 1: the body runs the three-stage pipeline (mixed only)
+    std::vector<int> b_pipe;       // [n_bodies] zeros: every body's images are those of the two-buffer loop
 };
 
-// Cuts every deformable body's Gauss points into chunks of at most `ecap` entries and at most
-// MEL_CHUNK_GP_FP64 points, or MEL_CHUNK_GP_MX points for a body that runs the mixed pass's
-// three-stage pipeline (its point threads are fewer).  mixed: dN pairs stored as FP32 instead of
-// FP64; a mixed body runs the pipeline when it has at least pipe_min_entries support entries
-// (out.b_pipe).  Returns MEL_OK or an error code with the message set.
-mel_status mel_build_chunks(const mel_model_desc* d, int ecap, mel_chunk_set& out, bool mixed = false,
-                            long long pipe_min_entries = 0);
-// support entries of deformable body b
-long long mel_body_entries(const mel_model_desc* d, int b);
+// Cuts the Gauss points of every deformable body of more than min_nodes nodes into chunks of at most
+// `ecap` entries and at most MEL_CHUNK_GP_FP64 points.  mixed: dN pairs stored as FP32 instead of
+// FP64, and pieces instead of pull slots (the number after it is not used).  Returns MEL_OK or an
+// error code with the message set.
+mel_status mel_build_chunks(const mel_model_desc* d, int ecap, mel_chunk_set& out, bool mixed = false, long long = 0,
+                            int min_nodes = 0);

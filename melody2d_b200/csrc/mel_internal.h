@@ -1,34 +1,31 @@
 // Internal definitions of the B200 solver: device-resident model and kernel entry points.
 // Layout (HBM): body-sorted structure-of-arrays; node pairs (x,y) as double2 for 16-byte
-// accesses; the Gauss points of a deformable body cut into chunks, each chunk one contiguous
-// 16-byte-aligned image (header, dN/dx-dN/dy pairs, 16-bit body-local support indices, pull
-// positions, per-point weights and offsets, touched-node records) that a single bulk copy
-// moves into shared memory; contact elements in the reference's mel_contact record.
+// accesses; the Gauss points of a deformable body cut into tiles (mel_tiles.h) that the body kernel
+// reads straight into registers, or, for bodies above MEL_MAX_BODY_NODES nodes, into chunks, each
+// chunk one contiguous 16-byte-aligned image (header, dN/dx-dN/dy pairs, 16-bit body-local support
+// indices, pull positions, per-point weights and offsets, touched-node records) that a single bulk
+// copy moves into shared memory; contact elements in the reference's mel_contact record.
 #pragma once
 
 #include <cstdint>
 #include <cuda_runtime.h>
 #include "melgpu.h"
 
-#define MEL_BODY_THREADS 256      // threads per body CTA: point warps, pull warps, warp 7 (copies, contacts)
-// The FP64 body kernel: warps 0-6 run each chunk's Gauss-point pass and then its pull, over two
-// chunk buffers.  The mixed kernel: a pipeline of point warps, pull warps and a copy warp over a
-// ring of three buffers.
-#define MEL_STAGES(mx) ((mx) ? 3 : 2)     // chunk buffers
-#define MEL_PT_WARPS_MX 4                 // point warps of the mixed pipeline (warps 4-6 pull)
-#define MEL_CHUNK_GP_FP64 224     // Gauss points per chunk: one point thread each
-#define MEL_CHUNK_GP_MX 128
-#define MEL_PULL_WARPS 7          // warps 0-6 of the two-buffer loop: point pass, then pull
+#define MEL_BODY_THREADS 256      // threads per body CTA: warps 0-6 Gauss points and their sums, warp 7 contacts
+#define MEL_TILE_GP 224           // Gauss points per tile (mel_tiles.h): one thread each
+#define MEL_CHUNK_GP_FP64 224     // Gauss points per chunk of a wide body: one point thread each
+#define MEL_PULL_WARPS 7          // warps 0-6 of the chunk loop: point pass, then pull
 #define MEL_PIECE 8               // entries of one node a lane of the mixed pull sums before the warp combines
-// mixed-precision bodies with at least this many support entries run the three-stage pipeline,
-// the others the two-buffer loop.  Measured on B200 (mixed body pass): the pipeline takes 0.537 ms
-// against 0.588 ms on the 2000-disc sample, but a 32-sample batch of the batched workload steps in
-// 3.36 ms with it against 2.02 ms with the loop; so by default no body runs the pipeline
-// (MELGPU_PIPE_MIN_ENTRIES, read by mel_create, sets another threshold)
-#define MEL_PIPE_MIN_ENTRIES (1LL << 62)
-#define MEL_BAR_BYTES 128         // the ring's mbarriers (3 per stage) and the abort flag
-#define MEL_CHUNK_E_MAX 2048      // support entries per chunk, upper bound (the host may choose less)
-#define MEL_CHUNK_E_MAX_MX 3584   // the same for the mixed pass's FP32 images (its caps above 2048 come from the tuning table)
+#define MEL_BAR_BYTES 128         // mbarriers and the abort flag
+#define MEL_PLACES(mixed) ((mixed) ? 16 : 8)      // slots of one shared-memory wavefront (8 or 16 bytes each)
+// head rows: derivative pairs of a point that its thread holds in registers (the rest are tail rows).
+// Measured on B200, body kernel of 700 grains of 384 nodes: FP64 with 16 / 12 / 8 / 4 head rows 237 /
+// 192 / 183 / 190 us (16 spill, few leave less shared memory for slots), mixed with 20 / 16 / 12 / 8
+// 149 / 147 / 146 / 147 us
+#define MEL_TILE_HEAD(mixed) ((mixed) ? 12 : 8)
+#define MEL_TILE_SLOTS 3840       // slots of a tile: 224 points of 15 supports on average, groups padded
+#define MEL_TILE_SLOTS_MAX 8192   // largest the tuning table may name
+#define MEL_CHUNK_E_MAX 2048      // support entries per chunk of a wide body, upper bound
 #define MEL_WAIT_NS 1000000000ull // bound of every device-side wait (1 s)
 #define MEL_NBR_CAP_DEFAULT 64    // neighbour slots per body (grown on overflow)
 #define MEL_MAX_BODY_NODES 4096   // nodes per deformable body held in shared memory
@@ -103,6 +100,23 @@ __host__ __device__ inline mel_chunk_layout mel_chunk_sections(int ngp, int ne, 
     return L;
 }
 
+// One tile of a body's Gauss points (sections: mel_tiles.h), a point's record and a pull slot's.
+// base: offset / 128; rec_idx: bytes / 16 of the head pairs | of the tail pairs and index words << 16;
+// counts: points | touched nodes << 16; pos: bytes / 16 of the position words | of the tail pairs << 16
+struct mel_tile { unsigned base, rec_idx, counts, pos; };
+struct mel_point { double c0; unsigned a, i; };     // weight x jacobian; a: first slot | supports << 16 | largest
+                                                    // of the group << 24; i: first index word | (group
+                                                    // width / 8 - 1) << 14 | slots of tail rows before << 16
+struct mel_pull { unsigned node, p0; };             // node | entries << 16; first position word
+__host__ __device__ inline size_t mel_tile_base(unsigned base) { return (size_t)base * 128; }
+__host__ __device__ inline int mel_tile_o_rec(unsigned rec_idx) { return 16 * (int)(rec_idx & 0xffffu); }
+__host__ __device__ inline int mel_tile_o_idx(unsigned rec_idx, unsigned counts) { return mel_tile_o_rec(rec_idx) + 16 * (int)(counts & 0xffffu); }
+__host__ __device__ inline int mel_tile_idx_bytes(unsigned rec_idx) { return 16 * (int)(rec_idx >> 16); }
+__host__ __device__ inline int mel_tile_o_slot(unsigned rec_idx, unsigned counts) { return mel_tile_o_idx(rec_idx, counts) + mel_tile_idx_bytes(rec_idx); }
+// tail pairs and index words, brought by one copy; so are pull slots and position words
+__host__ __device__ inline int mel_tile_pull_bytes(unsigned counts, unsigned pos) { return ((8 * (int)(counts >> 16) + 15) & ~15) + 16 * (int)(pos & 0xffffu); }
+__host__ __device__ inline int mel_tile_tail_bytes(unsigned pos) { return 16 * (int)(pos >> 16); }
+
 struct mel_dev {
     // sizes
     int nb, nn, nbd, ne, ng, nchunk, ncont, cont_cap;
@@ -167,10 +181,14 @@ struct mel_dev {
     const int* bd_sblk0;                      // [nbd+1] first superblock of each border
     const int* sblk_border;                   // border of each superblock
     double4* seg_sblk;                        // superblock boxes (unions of their block boxes)
-    // Gauss points: chunk table and chunk images
+    // Gauss points: tile table and tiles; chunk table and chunk images of the wide bodies
+    const mel_tile* tile;
+    const int* b_tile0;
+    const char* timg;
+    int tile_cap, tile_q, tile_i;             // slots of a tile; shared-memory bytes of its contributions
+                                              // and of its index words
+    unsigned long long tile_pad;              // four positions that name the zero slot
     const mel_chunk* chunk;
-    const int* b_pipe;                        // per body: 1 = three-stage pipeline (mixed pass), else
-                                              // the two-buffer loop; NULL for FP64
     const char* img;
     int img_cap;                              // bytes of one shared-memory staging buffer
     // contacts
@@ -230,7 +248,9 @@ void mel_launch_rigid_restore(const mel_dev& d, const double* rg_snap, cudaStrea
 // ordered first), then the rest with smem bytes
 void mel_launch_batch_step(const mel_dev* devs, const int* thr0, int nthr, const int* cta0, int ncta_small, int ncta,
                            int nsamp, int mixed, size_t smem_small, size_t smem, cudaStream_t s);
-size_t mel_body_smem_bytes(int max_nodes, int max_image_bytes, int mixed, int stages);
+// shared memory of a body CTA: node arrays of max_nodes nodes beside `stage` bytes of Gauss-point
+// contributions or the post-loop arrays, whichever are larger
+size_t mel_body_smem_bytes(int max_nodes, size_t stage, int mixed);
 void mel_launch_update_borders(const mel_dev& d, cudaStream_t s);
 void mel_launch_monitor(const mel_dev& d, double* part, const int* rigid_ids, int nrigid, double* out, cudaStream_t s);
 // Update_contact_pressures (Code/Proximity.h:1014-1069) from the current contact list

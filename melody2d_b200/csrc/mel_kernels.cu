@@ -309,22 +309,6 @@ __device__ void body_drivendof(const mel_dev& d, int b, double T, double* drv)
 // ------------------------------------------------------------------------------------------
 // body kernel: deformable path
 // ------------------------------------------------------------------------------------------
-// scatter v * N_j onto the supports of body-local node `node` (one warp; lanes over supports)
-__device__ __forceinline__ void warp_scatter(const mel_dev& d, int n0, int node, double fx, double fy, double2* acc, int lane,
-                                             int nlanes = 32)
-{
-    int gn = n0 + node;
-    int a = d.sup_ptr[gn], bnd = d.sup_ptr[gn + 1];
-    for (int j = a + lane; j < bnd; j += nlanes) {
-        double N = d.sup_N[j];
-        int t = d.sup_idx[j];
-        double2 f = acc[t];
-        f.x = f.x + fx * N;
-        f.y = f.y + fy * N;
-        acc[t] = f;
-    }
-}
-
 // scatter of up to 32 (node, force) pairs, one per lane, in lane order: pair by pair over the node's
 // supports, four pairs' support loads in flight at once.  A pair whose force is zero is passed over:
 // its terms are +-0, and an accumulator that started at +0 is never -0, so adding them changes nothing
@@ -452,19 +436,6 @@ __device__ __forceinline__ void fence_proxy_async() { asm volatile("fence.proxy.
 #define MEL_BODY_CTHREADS 224     // the FP64 kernel's Gauss-point warps (0-6); warp 7 scatters contacts
 // barrier of the FP64 kernel's Gauss-point warps only (warp 7 runs the contact scatter meanwhile)
 __device__ __forceinline__ void compute_sync() { asm volatile("bar.sync 1, %0;" :: "n"(MEL_BODY_CTHREADS) : "memory"); }
-__device__ __forceinline__ void mbar_arrive(uint64_t* bar)
-{
-    asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" :: "r"(smem_u32(bar)) : "memory");
-}
-// barrier of the pull warps alone (named barrier 3), returning whether any of them passed `v`
-template <int NT>
-__device__ __forceinline__ bool pull_group_any(bool v)
-{
-    unsigned r;
-    asm volatile("{\n\t.reg .pred p, q;\n\tsetp.ne.u32 p, %1, 0;\n\tbar.red.or.pred q, 3, %2, p;\n\tselp.u32 %0, 1, 0, q;\n}"
-                 : "=r"(r) : "r"((unsigned)v), "n"(NT) : "memory");
-    return r != 0;
-}
 // barrier of warps 1-7 in the body tail (warp 0 sums the works meanwhile)
 __device__ __forceinline__ void tail_sync() { asm volatile("bar.sync 2, %0;" :: "n"(MEL_BODY_THREADS - 32) : "memory"); }
 __device__ __forceinline__ unsigned long long global_ns()
@@ -692,310 +663,132 @@ __device__ __forceinline__ void chunk_points_mx(int t, int ngp, int mtype, float
 
 #undef E
 
-// Shared memory of a deformable body (n nodes, staging buffers of img_cap bytes each; two for the
-// two-buffer loop, MEL_STAGES(1) for the pipeline):
-//   s_up, s_f, s_fc        3 x n double2       displacements, internal forces, contact forces
-//   s_upf (mixed only)     n2 x float2         displacements relative to node 0 (n2 = n rounded to 2)
-//   ring mbarriers + abort flag                MEL_BAR_BYTES
-//   region                 max(MEL_STAGES img_cap, 128 n) bytes: the ring of chunk images during
-//                          the Gauss-point pass, then s_fn, s_fd, s_vp, s_ap (n double2 each), the
-//                          six work terms per node (6 x n double) and, in the first half-step of
-//                          Solver_step, the temporary displacement parameters (n double2)
-template <bool MX, bool AD, bool WIDE>
-__device__ void deformable_body(const mel_dev& d, int b, double T, double T0, char* smem)
+// Internal and contact forces of a body above MEL_MAX_BODY_NODES nodes, whose node arrays live in
+// global memory (s_up read in place; s_f, s_fc, s_upf in its part of gscr): a loop over its chunk
+// images with two shared-memory buffers, chunk k computed while chunk k+1 is copied.  Returns false
+// when a wait gave up.
+template <bool MX>
+__device__ bool chunk_forces(const mel_dev& d, int b, char* smem, const double2* s_up, double2* s_f, double2* s_fc, float2* s_upf)
 {
     const int tid = threadIdx.x;
     const int lane = tid & 31, warp = tid >> 5;
     const int n0 = d.b_node0[b];
     const int n = d.b_node0[b + 1] - n0;
-    const double dt = d.dt[0];
-    // a body above MEL_MAX_BODY_NODES nodes ("wide", its own instantiation so that the others keep
-    // plain shared-memory addressing) keeps its node arrays in global memory: it reads its
-    // displacement parameters in place and accumulates its forces in gscr; shared memory then holds
-    // only the mbarriers and the chunk images
-    constexpr bool wide = WIDE;
-    const long long go = WIDE ? d.b_gscr[b] : 0LL;
-    double2* s_up = wide ? d.up + n0 : reinterpret_cast<double2*>(smem);
-    double2* s_f = wide ? reinterpret_cast<double2*>(d.gscr + go) : s_up + n;
-    double2* s_fc = s_f + n;
-    float2* s_upf = reinterpret_cast<float2*>(s_fc + n);
-    char* const s_after = wide ? smem : (MX ? reinterpret_cast<char*>(s_upf + ((n + 1) & ~1)) : reinterpret_cast<char*>(s_fc + n));
-    // the chunk loop, which leaves the internal forces in s_f and the contact forces in s_fc
-    char* region;
-    volatile int* s_abort;
-    // the mixed pass runs the pipeline on bodies with many chunks and the two-buffer loop on the
-    // others, whose few chunks leave a three-stage pipeline mostly filling and draining
-    const bool pipe = MX && d.b_pipe && d.b_pipe[b];
-    if (!pipe) {
-        uint64_t* s_bar = reinterpret_cast<uint64_t*>(s_after);
-        s_abort = reinterpret_cast<volatile int*>(s_bar + 2);
-        region = reinterpret_cast<char*>(s_bar) + MEL_BAR_BYTES;
-        char* const buf0 = region;
-        char* const buf1 = region + d.img_cap;
-        const int ch0 = d.b_chunk0[b];
-        const int nch = d.b_chunk0[b + 1] - ch0;
+    uint64_t* s_bar = reinterpret_cast<uint64_t*>(smem);
+    volatile int* s_abort = reinterpret_cast<volatile int*>(s_bar + 2);
+    char* const buf0 = reinterpret_cast<char*>(s_bar) + MEL_BAR_BYTES;
+    char* const buf1 = buf0 + d.img_cap;
+    const int ch0 = d.b_chunk0[b];
+    const int nch = d.b_chunk0[b + 1] - ch0;
+    for (int i = tid; i < n; i += blockDim.x) {
+        s_f[i] = make_double2(0., 0.);
+        s_fc[i] = make_double2(0., 0.);
+    }
+    if (MX) {
+        const double2 u0 = d.up[n0];
         for (int i = tid; i < n; i += blockDim.x) {
-            if (!wide) s_up[i] = d.up[n0 + i];
-            s_f[i] = make_double2(0., 0.);
-            s_fc[i] = make_double2(0., 0.);
+            const double2 u = d.up[n0 + i];
+            s_upf[i] = make_float2((float)(u.x - u0.x), (float)(u.y - u0.y));
         }
-        if (MX) {
-            const double2 u0 = d.up[n0];
-            for (int i = tid; i < n; i += blockDim.x) {
-                const double2 u = d.up[n0 + i];
-                s_upf[i] = make_float2((float)(u.x - u0.x), (float)(u.y - u0.y));
-            }
-        }
-        if (tid == 0) {
-            mbar_init(&s_bar[0], 1);
-            mbar_init(&s_bar[1], 1);
-            mbar_init_fence();
-            *s_abort = 0;
-        }
-        __syncthreads();
-        if (warp < MEL_BODY_CTHREADS / 32) {
-            // ---- Update_internal_forces: chunk k is computed while chunk k+1 is in flight ----------
-            const int mat = d.b_mat[b];
-            const int mtype = d.mat_type[mat];
-            const double Mu = d.mat_p[MEL_MAT_NPARAM * mat + 3];
-            const double Lam = d.mat_p[MEL_MAT_NPARAM * mat + 4];
-            int issued = 0;
-            if (tid == 0)
-                for (; issued < 2 && issued < nch; issued++) {
-                    const mel_chunk c = d.chunk[ch0 + issued];
-                    mbar_arrive_expect_tx(&s_bar[issued], (unsigned)c.bytes);
-                    bulk_load(issued ? buf1 : buf0, d.img + c.img, (unsigned)c.bytes, &s_bar[issued]);
-                }
-            int k = 0;
-            for (; k < nch; k++) {
-                const int sel = k & 1;
-                char* bk = sel ? buf1 : buf0;
-                long long nxt_img = 0;
-                int nxt_bytes = 0;
-                if (tid == 0 && k + 2 < nch) { const mel_chunk c = d.chunk[ch0 + k + 2]; nxt_img = c.img; nxt_bytes = c.bytes; }
-                const bool ok = mbar_wait_bounded(&s_bar[sel], (unsigned)((k >> 1) & 1), d.wait_ns);
-                if (!ok) { atomicOr(&d.err[MEL_E_WAIT], 1u); *s_abort = 1; }
-                const int4 hdr = ok ? *reinterpret_cast<const int4*>(bk) : make_int4(0, 0, 0, 0);
-                const mel_chunk_layout L = mel_chunk_sections(hdr.x, hdr.y, hdr.z, hdr.w, MX ? 8 : 16, (!MX && wide) ? 1 : 0);
-                const uint16_t* s_idx = reinterpret_cast<const uint16_t*>(bk + L.idx);
-                const uint16_t* s_tpos = reinterpret_cast<const uint16_t*>(bk + L.tpos);
-                const unsigned* s_tn = reinterpret_cast<const unsigned*>(bk + L.tn);
-                const uint16_t* s_roff = reinterpret_cast<const uint16_t*>(bk + L.roff);
-                if (tid < hdr.x) {
-                    if (MX)
-                        chunk_points_mx(tid, hdr.x, mtype, (float)Mu, (float)Lam, s_upf, reinterpret_cast<float2*>(bk + L.dN), s_idx,
-                                        reinterpret_cast<const double*>(bk + L.c0), reinterpret_cast<const unsigned*>(bk + L.gpm),
-                                        reinterpret_cast<const uint16_t*>(bk + L.roff));
-                    else
-                        chunk_points(tid, hdr.x, mtype, Mu, Lam, s_up, reinterpret_cast<double2*>(bk + L.dN), s_idx,
-                                     reinterpret_cast<const double*>(bk + L.c0), reinterpret_cast<const unsigned*>(bk + L.gpm),
-                                     reinterpret_cast<const uint16_t*>(bk + L.roff));
-                }
-                compute_sync();
-                if (*s_abort) break;
-                if (MX) {
-                    // pull of the mixed form, a two-level segmented reduction in place of the ordered
-                    // chains: each lane sums one piece (at most MEL_PIECE entries of one node) in FP64,
-                    // then the pieces of a node, on consecutive lanes, are combined by a Hillis-Steele
-                    // scan over warp shuffles (equal node keys 2^i lanes apart mean one segment, as
-                    // keys are sorted) and the last lane of each segment subtracts the sum from the
-                    // node.  Warp w owns the pieces [wr[w], wr[w+1]), whole nodes only, balanced by
-                    // entries, so no two warps touch one node.
-                    const float2* s_q = reinterpret_cast<const float2*>(bk + L.dN);
-                    const uint16_t* s_wr = reinterpret_cast<const uint16_t*>(bk + L.tn);
-                    const unsigned* s_pc = reinterpret_cast<const unsigned*>(bk + L.tn + 16);
-                    const int p1 = s_wr[warp + 1];
-                    for (int p0 = s_wr[warp]; p0 < p1; p0 += 32) {
-                        const int pi = p0 + lane;
-                        const bool v = pi < p1;
-                        const unsigned rec = v ? s_pc[pi] : 0u;
-                        const int node = v ? (int)((rec >> 16) & 0xffffu) : -1;
-                        const int q0 = (int)(rec & 0x1fffu), cnt = v ? (int)((rec >> 13) & 7u) + 1 : 0;
-                        float2 c[MEL_PIECE];
-#pragma unroll
-                        for (int i = 0; i < MEL_PIECE; i++) c[i] = i < cnt ? s_q[s_tpos[q0 + i]] : make_float2(0.f, 0.f);
-                        double fx = 0., fy = 0.;
-#pragma unroll
-                        for (int i = 0; i < MEL_PIECE; i++) { fx = fx + (double)c[i].x; fy = fy + (double)c[i].y; }
-#pragma unroll
-                        for (int dd = 1; dd < 32; dd <<= 1) {
-                            const double ox = __shfl_up_sync(0xffffffffu, fx, dd);
-                            const double oy = __shfl_up_sync(0xffffffffu, fy, dd);
-                            const int on = __shfl_up_sync(0xffffffffu, node, dd);
-                            if (lane >= dd && on == node) { fx = fx + ox; fy = fy + oy; }
-                        }
-                        const int nn = __shfl_down_sync(0xffffffffu, node, 1);
-                        if (v && (lane == 31 || nn != node)) {
-                            double2 f = s_f[node];
-                            f.x = f.x - fx;
-                            f.y = f.y - fy;
-                            s_f[node] = f;
-                        }
-                        __syncwarp();     // a node continued by the next round reads this update
-                    }
-                } else {
-                    // pull: each touched node subtracts its contributions in ascending Gauss-point order.
-                    // Pull slot t is lane t & 31 of group t >> 5, its entry j at row j of the group's row
-                    // table.  Groups are sorted by entry count; warp w takes groups w, 13 - w, 14 + w, ...
-                    // (snake order), so the heaviest group has a warp to itself and the lighter ones pair up.
-                    const int ngrp = (hdr.z + 31) >> 5;
-                    for (int i = 0; 7 * i < ngrp; i++) {
-                        const int t = (7 * i + ((i & 1) ? 6 - warp : warp)) * 32 + lane;
-                        if (t >= hdr.z) continue;
-                        const unsigned rec = s_tn[t];
-                        const int node = wide ? (int)reinterpret_cast<const uint16_t*>(bk + L.tnode)[t] : (int)(rec & 0xfffu);
-                        const int cnt = (int)((rec >> 12) & 0xffu);
-                        const uint16_t* prow = s_roff + (rec >> 20);
-                        // rows every slot of a full group has: 32 wide and contiguous
-                        const int pfull = (t | 31) < hdr.z ? (int)((s_tn[t | 31] >> 12) & 0xffu) : 0;
-                        const int pbase = prow[0];
-        #define PQ(j) ((j) < pfull ? pbase + 32 * (j) + lane : prow[(j)] + lane)
-                        double2 f = s_f[node];
-                        int j = 0;
-                        const double2* s_p = reinterpret_cast<const double2*>(bk + L.dN);
-                        for (; j + 8 <= pfull; j += 8) {
-                            double2 c[8];
-#pragma unroll
-                            for (int i = 0; i < 8; i++) c[i] = s_p[s_tpos[pbase + 32 * (j + i) + lane]];
-#pragma unroll
-                            for (int i = 0; i < 8; i++) { f.x = f.x - c[i].x; f.y = f.y - c[i].y; }
-                        }
-                        for (; j + 8 <= cnt; j += 8) {      // remaining rows: row-table loads issued together
-                            int q[8];
-#pragma unroll
-                            for (int i = 0; i < 8; i++) q[i] = PQ(j + i);
-                            double2 c[8];
-#pragma unroll
-                            for (int i = 0; i < 8; i++) c[i] = s_p[s_tpos[q[i]]];
-#pragma unroll
-                            for (int i = 0; i < 8; i++) { f.x = f.x - c[i].x; f.y = f.y - c[i].y; }
-                        }
-                        for (; j + 4 <= cnt; j += 4) {
-                            double2 c[4];
-#pragma unroll
-                            for (int i = 0; i < 4; i++) c[i] = s_p[s_tpos[PQ(j + i)]];
-#pragma unroll
-                            for (int i = 0; i < 4; i++) { f.x = f.x - c[i].x; f.y = f.y - c[i].y; }
-                        }
-                        for (; j < cnt; j++) {
-                            const double2 c = s_p[s_tpos[PQ(j)]];
-                            f.x = f.x - c.x;
-                            f.y = f.y - c.y;
-                        }
-        #undef PQ
-                        s_f[node] = f;
-                    }
-                }
-                fence_proxy_async();
-                compute_sync();
-                if (tid == 0 && k + 2 < nch) {
-                    mbar_arrive_expect_tx(&s_bar[sel], (unsigned)nxt_bytes);
-                    bulk_load(bk, d.img + nxt_img, (unsigned)nxt_bytes, &s_bar[sel]);
-                    issued++;
-                }
-            }
-            if (tid == 0 && *s_abort)   // give the copies still in flight a bounded time to land
-                for (int c = k; c < issued; c++) mbar_wait_bounded(&s_bar[c & 1], (unsigned)((c >> 1) & 1));
-        } else {
-            // ---- contact forces (warp 7, meanwhile) --------------------------------------------
-            contact_scatter(d, b, n0, s_fc, lane);
-        }
-        __syncthreads();
-        if (*s_abort) return;
-    } else {
-        constexpr int NS = MEL_STAGES(1);
-        uint64_t* s_bar = reinterpret_cast<uint64_t*>(s_after);
-        // stage s of the ring: full[s] (the bulk copy landed), pointed[s] (every point thread has
-        // written its contributions), empty[s] (every pull thread is done with the buffer)
-        uint64_t* full = s_bar;
-        uint64_t* pointed = s_bar + NS;
-        uint64_t* empty = s_bar + 2 * NS;
-        s_abort = reinterpret_cast<volatile int*>(s_bar + 3 * NS);
-        region = reinterpret_cast<char*>(s_bar) + MEL_BAR_BYTES;
-        constexpr int PTW = MEL_PT_WARPS_MX;                  // point warps 0 .. PTW-1
-        constexpr int PLW = 7 - PTW;                          // pull warps PTW .. 6; warp 7 copies and scatters
-        const int ch0 = d.b_chunk0[b];
-        const int nch = d.b_chunk0[b + 1] - ch0;
-        for (int i = tid; i < n; i += blockDim.x) {
-            s_up[i] = d.up[n0 + i];
-            s_f[i] = make_double2(0., 0.);
-            s_fc[i] = make_double2(0., 0.);
-        }
-        if (MX) {
-            const double2 u0 = d.up[n0];
-            for (int i = tid; i < n; i += blockDim.x) {
-                const double2 u = d.up[n0 + i];
-                s_upf[i] = make_float2((float)(u.x - u0.x), (float)(u.y - u0.y));
-            }
-        }
-        if (tid == 0) {
-            for (int st = 0; st < NS; st++) {
-                mbar_init(&full[st], 1);
-                mbar_init(&pointed[st], 32 * PTW);
-                mbar_init(&empty[st], 32 * PLW);
-            }
-            mbar_init_fence();
-            *s_abort = 0;
-        }
-        __syncthreads();
-        // ---- Update_internal_forces as a pipeline over the body's chunks: warp 7 streams chunk images
-        // into a ring of NS buffers, the point warps form strain, stress and contributions of
-        // chunk k while the pull warps add those of chunk k-1 to the nodes (in ascending point order,
-        // chunk after chunk), so the two ordered chains and the copies overlap --------------------------
+    }
+    if (tid == 0) {
+        mbar_init(&s_bar[0], 1);
+        mbar_init(&s_bar[1], 1);
+        mbar_init_fence();
+        *s_abort = 0;
+    }
+    __syncthreads();
+    if (warp < MEL_BODY_CTHREADS / 32) {
+        // ---- Update_internal_forces: chunk k is computed while chunk k+1 is in flight ----------
         const int mat = d.b_mat[b];
         const int mtype = d.mat_type[mat];
         const double Mu = d.mat_p[MEL_MAT_NPARAM * mat + 3];
         const double Lam = d.mat_p[MEL_MAT_NPARAM * mat + 4];
-        if (warp < PTW) {
-            for (int k = 0; k < nch; k++) {
-                const int st = k % NS;
-                char* bk = region + st * d.img_cap;
-                if (*s_abort) break;
-                if (!mbar_wait_bounded(&full[st], (unsigned)((k / NS) & 1), d.wait_ns)) {
-                    atomicOr(&d.err[MEL_E_WAIT], 1u);
-                    *s_abort = 1;
-                    break;
-                }
-                const int4 hdr = *reinterpret_cast<const int4*>(bk);
-                const mel_chunk_layout L = mel_chunk_sections(hdr.x, hdr.y, hdr.z, hdr.w, MX ? 8 : 16);
-                if (tid < hdr.x) {
-                    if (MX)
-                        chunk_points_mx(tid, hdr.x, mtype, (float)Mu, (float)Lam, s_upf, reinterpret_cast<float2*>(bk + L.dN),
-                                        reinterpret_cast<const uint16_t*>(bk + L.idx), reinterpret_cast<const double*>(bk + L.c0),
-                                        reinterpret_cast<const unsigned*>(bk + L.gpm), reinterpret_cast<const uint16_t*>(bk + L.roff));
-                    else
-                        chunk_points(tid, hdr.x, mtype, Mu, Lam, s_up, reinterpret_cast<double2*>(bk + L.dN),
-                                     reinterpret_cast<const uint16_t*>(bk + L.idx), reinterpret_cast<const double*>(bk + L.c0),
-                                     reinterpret_cast<const unsigned*>(bk + L.gpm), reinterpret_cast<const uint16_t*>(bk + L.roff));
-                }
-                fence_proxy_async();      // these generic writes precede the copy that will refill the buffer
-                mbar_arrive(&pointed[st]);
+        int issued = 0;
+        if (tid == 0)
+            for (; issued < 2 && issued < nch; issued++) {
+                const mel_chunk c = d.chunk[ch0 + issued];
+                mbar_arrive_expect_tx(&s_bar[issued], (unsigned)c.bytes);
+                bulk_load(issued ? buf1 : buf0, d.img + c.img, (unsigned)c.bytes, &s_bar[issued]);
             }
-        } else if (warp < 7) {
-            // pull: each touched node subtracts its contributions in ascending Gauss-point order (the
-            // mixed form adds its FP32 contributions in FP64).  Pull slot t is lane t & 31 of group
-            // t >> 5, its entry j at row j of the group's row table.  Groups are sorted by entry count;
-            // pull warp w takes groups w, 2 PLW - 1 - w, 2 PLW + w, ... (snake order).  The group's
-            // barrier at the top of every chunk keeps a node's chunks in order when different warps
-            // hold it, and makes the group leave together when a wait gives up.
-            const int w = warp - PTW;
-            for (int k = 0; k < nch; k++) {
-                const int st = k % NS;
-                char* bk = region + st * d.img_cap;
-                const bool ok = !*s_abort && mbar_wait_bounded(&pointed[st], (unsigned)((k / NS) & 1), d.wait_ns);
-                if (!ok && !*s_abort) { atomicOr(&d.err[MEL_E_WAIT], 1u); *s_abort = 1; }
-                if (pull_group_any<32 * PLW>(!ok)) break;
-                const int4 hdr = *reinterpret_cast<const int4*>(bk);
-                const mel_chunk_layout L = mel_chunk_sections(hdr.x, hdr.y, hdr.z, hdr.w, MX ? 8 : 16);
-                const uint16_t* s_tpos = reinterpret_cast<const uint16_t*>(bk + L.tpos);
-                const unsigned* s_tn = reinterpret_cast<const unsigned*>(bk + L.tn);
-                const uint16_t* s_roff = reinterpret_cast<const uint16_t*>(bk + L.roff);
+        int k = 0;
+        for (; k < nch; k++) {
+            const int sel = k & 1;
+            char* bk = sel ? buf1 : buf0;
+            long long nxt_img = 0;
+            int nxt_bytes = 0;
+            if (tid == 0 && k + 2 < nch) { const mel_chunk c = d.chunk[ch0 + k + 2]; nxt_img = c.img; nxt_bytes = c.bytes; }
+            const bool ok = mbar_wait_bounded(&s_bar[sel], (unsigned)((k >> 1) & 1), d.wait_ns);
+            if (!ok) { atomicOr(&d.err[MEL_E_WAIT], 1u); *s_abort = 1; }
+            const int4 hdr = ok ? *reinterpret_cast<const int4*>(bk) : make_int4(0, 0, 0, 0);
+            const mel_chunk_layout L = mel_chunk_sections(hdr.x, hdr.y, hdr.z, hdr.w, MX ? 8 : 16, MX ? 0 : 1);
+            const uint16_t* s_idx = reinterpret_cast<const uint16_t*>(bk + L.idx);
+            const uint16_t* s_tpos = reinterpret_cast<const uint16_t*>(bk + L.tpos);
+            const unsigned* s_tn = reinterpret_cast<const unsigned*>(bk + L.tn);
+            const uint16_t* s_roff = reinterpret_cast<const uint16_t*>(bk + L.roff);
+            if (tid < hdr.x) {
+                if (MX)
+                    chunk_points_mx(tid, hdr.x, mtype, (float)Mu, (float)Lam, s_upf, reinterpret_cast<float2*>(bk + L.dN), s_idx,
+                                    reinterpret_cast<const double*>(bk + L.c0), reinterpret_cast<const unsigned*>(bk + L.gpm),
+                                    reinterpret_cast<const uint16_t*>(bk + L.roff));
+                else
+                    chunk_points(tid, hdr.x, mtype, Mu, Lam, s_up, reinterpret_cast<double2*>(bk + L.dN), s_idx,
+                                 reinterpret_cast<const double*>(bk + L.c0), reinterpret_cast<const unsigned*>(bk + L.gpm),
+                                 reinterpret_cast<const uint16_t*>(bk + L.roff));
+            }
+            compute_sync();
+            if (*s_abort) break;
+            if (MX) {
+                // pull of the mixed form, a two-level segmented reduction in place of the ordered
+                // chains: each lane sums one piece (at most MEL_PIECE entries of one node) in FP64,
+                // then the pieces of a node, on consecutive lanes, are combined by a Hillis-Steele
+                // scan over warp shuffles (equal node keys 2^i lanes apart mean one segment, as
+                // keys are sorted) and the last lane of each segment subtracts the sum from the
+                // node.  Warp w owns the pieces [wr[w], wr[w+1]), whole nodes only, balanced by
+                // entries, so no two warps touch one node.
+                const float2* s_q = reinterpret_cast<const float2*>(bk + L.dN);
+                const uint16_t* s_wr = reinterpret_cast<const uint16_t*>(bk + L.tn);
+                const unsigned* s_pc = reinterpret_cast<const unsigned*>(bk + L.tn + 16);
+                const int p1 = s_wr[warp + 1];
+                for (int p0 = s_wr[warp]; p0 < p1; p0 += 32) {
+                    const int pi = p0 + lane;
+                    const bool v = pi < p1;
+                    const unsigned rec = v ? s_pc[pi] : 0u;
+                    const int node = v ? (int)((rec >> 16) & 0xffffu) : -1;
+                    const int q0 = (int)(rec & 0x1fffu), cnt = v ? (int)((rec >> 13) & 7u) + 1 : 0;
+                    float2 c[MEL_PIECE];
+#pragma unroll
+                    for (int i = 0; i < MEL_PIECE; i++) c[i] = i < cnt ? s_q[s_tpos[q0 + i]] : make_float2(0.f, 0.f);
+                    double fx = 0., fy = 0.;
+#pragma unroll
+                    for (int i = 0; i < MEL_PIECE; i++) { fx = fx + (double)c[i].x; fy = fy + (double)c[i].y; }
+#pragma unroll
+                    for (int dd = 1; dd < 32; dd <<= 1) {
+                        const double ox = __shfl_up_sync(0xffffffffu, fx, dd);
+                        const double oy = __shfl_up_sync(0xffffffffu, fy, dd);
+                        const int on = __shfl_up_sync(0xffffffffu, node, dd);
+                        if (lane >= dd && on == node) { fx = fx + ox; fy = fy + oy; }
+                    }
+                    const int nn = __shfl_down_sync(0xffffffffu, node, 1);
+                    if (v && (lane == 31 || nn != node)) {
+                        double2 f = s_f[node];
+                        f.x = f.x - fx;
+                        f.y = f.y - fy;
+                        s_f[node] = f;
+                    }
+                    __syncwarp();     // a node continued by the next round reads this update
+                }
+            } else {
+                // pull: each touched node subtracts its contributions in ascending Gauss-point order.
+                // Pull slot t is lane t & 31 of group t >> 5, its entry j at row j of the group's row
+                // table.  Groups are sorted by entry count; warp w takes groups w, 13 - w, 14 + w, ...
+                // (snake order), so the heaviest group has a warp to itself and the lighter ones pair up.
                 const int ngrp = (hdr.z + 31) >> 5;
-                for (int i = 0; PLW * i < ngrp; i++) {
-                    const int t = (PLW * i + ((i & 1) ? PLW - 1 - w : w)) * 32 + lane;
+                for (int i = 0; 7 * i < ngrp; i++) {
+                    const int t = (7 * i + ((i & 1) ? 6 - warp : warp)) * 32 + lane;
                     if (t >= hdr.z) continue;
                     const unsigned rec = s_tn[t];
-                    const int node = (int)(rec & 0xfffu);
+                    const int node = (int)reinterpret_cast<const uint16_t*>(bk + L.tnode)[t];
                     const int cnt = (int)((rec >> 12) & 0xffu);
                     const uint16_t* prow = s_roff + (rec >> 20);
                     // rows every slot of a full group has: 32 wide and contiguous
@@ -1004,125 +797,449 @@ __device__ void deformable_body(const mel_dev& d, int b, double T, double T0, ch
     #define PQ(j) ((j) < pfull ? pbase + 32 * (j) + lane : prow[(j)] + lane)
                     double2 f = s_f[node];
                     int j = 0;
-                    if (MX) {
-                        const float2* s_q = reinterpret_cast<const float2*>(bk + L.dN);
-                        for (; j + 8 <= pfull; j += 8) {
-                            float2 c[8];
-    #pragma unroll
-                            for (int i = 0; i < 8; i++) c[i] = s_q[s_tpos[pbase + 32 * (j + i) + lane]];
-    #pragma unroll
-                            for (int i = 0; i < 8; i++) { f.x = f.x - (double)c[i].x; f.y = f.y - (double)c[i].y; }
-                        }
-                        for (; j + 8 <= cnt; j += 8) {      // remaining rows: row-table loads issued together
-                            int q[8];
-    #pragma unroll
-                            for (int i = 0; i < 8; i++) q[i] = PQ(j + i);
-                            float2 c[8];
-    #pragma unroll
-                            for (int i = 0; i < 8; i++) c[i] = s_q[s_tpos[q[i]]];
-    #pragma unroll
-                            for (int i = 0; i < 8; i++) { f.x = f.x - (double)c[i].x; f.y = f.y - (double)c[i].y; }
-                        }
-                        for (; j + 4 <= cnt; j += 4) {
-                            float2 c[4];
-    #pragma unroll
-                            for (int i = 0; i < 4; i++) c[i] = s_q[s_tpos[PQ(j + i)]];
-    #pragma unroll
-                            for (int i = 0; i < 4; i++) { f.x = f.x - (double)c[i].x; f.y = f.y - (double)c[i].y; }
-                        }
-                        for (; j < cnt; j++) {
-                            const float2 c = s_q[s_tpos[PQ(j)]];
-                            f.x = f.x - (double)c.x;
-                            f.y = f.y - (double)c.y;
-                        }
-                    } else {
-                        const double2* s_p = reinterpret_cast<const double2*>(bk + L.dN);
-                        for (; j + 8 <= pfull; j += 8) {
-                            double2 c[8];
-    #pragma unroll
-                            for (int i = 0; i < 8; i++) c[i] = s_p[s_tpos[pbase + 32 * (j + i) + lane]];
-    #pragma unroll
-                            for (int i = 0; i < 8; i++) { f.x = f.x - c[i].x; f.y = f.y - c[i].y; }
-                        }
-                        for (; j + 8 <= cnt; j += 8) {      // remaining rows: row-table loads issued together
-                            int q[8];
-    #pragma unroll
-                            for (int i = 0; i < 8; i++) q[i] = PQ(j + i);
-                            double2 c[8];
-    #pragma unroll
-                            for (int i = 0; i < 8; i++) c[i] = s_p[s_tpos[q[i]]];
-    #pragma unroll
-                            for (int i = 0; i < 8; i++) { f.x = f.x - c[i].x; f.y = f.y - c[i].y; }
-                        }
-                        for (; j + 4 <= cnt; j += 4) {
-                            double2 c[4];
-    #pragma unroll
-                            for (int i = 0; i < 4; i++) c[i] = s_p[s_tpos[PQ(j + i)]];
-    #pragma unroll
-                            for (int i = 0; i < 4; i++) { f.x = f.x - c[i].x; f.y = f.y - c[i].y; }
-                        }
-                        for (; j < cnt; j++) {
-                            const double2 c = s_p[s_tpos[PQ(j)]];
-                            f.x = f.x - c.x;
-                            f.y = f.y - c.y;
-                        }
+                    const double2* s_p = reinterpret_cast<const double2*>(bk + L.dN);
+                    for (; j + 8 <= pfull; j += 8) {
+                        double2 c[8];
+#pragma unroll
+                        for (int i = 0; i < 8; i++) c[i] = s_p[s_tpos[pbase + 32 * (j + i) + lane]];
+#pragma unroll
+                        for (int i = 0; i < 8; i++) { f.x = f.x - c[i].x; f.y = f.y - c[i].y; }
+                    }
+                    for (; j + 8 <= cnt; j += 8) {      // remaining rows: row-table loads issued together
+                        int q[8];
+#pragma unroll
+                        for (int i = 0; i < 8; i++) q[i] = PQ(j + i);
+                        double2 c[8];
+#pragma unroll
+                        for (int i = 0; i < 8; i++) c[i] = s_p[s_tpos[q[i]]];
+#pragma unroll
+                        for (int i = 0; i < 8; i++) { f.x = f.x - c[i].x; f.y = f.y - c[i].y; }
+                    }
+                    for (; j + 4 <= cnt; j += 4) {
+                        double2 c[4];
+#pragma unroll
+                        for (int i = 0; i < 4; i++) c[i] = s_p[s_tpos[PQ(j + i)]];
+#pragma unroll
+                        for (int i = 0; i < 4; i++) { f.x = f.x - c[i].x; f.y = f.y - c[i].y; }
+                    }
+                    for (; j < cnt; j++) {
+                        const double2 c = s_p[s_tpos[PQ(j)]];
+                        f.x = f.x - c.x;
+                        f.y = f.y - c.y;
                     }
     #undef PQ
                     s_f[node] = f;
                 }
-                fence_proxy_async();
-                mbar_arrive(&empty[st]);
             }
-        } else if (lane == 0) {
-            // ---- producer: the first NS chunks at once, then each chunk into the buffer the
-            // pull warps released ----------------------------------------------------------------------
-            int issued = 0;
-            for (; issued < NS && issued < nch; issued++) {
-                const mel_chunk c = d.chunk[ch0 + issued];
-                mbar_arrive_expect_tx(&full[issued], (unsigned)c.bytes);
-                bulk_load(region + issued * d.img_cap, d.img + c.img, (unsigned)c.bytes, &full[issued]);
+            fence_proxy_async();
+            compute_sync();
+            if (tid == 0 && k + 2 < nch) {
+                mbar_arrive_expect_tx(&s_bar[sel], (unsigned)nxt_bytes);
+                bulk_load(bk, d.img + nxt_img, (unsigned)nxt_bytes, &s_bar[sel]);
+                issued++;
             }
-            for (; issued < nch; issued++) {
-                const int st = issued % NS;
-                const mel_chunk c = d.chunk[ch0 + issued];
-                if (*s_abort) break;
-                if (!mbar_wait_bounded(&empty[st], (unsigned)((issued / NS - 1) & 1), d.wait_ns)) {
-                    atomicOr(&d.err[MEL_E_WAIT], 1u);
-                    *s_abort = 1;
-                    break;
+        }
+        if (tid == 0 && *s_abort)   // give the copies still in flight a bounded time to land
+            for (int c = k; c < issued; c++) mbar_wait_bounded(&s_bar[c & 1], (unsigned)((c >> 1) & 1));
+    } else {
+        // ---- contact forces (warp 7, meanwhile) --------------------------------------------
+        contact_scatter(d, b, n0, s_fc, lane);
+    }
+    __syncthreads();
+    return *s_abort == 0;
+}
+
+// ---- Gauss-point pass over tiles (layout in mel_tiles.h) -------------------------------------
+// Loads that are issued where they stand: the compiler must not sink them past a barrier to their
+// first use.  A predicated load leaves its target alone where `on` is false.
+__device__ __forceinline__ void ld_pair_if(double2& v, const double2* p, bool on)
+{
+    asm volatile("{\n\t.reg .pred p;\n\tsetp.ne.u32 p, %3, 0;\n\t@p ld.global.nc.L1::no_allocate.v2.f64 {%0, %1}, [%2];\n\t}"
+                 : "+d"(v.x), "+d"(v.y) : "l"(p), "r"((unsigned)on));
+}
+__device__ __forceinline__ void ld_pair_if(float4& v, const float4* p, bool on)
+{
+    asm volatile("{\n\t.reg .pred p;\n\tsetp.ne.u32 p, %5, 0;\n\t@p ld.global.nc.L1::no_allocate.v4.f32 {%0, %1, %2, %3}, [%4];\n\t}"
+                 : "+f"(v.x), "+f"(v.y), "+f"(v.z), "+f"(v.w) : "l"(p), "r"((unsigned)on));
+}
+// asks for `bytes` (a multiple of 16) from p (16-byte aligned) to be brought into L2
+__device__ __forceinline__ void l2_prefetch(const void* p, unsigned bytes)
+{
+    asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" :: "l"(p), "r"(bytes) : "memory");
+}
+__device__ __forceinline__ uint4 ld_quad(const void* p)
+{
+    uint4 v;
+    asm volatile("ld.global.nc.v4.u32 {%0, %1, %2, %3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "l"(p));
+    return v;
+}
+
+// `load` brings `per` rows of derivative pairs
+template <bool MX> struct tile_rows_t;
+template <> struct tile_rows_t<false> { typedef double2 load; typedef double2 pair; static constexpr int per = 1; };
+template <> struct tile_rows_t<true> { typedef float4 load; typedef float2 pair; static constexpr int per = 2; };
+
+__device__ __forceinline__ double2 row_of(const double2& v, int) { return v; }
+__device__ __forceinline__ float2 row_of(const float4& v, int r) { return r ? make_float2(v.z, v.w) : make_float2(v.x, v.y); }
+
+// The pass (Body::Update_internal_forces, Code/Body.h:937-1049) of warps 0-6 over body b's tiles: a
+// thread per Gauss point forms strain, stress and contributions, then a thread per touched node
+// subtracts its contributions.  Strain sums run in support order and every node's in ascending
+// point order, tile after tile, as the reference adds them.  The mixed form keeps derivative pairs,
+// strain, stress and contributions in FP32 (displacements relative to the body's first node) and the
+// nodes' sums in FP64.  Sets *s_abort when a wait gives up.
+//
+// What bounds it: latency.  The derivative pairs are read once (16 of the 20 bytes an entry), half of
+// them into registers, asked for while the tile before is finished, and half by a bulk copy; the
+// next tile's pairs are brought to L2 a tile ahead.  Shared memory carries the displacement gathers,
+// the contributions (each written and read once, without bank conflicts) and what the copies bring.
+// Measured on B200, 700 grains of 384 nodes: FP64 272 -> 183 us a launch, mixed 193 -> 146 us, against
+// whole chunk images in two shared-memory buffers (each pair read three times there, both gathers
+// meeting banks twice on average, 134 points a chunk for 7 warps); 50 grains of 192 to 576 nodes,
+// one body an SM, FP64 122 -> 69 us.
+template <bool MX>
+__device__ __forceinline__ void tile_forces(const mel_dev& d, int b, const typename tile_rows_t<MX>::pair* s_u, double2* s_f,
+                                            char* region, uint64_t* s_bar, volatile int* s_abort, int tid, int lane, int warp)
+{
+    typedef tile_rows_t<MX> rows_t;
+    typedef typename rows_t::load load_t;
+    typedef typename rows_t::pair pair_t;
+    constexpr int PER = rows_t::per, HEAD = MEL_TILE_HEAD(MX);
+    const int mat = d.b_mat[b];
+    const int mtype = d.mat_type[mat];
+    const double Mu = d.mat_p[MEL_MAT_NPARAM * mat + 3];
+    const double Lam = d.mat_p[MEL_MAT_NPARAM * mat + 4];
+    const int t1 = d.b_tile0[b + 1];
+    int t = d.b_tile0[b];
+    if (t >= t1) return;
+    // region: contributions (tile_cap slots and a zero one that padded positions name), index words,
+    // then pull slots and position words
+    pair_t* const s_q = reinterpret_cast<pair_t*>(region);
+    char* const s_idx = region + d.tile_q;
+    char* const s_pull = s_idx + d.tile_i;
+    uint64_t* const bar_i = s_bar + 1;
+    uint64_t* const bar_p = s_bar + 2;
+    uint4 T = ld_quad(d.tile + t), Tn = t + 1 < t1 ? ld_quad(d.tile + t + 1) : make_uint4(0u, 0u, 0u, 0u);
+    auto issue_idx = [&](const uint4& H) {
+        const int bytes = mel_tile_idx_bytes(H.y);
+        mbar_arrive_expect_tx(bar_i, (unsigned)bytes);
+        bulk_load(s_idx, d.timg + mel_tile_base(H.x) + mel_tile_o_idx(H.y, H.z), (unsigned)bytes, bar_i);
+    };
+    auto issue_pull = [&](const uint4& H) {
+        const int bytes = mel_tile_pull_bytes(H.z, H.w);
+        mbar_arrive_expect_tx(bar_p, (unsigned)bytes);
+        bulk_load(s_pull, d.timg + mel_tile_base(H.x) + mel_tile_o_slot(H.y, H.z), (unsigned)bytes, bar_p);
+    };
+    if (tid == 0) { issue_idx(T); issue_pull(T); }
+    // this thread's point: its rows' address, supports, the group's rows and width, first slot and
+    // index word, c0.  Lanes beyond the group's points follow with no supports of their own
+    struct lane_t { const load_t* dn; double c0; int ns, K, w; unsigned s0, i0, t0; };
+    auto point = [&](const uint4& H) {
+        const int last = (int)(H.z & 0xffffu) - 1;
+        return ld_quad(reinterpret_cast<const mel_point*>(d.timg + mel_tile_base(H.x) + mel_tile_o_rec(H.y)) + min(tid, last));
+    };
+    auto take = [&](const uint4& r, const uint4& H) {
+        lane_t L;
+        const int np = (int)(H.z & 0xffffu);
+        L.c0 = __hiloint2double((int)r.y, (int)r.x);
+        L.w = 8 * (int)((r.w >> 14) & 3u) + 8;
+        L.ns = tid < np ? (int)((r.z >> 16) & 0xffu) : 0;
+        L.K = (warp << 5) < np ? (int)(r.z >> 24) : 0;
+        L.s0 = r.z & 0xffffu;
+        L.i0 = r.w & 0x3fffu;
+        L.t0 = r.w >> 16;
+        L.dn = reinterpret_cast<const load_t*>(d.timg + mel_tile_base(H.x)) + (L.s0 - L.t0) / PER + min(lane, L.w - 1);
+        return L;
+    };
+    // rows k .. k + PER - 1 of the point of L, zero beyond its supports
+    auto fetch = [&](load_t& v, const lane_t& L, int k) {
+        memset(&v, 0, sizeof v);
+        ld_pair_if(v, L.dn + k / PER * L.w, k < L.ns);
+    };
+    lane_t L = take(point(T), T);
+    load_t g[HEAD / PER];
+#pragma unroll
+    for (int k = 0; k < HEAD; k += PER) fetch(g[k / PER], L, k);
+    const unsigned long long pad_i = (unsigned long long)(d.b_node0[b + 1] - d.b_node0[b]) * 0x0001000100010001ull;
+    unsigned phase = 0, phase_i = 0;        // of the copies in flight: pull sections, index words
+    for (; t < t1; t++) {
+        const uint4 Tnn = t + 2 < t1 ? ld_quad(d.tile + t + 2) : make_uint4(0u, 0u, 0u, 0u);
+        const bool more = t + 1 < t1;
+        if (more && tid == 0) l2_prefetch(d.timg + mel_tile_base(Tn.x), (unsigned)mel_tile_o_idx(Tn.y, Tn.z));
+        const uint4 rn = point(more ? Tn : T);
+        lane_t N = L;
+        bool ok = mbar_wait_bounded(bar_i, phase_i, d.wait_ns);
+        if (!ok) { atomicOr(&d.err[MEL_E_WAIT], 1u); *s_abort = 1; }
+        if (ok && L.K > 0) {
+            const int lw = min(lane, L.w - 1);
+            const load_t* const tail = reinterpret_cast<const load_t*>(s_idx) + L.t0 / PER + lw;
+            const unsigned long long* ix = reinterpret_cast<const unsigned long long*>(s_idx + mel_tile_tail_bytes(T.w)) + L.i0 + lw;
+            pair_t* const q0 = s_q + L.s0 + (lane & ~(MEL_PLACES(MX) - 1));
+            unsigned long long wd[HEAD / 4];
+#pragma unroll
+            for (int k = 0; k < HEAD; k += 4) wd[k / 4] = k < L.K ? ix[(k >> 2) * L.w] : pad_i;
+            // f(k, pair, word) for this point's rows in order: those in registers without a branch
+            // between them, so that their gathers overlap (a row beyond its supports has a zero pair
+            // and names a zero displacement), then the tail rows; after(k) follows the first HEAD
+            auto rows = [&](auto&& f, auto&& after) {
+#pragma unroll
+                for (int k = 0; k < HEAD; k++) {
+                    f(k, row_of(g[k / PER], k & (PER - 1)), (unsigned)(wd[k / 4] >> (16 * (k & 3))) & 0xffffu);
+                    if ((k & (PER - 1)) == PER - 1) after(k - (PER - 1));
                 }
-                mbar_arrive_expect_tx(&full[st], (unsigned)c.bytes);
-                bulk_load(region + st * d.img_cap, d.img + c.img, (unsigned)c.bytes, &full[st]);
-            }
-            if (*s_abort)   // give the copies still in flight a bounded time to land before the CTA ends
-                for (int c = issued - 1; c >= 0 && c >= issued - NS; c--)
-                    mbar_wait_bounded(&full[c % NS], (unsigned)((c / NS) & 1));
-        } else {
-            // ---- contact forces (lanes 1-31 of warp 7, meanwhile): slave scatter in list order, then
-            // master scatter in send order (Body::Update_contact_forces, Code/Body.h:1642-1900) ---------
-            const unsigned mask = 0xfffffffeu;
-            for (int c = d.b_cont0[b]; c < d.b_cont0[b + 1]; c++) {
-                const mel_contact* ct = d.cont + c;
-                if (d.table[d.b_mat[b] * d.nmat + d.b_mat[ct->bodyM]] <= -1) continue;
-                double Fsx = ct->fx, Fsy = ct->fy;
-                warp_scatter(d, n0, ct->nodeS, Fsx, Fsy, s_fc, lane - 1, 31);
-                __syncwarp(mask);
-            }
-            for (int r = d.b_inc0[b]; r < d.b_inc0[b + 1]; r++) {
-                int2 rg = d.inc_rng[r];
-                for (int c = rg.x; c < rg.y; c++) {
-                    const mel_contact* ct = d.cont + c;
-                    if (d.table[d.b_mat[ct->bodyS] * d.nmat + d.b_mat[b]] <= -1) continue;
-                    double Fsx = ct->fx, Fsy = ct->fy;
-                    for (int k = 0; k < 4; k++) {
-                        double sk = ct->shapeM[k];
-                        warp_scatter(d, n0, ct->nodeM[k], -Fsx * sk, -Fsy * sk, s_fc, lane - 1, 31);
-                        __syncwarp(mask);
+                for (int k = HEAD; k < L.K; k += 4) {
+                    const unsigned long long wk = ix[(k >> 2) * L.w];
+                    load_t v[4 / PER];
+#pragma unroll
+                    for (int r = 0; r < 4; r += PER) {
+                        memset(&v[r / PER], 0, sizeof v[0]);
+                        if (k + r < L.ns) v[r / PER] = tail[(k - HEAD + r) / PER * L.w];
                     }
+#pragma unroll
+                    for (int r = 0; r < 4; r++)
+                        f(k + r, row_of(v[r / PER], r & (PER - 1)), (unsigned)(wk >> (16 * r)) & 0xffffu);
+                }
+            };
+            auto nothing = [](int) {};
+            // the next tile's rows take the registers of this one's as their contributions are written
+            auto refill = [&](int k) { fetch(g[k / PER], N, k); };
+            auto next = [&]() { N = take(rn, more ? Tn : T); if (!more) N.ns = 0; };
+            auto put = [&](int k, unsigned w16, auto qx, auto qy) {
+                if (k < L.ns) { pair_t q; q.x = qx; q.y = qy; q0[k * L.w + (int)(w16 >> 12)] = q; }
+            };
+            const double c0 = L.c0;
+            if constexpr (!MX) {
+                if (mtype == MEL_MAT_ELASTIC_LINEAR) {
+                    double E11 = 0., E12 = 0., E22 = 0.;
+                    rows([&](int, const double2& n, unsigned w16) {
+                        const double2 u = s_u[w16 & 0xfffu];
+                        E11 = E11 + n.x * u.x;
+                        E12 = E12 + (n.x * u.y + n.y * u.x);
+                        E22 = E22 + n.y * u.y;
+                    }, nothing);
+                    E12 = 0.5 * E12;
+                    const double J = 1. + E11 + E22;               // Apply_Elastic_Linear (Code/Model.h:19-29)
+                    const double S33 = Lam * (J - 1.);
+                    const double Mu2 = 2 * Mu;
+                    const double S11 = S33 + Mu2 * E11, S22 = S33 + Mu2 * E22, S12 = Mu2 * E12;
+                    next();
+                    rows([&](int k, const double2& n, unsigned w16) {
+                        put(k, w16, c0 * (n.x * S11 + n.y * S12), c0 * (n.y * S22 + n.x * S12));
+                    }, refill);
+                } else {
+                    double F11 = 1., F12 = 0., F21 = 0., F22 = 1.;
+                    rows([&](int, const double2& n, unsigned w16) {
+                        const double2 u = s_u[w16 & 0xfffu];
+                        F11 += n.x * u.x; F12 += n.y * u.x; F21 += n.x * u.y; F22 += n.y * u.y;
+                    }, nothing);
+                    const double Kappa = Lam;                       // Apply_NeoHookean (Code/Model.h:52-73)
+                    const double F11F12 = F11 * F11 + F12 * F12, F21F22 = F21 * F21 + F22 * F22;
+                    const double J = F11 * F22 - F12 * F21;
+                    const double invJ = 1. / J;
+                    const double KJ = Kappa * (J - 1.);
+                    const double MuJ53 = Mu * pow(J, -1.666666666667);
+                    const double trB = 0.333333333333 * (F11F12 + F21F22 + 1.);
+                    const double s11 = KJ + MuJ53 * (F11F12 - trB), s22 = KJ + MuJ53 * (F21F22 - trB);
+                    const double s12 = MuJ53 * (F11 * F21 + F12 * F22);
+                    const double S11 = (F12 * (F12 * s22 - F22 * s12) - F22 * (F12 * s12 - F22 * s11)) * invJ;
+                    const double S22 = (F11 * (F11 * s22 - F21 * s12) - F21 * (F11 * s12 - F21 * s11)) * invJ;
+                    const double S12 = (F21 * (F12 * s12 - F22 * s11) - F11 * (F12 * s22 - F22 * s12)) * invJ;
+                    const double A1 = F11 * S11 + F12 * S12, B1 = F12 * S22 + F11 * S12;
+                    const double A2 = F21 * S11 + F22 * S12, B2 = F22 * S22 + F21 * S12;
+                    next();
+                    rows([&](int k, const double2& n, unsigned w16) {
+                        put(k, w16, c0 * (n.x * A1 + n.y * B1), c0 * (n.x * A2 + n.y * B2));
+                    }, refill);
+                }
+            } else {
+                const float c0f = (float)c0, Muf = (float)Mu, Lamf = (float)Lam;
+                if (mtype == MEL_MAT_ELASTIC_LINEAR) {
+                    float E11 = 0.f, E12 = 0.f, E22 = 0.f;
+                    rows([&](int, const float2& n, unsigned w16) {
+                        const float2 u = s_u[w16 & 0xfffu];
+                        E11 = __fmaf_rn(n.x, u.x, E11);
+                        E12 = __fmaf_rn(n.x, u.y, __fmaf_rn(n.y, u.x, E12));
+                        E22 = __fmaf_rn(n.y, u.y, E22);
+                    }, nothing);
+                    E12 = 0.5f * E12;
+                    const float S33 = Lamf * (E11 + E22);     // Apply_Elastic_Linear (Code/Model.h:19-29), J - 1 = tr E
+                    const float Mu2 = 2.f * Muf;
+                    const float S11 = __fmaf_rn(Mu2, E11, S33), S22 = __fmaf_rn(Mu2, E22, S33), S12 = Mu2 * E12;
+                    next();
+                    rows([&](int k, const float2& n, unsigned w16) {
+                        put(k, w16, c0f * __fmaf_rn(n.x, S11, n.y * S12), c0f * __fmaf_rn(n.y, S22, n.x * S12));
+                    }, refill);
+                } else {
+                    float G11 = 0.f, G12 = 0.f, G21 = 0.f, G22 = 0.f;   // F - I
+                    rows([&](int, const float2& n, unsigned w16) {
+                        const float2 u = s_u[w16 & 0xfffu];
+                        G11 = __fmaf_rn(n.x, u.x, G11); G12 = __fmaf_rn(n.y, u.x, G12);
+                        G21 = __fmaf_rn(n.x, u.y, G21); G22 = __fmaf_rn(n.y, u.y, G22);
+                    }, nothing);
+                    const float F11 = 1.f + G11, F12 = G12, F21 = G21, F22 = 1.f + G22;
+                    const float Kappa = Lamf;                  // Apply_NeoHookean (Code/Model.h:52-73)
+                    const float F11F12 = F11 * F11 + F12 * F12, F21F22 = F21 * F21 + F22 * F22;
+                    const float Jm1 = G11 + G22 + (G11 * G22 - G12 * G21);   // J - 1 without cancellation
+                    const float J = 1.f + Jm1;
+                    const float invJ = 1.f / J;
+                    const float KJ = Kappa * Jm1;
+                    const float MuJ53 = Muf * powf(J, -1.666666667f);
+                    const float trB = 0.333333333f * (F11F12 + F21F22 + 1.f);
+                    const float s11 = KJ + MuJ53 * (F11F12 - trB), s22 = KJ + MuJ53 * (F21F22 - trB);
+                    const float s12 = MuJ53 * (F11 * F21 + F12 * F22);
+                    const float S11 = (F12 * (F12 * s22 - F22 * s12) - F22 * (F12 * s12 - F22 * s11)) * invJ;
+                    const float S22 = (F11 * (F11 * s22 - F21 * s12) - F21 * (F11 * s12 - F21 * s11)) * invJ;
+                    const float S12 = (F21 * (F12 * s12 - F22 * s11) - F11 * (F12 * s22 - F22 * s12)) * invJ;
+                    const float A1 = F11 * S11 + F12 * S12, B1 = F12 * S22 + F11 * S12;
+                    const float A2 = F21 * S11 + F22 * S12, B2 = F22 * S22 + F21 * S12;
+                    next();
+                    rows([&](int k, const float2& n, unsigned w16) {
+                        put(k, w16, c0f * (n.x * A1 + n.y * B1), c0f * (n.x * A2 + n.y * B2));
+                    }, refill);
                 }
             }
         }
-        __syncwarp();
+        else if (ok && more) {        // no point in this tile's group: the next tile's rows
+            N = take(rn, Tn);
+#pragma unroll
+            for (int k = 0; k < HEAD; k += PER) fetch(g[k / PER], N, k);
+        }
+        compute_sync();
+        if (*s_abort) break;
+        if (more) {
+            phase_i ^= 1u;
+            if (tid == 0) { fence_proxy_async(); issue_idx(Tn); }
+        }
+        ok = mbar_wait_bounded(bar_p, phase, d.wait_ns);
+        if (!ok) { atomicOr(&d.err[MEL_E_WAIT], 1u); *s_abort = 1; }
+        else {
+            // pull: slot s is lane s & 31 of group s >> 5, groups sorted by entry count; warp w takes
+            // groups w, 13 - w, 14 + w, ... so that the heavy ones are spread over the warps
+            const int nslot = (int)(T.z >> 16), ngrp = (nslot + 31) >> 5;
+            const uint2* slots = reinterpret_cast<const uint2*>(s_pull);
+            const unsigned long long* pos = reinterpret_cast<const unsigned long long*>(s_pull + ((8 * nslot + 15) & ~15));
+            for (int i = 0; 7 * i < ngrp; i++) {
+                const int grp = 7 * i + ((i & 1) ? 6 - warp : warp);
+                if (grp >= ngrp) continue;
+                const int s = grp * 32 + lane;
+                const uint2 sl = slots[min(s, nslot - 1)];
+                const int node = (int)(sl.x & 0xffffu);
+                const int cmax = (int)(slots[grp * 32].x >> 16);      // the group's first slot has the most
+                const unsigned long long* pw = pos + sl.y + lane;
+                double2 f = s_f[node];
+                // four contributions are on their way while the four before them are subtracted; positions
+                // past the group's last name the zero slot
+                auto word = [&](int j) { return j < cmax ? pw[8 * j] : d.tile_pad; };
+                auto load = [&](pair_t (&c)[4], unsigned long long wq) {
+#pragma unroll
+                    for (int r = 0; r < 4; r++) c[r] = s_q[(unsigned)(wq >> (16 * r)) & 0xffffu];
+                };
+                auto sub = [&](const pair_t (&c)[4]) {
+#pragma unroll
+                    for (int r = 0; r < 4; r++) { f.x = f.x - (double)c[r].x; f.y = f.y - (double)c[r].y; }
+                };
+                pair_t c[4], e[4];
+                unsigned long long wc = word(0), we = word(4);
+                load(c, wc);
+                for (int j = 0; j < cmax; j += 8) {
+                    wc = word(j + 8);
+                    load(e, we);
+                    sub(c);
+                    we = word(j + 12);
+                    load(c, wc);
+                    sub(e);
+                }
+                if (s < nslot) s_f[node] = f;
+            }
+        }
+        compute_sync();
+        if (*s_abort) break;
+        if (tid == 0 && more) { fence_proxy_async(); issue_pull(Tn); }
+        L = N;
+        T = Tn;
+        Tn = Tnn;
+        phase ^= 1u;
+    }
+    if (*s_abort && tid == 0) {       // give the copies still in flight a bounded time to land
+        mbar_wait_bounded(bar_i, phase_i);
+        mbar_wait_bounded(bar_p, phase);
+    }
+}
+
+// Shared memory of a deformable body of n nodes (at most MEL_MAX_BODY_NODES):
+//   s_up                   n + 1 double2       displacements (and a zero that padded rows name)
+//   s_f, s_fc              2 x n double2       internal forces, contact forces
+//   s_upf (mixed only)     n2 x float2         displacements relative to node 0 (n2 = n + 1 rounded to 2)
+//   mbarriers + abort flag                     MEL_BAR_BYTES
+//   region                 a tile's contributions, index words and pull slots during the Gauss-point
+//                          pass, then s_fn, s_fd, s_vp, s_ap (n double2 each), the six work terms per
+//                          node (6 x n double) and, in the first half-step of Solver_step, the
+//                          temporary displacement parameters (n double2)
+// A larger body ("wide", its own instantiation so that the others keep plain shared-memory
+// addressing) keeps its node arrays in global memory; shared memory then holds the mbarriers and
+// its two chunk images.
+template <bool MX, bool AD, bool WIDE>
+__device__ void deformable_body(const mel_dev& d, int b, double T, double T0, char* smem)
+{
+    const int tid = threadIdx.x;
+    const int lane = tid & 31, warp = tid >> 5;
+    const int n0 = d.b_node0[b];
+    const int n = d.b_node0[b + 1] - n0;
+    const double dt = d.dt[0];
+    constexpr bool wide = WIDE;
+    const long long go = WIDE ? d.b_gscr[b] : 0LL;
+    double2* s_up = wide ? d.up + n0 : reinterpret_cast<double2*>(smem);
+    double2* s_f = wide ? reinterpret_cast<double2*>(d.gscr + go) : s_up + n + 1;
+    double2* s_fc = s_f + n;
+    float2* s_upf = reinterpret_cast<float2*>(s_fc + n);
+    char* const s_after = wide ? smem : (MX ? reinterpret_cast<char*>(s_upf + ((n + 2) & ~1)) : reinterpret_cast<char*>(s_fc + n));
+    // the Gauss-point pass, which leaves the internal forces in s_f and the contact forces in s_fc
+    char* const region = s_after + MEL_BAR_BYTES;
+    if (wide) {
+        if (!chunk_forces<MX>(d, b, smem, s_up, s_f, s_fc, s_upf)) return;
+    } else {
+        uint64_t* s_bar = reinterpret_cast<uint64_t*>(s_after);
+        volatile int* s_abort = reinterpret_cast<volatile int*>(s_bar + 3);
+        // warp 0 has the displacement parameters brought by one bulk copy and waits for it; the others
+        // clear the force sums.  s_bar[1] and s_bar[2] serve the tiles
+        if (warp == 0) {
+            if (lane == 0) {
+                for (int i = 0; i < 3; i++) mbar_init(s_bar + i, 1);
+                mbar_init_fence();
+                *s_abort = 0;
+                mbar_arrive_expect_tx(s_bar, (unsigned)(sizeof(double2) * n));
+                bulk_load(s_up, d.up + n0, (unsigned)(sizeof(double2) * n), s_bar);
+                // what padded rows and positions name: a zero displacement and a zero contribution
+                s_up[n] = make_double2(0., 0.);
+                if (MX) { s_upf[n] = make_float2(0.f, 0.f); reinterpret_cast<float2*>(region)[d.tile_cap] = make_float2(0.f, 0.f); }
+                else reinterpret_cast<double2*>(region)[d.tile_cap] = make_double2(0., 0.);
+            }
+            __syncwarp();
+            if (!mbar_wait_bounded(s_bar, 0u, d.wait_ns)) { atomicOr(&d.err[MEL_E_WAIT], 1u); *s_abort = 1; }
+        } else {
+            for (int i = tid - 32; i < n; i += blockDim.x - 32) {
+                s_f[i] = make_double2(0., 0.);
+                s_fc[i] = make_double2(0., 0.);
+            }
+        }
+        __syncthreads();
+        if (*s_abort) {
+            if (tid == 0) mbar_wait_bounded(s_bar, 0u);   // give the copy in flight a bounded time to land
+            return;
+        }
+        mbar_wait_bounded(s_bar, 0u);                     // complete: every thread sees what the copy wrote
+        if (MX) {
+            const double2 u0 = s_up[0];
+            for (int i = tid; i < n; i += blockDim.x) {
+                const double2 u = s_up[i];
+                s_upf[i] = make_float2((float)(u.x - u0.x), (float)(u.y - u0.y));
+            }
+            __syncthreads();
+        }
+        if (warp < MEL_BODY_CTHREADS / 32) {
+            if constexpr (MX) tile_forces<true>(d, b, s_upf, s_f, region, s_bar, s_abort, tid, lane, warp);
+            else tile_forces<false>(d, b, s_up, s_f, region, s_bar, s_abort, tid, lane, warp);
+        } else contact_scatter(d, b, n0, s_fc, lane);      // warp 7, meanwhile
         __syncthreads();
         if (*s_abort) return;
     }
@@ -1622,7 +1739,7 @@ __device__ __forceinline__ void wide_body_cta(const mel_dev& d, int bb, double T
     deformable_body<MX, AD, true>(d, b, T, T0, smem);
 }
 
-__global__ void __launch_bounds__(128) contact_kernel(mel_dev d, double law_dt_scale, int czm_init)
+__global__ void __launch_bounds__(128) contact_kernel(const __grid_constant__ mel_dev d, double law_dt_scale, int czm_init)
 {
     contact_thread(d, blockIdx.x * blockDim.x + threadIdx.x, law_dt_scale, czm_init);
 }
@@ -1630,7 +1747,7 @@ __global__ void __launch_bounds__(128) contact_kernel(mel_dev d, double law_dt_s
 // One model: CTA i is the body d.b_order[i]; time2[parity] is the step's start time, the step's
 // end time goes to time2[parity ^ 1] (the next launch reads it).
 template <bool MX>
-__global__ void __launch_bounds__(MEL_BODY_THREADS, 2) body_kernel(mel_dev d, int parity)
+__global__ void __launch_bounds__(MEL_BODY_THREADS, 2) body_kernel(const __grid_constant__ mel_dev d, int parity)
 {
     extern __shared__ __align__(16) char smem[];
     const double T = d.time2[parity];
@@ -1641,7 +1758,7 @@ __global__ void __launch_bounds__(MEL_BODY_THREADS, 2) body_kernel(mel_dev d, in
 // One half-step of Solver_step (d.phase 1 or 2) of one model: T0 = Time, Tf = the time the
 // border conditions of the forces are taken at.  The host keeps the time.
 template <bool MX>
-__global__ void __launch_bounds__(MEL_BODY_THREADS, 2) body_kernel_adaptive(mel_dev d, double T0, double Tf)
+__global__ void __launch_bounds__(MEL_BODY_THREADS, 2) body_kernel_adaptive(const __grid_constant__ mel_dev d, double T0, double Tf)
 {
     extern __shared__ __align__(16) char smem[];
     body_cta<MX, true>(d, blockIdx.x, Tf, smem, T0);
@@ -1650,7 +1767,7 @@ __global__ void __launch_bounds__(MEL_BODY_THREADS, 2) body_kernel_adaptive(mel_
 // The wide bodies b_order[first + i]; the step's end time is written here when the launch above
 // had no CTA (set_time)
 template <bool MX>
-__global__ void __launch_bounds__(MEL_BODY_THREADS, 2) body_kernel_wide(mel_dev d, int parity, int first, int set_time)
+__global__ void __launch_bounds__(MEL_BODY_THREADS, 2) body_kernel_wide(const __grid_constant__ mel_dev d, int parity, int first, int set_time)
 {
     extern __shared__ __align__(16) char smem[];
     const double T = d.time2[parity];
@@ -1659,14 +1776,14 @@ __global__ void __launch_bounds__(MEL_BODY_THREADS, 2) body_kernel_wide(mel_dev 
 }
 
 template <bool MX>
-__global__ void __launch_bounds__(MEL_BODY_THREADS, 2) body_kernel_adaptive_wide(mel_dev d, double T0, double Tf, int first)
+__global__ void __launch_bounds__(MEL_BODY_THREADS, 2) body_kernel_adaptive_wide(const __grid_constant__ mel_dev d, double T0, double Tf, int first)
 {
     extern __shared__ __align__(16) char smem[];
     wide_body_cta<MX, true>(d, first + blockIdx.x, Tf, smem, T0);
 }
 
 // Solver_step's sums over bodies in body order (Code/Solver.h:289-331)
-__global__ void error_reduce_kernel(mel_dev d, double* out)
+__global__ void error_reduce_kernel(const __grid_constant__ mel_dev d, double* out)
 {
     if (threadIdx.x != 0 || blockIdx.x != 0) return;
     double mean = 0., mx = 0., tm = 0., mm = 0.;
@@ -1738,7 +1855,7 @@ __global__ void advance_kernel(const mel_dev* devs, int nsamp)
 // active contact elements; block partials then a fixed-order final sum (deterministic)
 // ------------------------------------------------------------------------------------------
 #define MON_BLOCKS 148
-__global__ void monitor_partial_kernel(mel_dev d, double* part)
+__global__ void monitor_partial_kernel(const __grid_constant__ mel_dev d, double* part)
 {
     __shared__ double s[5][256];
     double ke = 0., ux = 0., uy = 0., mt = 0., act = 0.;
@@ -1759,7 +1876,7 @@ __global__ void monitor_partial_kernel(mel_dev d, double* part)
     if (threadIdx.x < 5) part[threadIdx.x * MON_BLOCKS + blockIdx.x] = s[threadIdx.x][0];
 }
 
-__global__ void monitor_final_kernel(mel_dev d, const double* part, const int* rigid_ids, int nrigid, double* out)
+__global__ void monitor_final_kernel(const __grid_constant__ mel_dev d, const double* part, const int* rigid_ids, int nrigid, double* out)
 {
     if (threadIdx.x == 0) {
         double t[5] = { 0., 0., 0., 0., 0. };
@@ -1791,13 +1908,13 @@ __device__ __forceinline__ void pressure_push(const mel_dev& d, int e, int v)
     else set_err(d, MEL_E_PRESSURE);
 }
 
-__global__ void pressure_clear_kernel(mel_dev d)
+__global__ void pressure_clear_kernel(const __grid_constant__ mel_dev d)
 {
     const int e = blockIdx.x * blockDim.x + threadIdx.x;
     if (e < d.ne) d.cp_cnt[e] = 0;
 }
 
-__global__ void pressure_push_kernel(mel_dev d)
+__global__ void pressure_push_kernel(const __grid_constant__ mel_dev d)
 {
     const int c = blockIdx.x * blockDim.x + threadIdx.x;
     if (c >= d.ncont) return;
@@ -1810,7 +1927,7 @@ __global__ void pressure_push_kernel(mel_dev d)
     pressure_push(d, eM + 1, (c << 2) | 2);
 }
 
-__global__ void pressure_sum_kernel(mel_dev d)
+__global__ void pressure_sum_kernel(const __grid_constant__ mel_dev d)
 {
     const int e = blockIdx.x * blockDim.x + threadIdx.x;
     if (e >= d.ne) return;
@@ -1852,7 +1969,7 @@ namespace mel {
 // Body::Update_damping_forces (Code/Body.h:1057-1154): each degree of freedom subtracts its terms
 // v_param(source) * c in matrix-entry order, the order the reference's loop over the entries adds
 // them in; one thread per degree of freedom
-__global__ void __launch_bounds__(256) damping_kernel(mel_dev d)
+__global__ void __launch_bounds__(256) damping_kernel(const __grid_constant__ mel_dev d)
 {
     const int k = blockIdx.x * blockDim.x + threadIdx.x;
     if (k >= 2 * d.nn) return;
@@ -1871,7 +1988,7 @@ namespace mel {
 // where the reference reads past its vector), then per degree of freedom the nodal term
 // -beta m (v - pv) followed by its stiffness terms -(v_param(source) - pv(source)) d in the
 // order the reference's entry loop adds them; a direction without history keeps a zero force
-__global__ void __launch_bounds__(256) alid_kernel(mel_dev d, int parity, double T, int use_T)
+__global__ void __launch_bounds__(256) alid_kernel(const __grid_constant__ mel_dev d, int parity, double T, int use_T)
 {
     const int b = d.alid_b[blockIdx.x];
     __shared__ double s_pv[2];
@@ -1930,11 +2047,10 @@ void mel_launch_czm_init(const mel_dev& d, cudaStream_t s)
     mel::contact_kernel<<<(d.ncont + 127) / 128, 128, 0, s>>>(d, 1.0, 1);
 }
 
-size_t mel_body_smem_bytes(int max_nodes, int max_image_bytes, int mixed, int stages)
+size_t mel_body_smem_bytes(int max_nodes, size_t stage, int mixed)
 {
-    size_t base = 3 * sizeof(double2) * (size_t)max_nodes + MEL_BAR_BYTES;
-    if (mixed) base += sizeof(float2) * (size_t)((max_nodes + 1) & ~1);
-    size_t stage = (size_t)stages * (size_t)max_image_bytes;
+    size_t base = sizeof(double2) * (3 * (size_t)max_nodes + 1) + MEL_BAR_BYTES;
+    if (mixed) base += sizeof(float2) * (size_t)((max_nodes + 2) & ~1);
     size_t post = (5 * sizeof(double2) + 6 * sizeof(double)) * (size_t)max_nodes;
     size_t rigid = (64 + 6 * MEL_RIGID_BATCH) * sizeof(double);
     size_t r = base + (stage > post ? stage : post);
@@ -1991,7 +2107,7 @@ namespace mel {
 // Body::Restore of a rigid body's own kinematics (Code/Body.h:2650-2658): current position,
 // displacement and velocity; its accelerations, driven values and mass-scaling factor are not
 // part of the snapshot
-__global__ void rigid_restore_kernel(mel_dev d, const double* rg_snap)
+__global__ void rigid_restore_kernel(const __grid_constant__ mel_dev d, const double* rg_snap)
 {
     const int b = blockIdx.x * blockDim.x + threadIdx.x;
     if (b >= d.nb || d.b_type[b] != MEL_BODY_RIGID) return;
@@ -2004,7 +2120,7 @@ __global__ void rigid_restore_kernel(mel_dev d, const double* rg_snap)
 
 namespace mel {
 // Update_bc(Time) of every body's driven borders (the set-up call of Code/main.cpp:104-127)
-__global__ void drivendof_kernel(mel_dev d, double T)
+__global__ void drivendof_kernel(const __grid_constant__ mel_dev d, double T)
 {
     const int b = blockIdx.x * blockDim.x + threadIdx.x;
     if (b < d.nb) body_drivendof(d, b, T, d.drv + 8 * (size_t)b);

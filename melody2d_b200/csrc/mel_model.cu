@@ -15,6 +15,7 @@
 #include "mel_internal.h"
 #include "mel_prox_host.h"
 #include "mel_chunks.h"
+#include "mel_tiles.h"
 #include "mel_material.h"
 #include "mel_host.h"   // .asc loader (mel_loader.cpp)
 #include "mel_sincos.h"
@@ -71,8 +72,7 @@ struct mel_handle {
     size_t body_smem = 0;
     int nblocks_body = 0;     // body-kernel CTAs, and the wide bodies' CTAs after them
     int nwide = 0;
-    int chunk_cap = 0;          // support entries per chunk chosen at build time
-    int body_stages = 2;        // image buffers per CTA (3 when a body runs the mixed pipeline)
+    int chunk_cap = 0;          // slots per tile chosen at build time
     double img_bytes = 0.;      // bytes of all chunk images
     long long n_pad = 0;        // padding entries in the chunk images
     int launches = 0;
@@ -255,7 +255,7 @@ static int tuned_chunk_cap(int precision, int max_nodes)
 {
     if (const char* c = getenv("MELGPU_CHUNK_CAP")) {
         const int v = atoi(c);
-        if (v >= 64 && v <= (precision == MEL_PREC_MIXED ? MEL_CHUNK_E_MAX_MX : MEL_CHUNK_E_MAX)) return v & ~7;
+        if (v >= 64 && v <= MEL_TILE_SLOTS_MAX) return (v + 127) & ~127;
     }
     const char* path = getenv("MELGPU_TUNE_FILE");
     if (!path) return 0;
@@ -266,15 +266,17 @@ static int tuned_chunk_cap(int precision, int max_nodes)
     while (fgets(line, sizeof line, f)) {
         if (line[0] == '#') continue;
         int p = -1, mn = 0, c = 0;
-        if (sscanf(line, "%d %d %d", &p, &mn, &c) == 3 && p == precision && max_nodes <= mn && c >= 64 &&
-            c <= (precision == MEL_PREC_MIXED ? MEL_CHUNK_E_MAX_MX : MEL_CHUNK_E_MAX)) {
-            cap = c & ~7;
+        if (sscanf(line, "%d %d %d", &p, &mn, &c) == 3 && p == precision && max_nodes <= mn && c >= 64 && c <= MEL_TILE_SLOTS_MAX) {
+            cap = (c + 127) & ~127;
             break;
         }
     }
     fclose(f);
     return cap;
 }
+
+// shared-memory bytes of a tile's contributions: `cap` slots and the zero slot that padding names
+static int tile_q(int cap, bool mixed) { return ((cap + 1) * (mixed ? 8 : 16) + 15) & ~15; }
 
 static mel_status build(mel_handle* h, const mel_model_desc* d, const mel_options* opt)
 {
@@ -712,92 +714,69 @@ static mel_status build(mel_handle* h, const mel_model_desc* d, const mel_option
         D.gscr = reinterpret_cast<char*>(dalloc<double>(h, (size_t)(tot / 8) + 32));
     }
     mel_chunk_set CS;
-    long long pipe_min = 0;
+    mel_tile_set TS;
     int smem_sm = 0, smem_blk = 0, smem_res = 0;
     cudaDeviceGetAttribute(&smem_sm, cudaDevAttrMaxSharedMemoryPerMultiprocessor, h->device);
     cudaDeviceGetAttribute(&smem_blk, cudaDevAttrMaxSharedMemoryPerBlockOptin, h->device);
     cudaDeviceGetAttribute(&smem_res, cudaDevAttrReservedSharedMemoryPerBlock, h->device);
     const size_t two_per_sm = (size_t)(smem_sm / 2 - smem_res);
+    const bool mixed = h->precision == MEL_PREC_MIXED;
     {
-        const bool mixed = h->precision == MEL_PREC_MIXED;
-        // which mixed bodies run the three-stage pipeline: those with at least pipe_min support
-        // entries (MELGPU_PIPE_MIN_ENTRIES overrides the default); the others run the two-buffer loop
-        if (mixed) {
-            pipe_min = MEL_PIPE_MIN_ENTRIES;
-            if (const char* e = getenv("MELGPU_PIPE_MIN_ENTRIES")) pipe_min = atoll(e);
-        }
-        bool any_pipe = false, any_loop = false;
-        for (int b = 0; b < nb; b++)
-            if (d->body_type[b] == MEL_BODY_DEFORMABLE) {
-                if (mixed && mel_body_entries(d, b) >= pipe_min) any_pipe = true; else any_loop = true;
-            }
-        const int stages = any_pipe ? MEL_STAGES(1) : 2;
-        // FP32 images hold 12 bytes per entry instead of 20; pipeline bodies have fewer point threads
-        const int gpcap = any_loop ? MEL_CHUNK_GP_FP64 : MEL_CHUNK_GP_MX;
-        const int caps_fp64[] = { MEL_CHUNK_E_MAX, 1792, 1536, 1408, 1344, 1280, 1216, 1152, 1024, 768, 512, 256 };
-        const int caps_mixed[] = { MEL_CHUNK_E_MAX, 1920, 1792, 1664, 1536, 1408, 1280, 1024, 768, 512, 256 };
-        std::vector<int> caps = mixed ? std::vector<int>(std::begin(caps_mixed), std::end(caps_mixed))
-                                      : std::vector<int>(std::begin(caps_fp64), std::end(caps_fp64));
-        // the cap is chosen from an upper bound of the image size (a chunk holds at most ecap
-        // entries, gpcap points, min(ecap, nodes) touched nodes and one row per support
-        // of each group's largest point), so the images are built once
-        // Pull rows: the first pull group has at most (the most points any node supports) rows,
-        // and each later group at most its predecessor's smallest count, so all later groups
-        // together at most ecap / 32.
-        int max_ns = 1, max_use = 1;
-        std::vector<int> use;
-        for (int b = 0; b < nb; b++)
-            if (d->body_type[b] == MEL_BODY_DEFORMABLE) {
-                use.assign(d->body_node_ptr[b + 1] - d->body_node_ptr[b], 0);
-                for (int g = d->body_gp_ptr[b]; g < d->body_gp_ptr[b + 1]; g++) {
-                    max_ns = std::max(max_ns, d->gp_sup_ptr[g + 1] - d->gp_sup_ptr[g]);
-                    for (int j = d->gp_sup_ptr[g]; j < d->gp_sup_ptr[g + 1]; j++) {
-                        const int v = d->gp_sup_idx[j];
-                        if (v >= 0 && v < (int)use.size()) max_use = std::max(max_use, ++use[v]);
-                    }
+        // slots per tile: MEL_TILE_SLOTS hold a full tile's points; fewer where the node arrays leave
+        // less room beside them for two CTAs per SM, and one CTA per SM for bodies too large for that.
+        // The tuning table (MELGPU_TUNE_FILE, written by melody2d_b200.autotune) or MELGPU_CHUNK_CAP
+        // (the tuner's own runs) name another number, taken when it fits the shared memory.
+        const int least = 256 * MEL_PLACES(mixed);
+        // shared memory of the tiles of a plan: contributions and a zero slot, index words, pull slots
+        auto stage = [&]() { return tile_q(TS.cap, mixed) + TS.max_idx + TS.max_pull; };
+        auto need = [&]() { return mel_body_smem_bytes(max_def_nodes, (size_t)stage(), mixed); };
+        auto plan = [&](int cap) { return mel_plan_tiles(d, cap, mixed, TS); };
+        mel_status rc = MEL_OK;
+        int cap = tuned_chunk_cap(h->precision, max_def_nodes);
+        if (cap > 0 && (rc = plan(std::max(cap, least))) != MEL_OK) return rc;
+        if (cap == 0 || need() > (size_t)smem_blk)
+            for (size_t room : { two_per_sm, (size_t)smem_blk }) {
+                for (cap = std::max(MEL_TILE_SLOTS, least); ; cap = std::max(cap - 256, least)) {
+                    if ((rc = plan(cap)) != MEL_OK) return rc;
+                    if (need() <= room || cap == least) break;
                 }
+                if (need() <= room) break;
             }
-        auto bound = [&](int ecap) {
-            const int ne = std::min(ecap, gpcap * max_ns);
-            const int groups = (gpcap + 31) / 32;
-            const int pull_rows = std::min(max_use, gpcap) + ne / 32;
-            // pull records: touched-node slots, or (mixed two-buffer loop) the segmented list
-            // pull records: touched-node slots, or (mixed two-buffer loop) the warp bounds and at most
-            // one piece per touched node plus one per MEL_PIECE entries
-            int tn_words = std::max(std::min(ne, max_all_nodes), mixed ? 5 + std::min(ne, max_all_nodes) + ne / MEL_PIECE : 0);
-            if (any_wide && !mixed) tn_words += (tn_words + 1) / 2 + 4;     // the 16-bit node section of wide bodies
-            return mel_chunk_sections(gpcap, ne, tn_words, std::min(1023, groups * max_ns) + pull_rows, mixed ? 8 : 16).bytes;
-        };
-        int chosen = -1;
-        // a cap from the tuning table (MELGPU_TUNE_FILE, written by melody2d_b200.autotune), or forced
-        // by MELGPU_CHUNK_CAP (the tuner's own runs), is taken when it fits the shared memory
-        const int tuned = tuned_chunk_cap(h->precision, max_def_nodes);
-        if (tuned > 0 && mel_body_smem_bytes(max_def_nodes, bound(tuned), mixed, stages) <= (size_t)smem_blk) chosen = tuned;
-        if (chosen < 0)
-            for (int ecap : caps)
-                if (mel_body_smem_bytes(max_def_nodes, bound(ecap), mixed, stages) <= two_per_sm) { chosen = ecap; break; }
-        if (chosen < 0)     // one CTA per SM: largest cap that fits
-            for (int ecap : caps)
-                if (mel_body_smem_bytes(max_def_nodes, bound(ecap), mixed, stages) <= (size_t)smem_blk) { chosen = ecap; break; }
-        if (chosen < 0) {
+        if (need() > (size_t)smem_blk) {
             mel_set_error("deformable body of %d nodes does not fit the body kernel's shared memory", max_def_nodes);
             return MEL_ERR_UNSUPPORTED;
         }
-        mel_status rc = mel_build_chunks(d, chosen, CS, mixed, pipe_min);
-        if (rc) return rc;
-        h->chunk_cap = chosen;
+        if ((rc = mel_fill_tiles(d, TS)) != MEL_OK) return rc;
+        h->chunk_cap = TS.cap;
+        h->body_smem = need();
+        D.tile_cap = TS.cap;
+        D.tile_q = tile_q(TS.cap, mixed);
+        D.tile_i = TS.max_idx;
+        D.tile_pad = (unsigned long long)TS.cap * 0x0001000100010001ull;
     }
-    h->nge = (int)CS.n_entries;
+    if (any_wide) {
+        // chunk images of the wide bodies: the largest entry cap whose two buffers leave room for two
+        // CTAs per SM (FP32 images hold 12 bytes an entry instead of 20)
+        for (int ecap : { MEL_CHUNK_E_MAX, 1792, 1536, 1280, 1024, 768, 512, 256 }) {
+            mel_status rc = mel_build_chunks(d, ecap, CS, mixed, 0, MEL_MAX_BODY_NODES);
+            if (rc) return rc;
+            if (MEL_BAR_BYTES + 2 * (size_t)CS.img_max <= two_per_sm) break;
+        }
+        h->body_smem = std::max(h->body_smem, MEL_BAR_BYTES + 2 * (size_t)CS.img_max);
+    }
+    h->nge = (int)(TS.n_entries + CS.n_entries);
     h->n_pad = CS.n_pad;
-    D.nchunk = (int)CS.chunks.size();
-    D.chunk = dupload(h, CS.chunks);
-    D.b_chunk0 = dupload(h, CS.b_chunk0);
-    D.img = reinterpret_cast<const char*>(dupload(h, CS.img));
-    D.img_cap = CS.img_max;
-    if (h->precision == MEL_PREC_MIXED) D.b_pipe = dupload(h, CS.b_pipe);
-    h->body_stages = 2;
-    for (int v : CS.b_pipe) if (v) h->body_stages = MEL_STAGES(1);
-    h->img_bytes = (double)CS.img.size();
+    D.tile = dupload(h, TS.tiles);
+    D.b_tile0 = dupload(h, TS.b_tile0);
+    D.timg = reinterpret_cast<const char*>(dupload(h, TS.data, TS.bytes));
+    if (any_wide) {
+        D.nchunk = (int)CS.chunks.size();
+        D.chunk = dupload(h, CS.chunks);
+        D.b_chunk0 = dupload(h, CS.b_chunk0);
+        D.img = reinterpret_cast<const char*>(dupload(h, CS.img));
+        D.img_cap = CS.img_max;
+        h->img_bytes = (double)CS.img.size();
+    }
     // contacts and proximity buffers
     D.err = dalloc<unsigned>(h, MEL_E_NWORDS);
     D.ncont = 0;
@@ -870,7 +849,6 @@ static mel_status build(mel_handle* h, const mel_model_desc* d, const mel_option
     if (cudaMalloc(&P.inc_rng, sizeof(int2) * 16) != cudaSuccess) return MEL_ERR_OOM;
     P.inc_rng_bytes = sizeof(int2) * 16;
     D.inc_rng = P.inc_rng;
-    h->body_smem = mel_body_smem_bytes(max_def_nodes, CS.img_max, h->precision == MEL_PREC_MIXED, h->body_stages);
     if (mel_body_kernel_configure(h->body_smem) != MEL_OK) return MEL_ERR_CUDA;
     h->d_monitor = dalloc<double>(h, 32);
     h->d_monitor_part = dalloc<double>(h, 5 * 148);
@@ -881,9 +859,8 @@ static mel_status build(mel_handle* h, const mel_model_desc* d, const mel_option
         h->d_rigid_ids = dupload(h, rid);
     }
     // algorithmic bytes moved by one launch of each step kernel (exact array sizes):
-    // body kernel: the chunk images without their padding entries (entries: dN/dx,dN/dy + 16-bit
-    // index + 16-bit pull position; points: c0 + slot record; touched-node records; row tables)
-    // and the chunk table; node state read (up,
+    // body kernel: the tiles without their padding (entries: dN/dx,dN/dy + 16-bit index + 16-bit pull
+    // position; point and touched-node records; the tile table) and the wide bodies' chunk images; node state read (up,
     // vp, m, 1/m, X0) and written (up, vp, ap, u, v, a, x); node supports (16-bit index + N) and
     // their offsets.  Contact records are left out (a few hundred bytes per body).
     {
@@ -894,8 +871,10 @@ static mel_status build(mel_handle* h, const mel_model_desc* d, const mel_option
         for (int b = 0; b < nb; b++)
             if (d->body_type[b] == MEL_BODY_DEFORMABLE)
                 nse_def += d->node_sup_ptr[d->body_node_ptr[b + 1]] - d->node_sup_ptr[d->body_node_ptr[b]];
-        const double entry_bytes = h->precision == MEL_PREC_MIXED ? 12. : 20.;
-        h->bytes_body = h->img_bytes - entry_bytes * (double)h->n_pad + (double)CS.chunks.size() * sizeof(mel_chunk) + nd * (5 * 16 + 7 * 16) +
+        const double entry_bytes = mixed ? 12. : 20.;
+        h->bytes_body = entry_bytes * (double)TS.n_entries + (double)TS.n_points * sizeof(mel_point) + (double)TS.n_pull * sizeof(mel_pull) +
+                        (double)TS.tiles.size() * sizeof(mel_tile) +
+                        h->img_bytes - entry_bytes * (double)h->n_pad + (double)CS.chunks.size() * sizeof(mel_chunk) + nd * (5 * 16 + 7 * 16) +
                         nse_def * (2 + 8) + (nd + 1) * 4;
         h->bytes_contact = (double)ne * (4 * 4 + 4 * 4 + 8 + 8);   // refreshed border lengths (contacts added per call)
     }
