@@ -58,6 +58,12 @@ __device__ __forceinline__ double entry_length(const mel_dev& d, int b, int g, i
     return d.e_len0[d.bd_e0[g] + j];
 }
 
+// Programmatic dependent launch of the step's kernels.  grid_wait: what the kernels before this one
+// wrote is there from here on (nothing to wait for in an ordinary launch); grid_release: the next
+// kernel of the stream may start.
+__device__ __forceinline__ void grid_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void grid_release() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+
 // ------------------------------------------------------------------------------------------
 // contact kernel
 // ------------------------------------------------------------------------------------------
@@ -1239,7 +1245,10 @@ __device__ void deformable_body(const mel_dev& d, int b, double T, double T0, ch
         if (warp < MEL_BODY_CTHREADS / 32) {
             if constexpr (MX) tile_forces<true>(d, b, s_upf, s_f, region, s_bar, s_abort, tid, lane, warp);
             else tile_forces<false>(d, b, s_up, s_f, region, s_bar, s_abort, tid, lane, warp);
-        } else contact_scatter(d, b, n0, s_fc, lane);      // warp 7, meanwhile
+        } else {                                           // warp 7, meanwhile
+            grid_wait();
+            contact_scatter(d, b, n0, s_fc, lane);
+        }
         __syncthreads();
         if (*s_abort) return;
     }
@@ -1537,6 +1546,7 @@ __device__ void rigid_body(const mel_dev& d, int b, double T, double T0, char* s
     // loads from memory for each ---------------------------------------------------------------
     double con = 0.;
     const int kcon = tid - 8;
+    grid_wait();
     {
         const int c0 = d.b_cont0[b], nown = d.b_cont0[b + 1] - c0;
         for (int w0 = 0; w0 < nown; w0 += MEL_RIGID_STAGE) {
@@ -1722,7 +1732,7 @@ __device__ __forceinline__ void body_cta(const mel_dev& d, int bb, double T, cha
 {
     int b = d.b_order[bb];
     if (d.b_status[b] == MEL_STATUS_INACTIVE) return;
-    if (d.any_damped && threadIdx.x == 32) contact_work(d, b);
+    if (d.any_damped && threadIdx.x == 32) { grid_wait(); contact_work(d, b); }
     if (d.b_type[b] == MEL_BODY_RIGID) rigid_body<AD>(d, b, T, T0, smem);
     else deformable_body<MX, AD, false>(d, b, T, T0, smem);
 }
@@ -1739,8 +1749,17 @@ __device__ __forceinline__ void wide_body_cta(const mel_dev& d, int bb, double T
     deformable_body<MX, AD, true>(d, b, T, T0, smem);
 }
 
+// The step's two kernels overlap (programmatic dependent launch).  The contact pass is a chain of
+// dependent loads, 13 to 17 us long whatever the sample's size, and the Gauss-point pass does not
+// need its results: the body kernel starts beside it and waits (grid_wait) where it reads contact
+// forces, and before any CTA writes the positions and velocities that the contact pass reads.  The
+// contact pass waits for the body kernel before it, and only then lets the next one start, so that
+// no two body kernels ever run together.  Measured on B200, a step: 4x4 lattice 68 -> 61 us, 50 grains
+// FP64 127 -> 116 us, 700 grains FP64 251 -> 235 us, mixed 215 -> 200 us.
 __global__ void __launch_bounds__(128) contact_kernel(const __grid_constant__ mel_dev d, double law_dt_scale, int czm_init)
 {
+    grid_wait();
+    grid_release();
     contact_thread(d, blockIdx.x * blockDim.x + threadIdx.x, law_dt_scale, czm_init);
 }
 
@@ -1750,8 +1769,10 @@ template <bool MX>
 __global__ void __launch_bounds__(MEL_BODY_THREADS, 2) body_kernel(const __grid_constant__ mel_dev d, int parity)
 {
     extern __shared__ __align__(16) char smem[];
+    grid_release();
     const double T = d.time2[parity];
     body_cta<MX>(d, blockIdx.x, T, smem);
+    grid_wait();          // a CTA that had nothing to wait for ends no earlier than the contact pass
     if (blockIdx.x == 0 && threadIdx.x == 0) d.time2[parity ^ 1] = T + d.dt[0];
 }
 
@@ -1821,6 +1842,8 @@ __device__ __forceinline__ int batch_member(const int* prefix, int nsamp, int i)
 __global__ void __launch_bounds__(128) contact_kernel_batch(const mel_dev* devs, const int* thr0, int nsamp,
                                                             double law_dt_scale)
 {
+    grid_wait();
+    grid_release();
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= thr0[nsamp]) return;
     const int s = batch_member(thr0, nsamp, i);
@@ -1842,6 +1865,7 @@ __global__ void __launch_bounds__(MEL_BODY_THREADS, 2) body_kernel_batch(const m
     }
     __syncthreads();
     body_cta<MX>(sd, c - cta0[s], sd.time2[0], smem);
+    grid_wait();
 }
 
 __global__ void advance_kernel(const mel_dev* devs, int nsamp)
@@ -2034,11 +2058,25 @@ void mel_launch_damping(const mel_dev& d, cudaStream_t s)
     mel::damping_kernel<<<(2 * d.nn + 255) / 256, 256, 0, s>>>(d);
 }
 
+// launch that may start as soon as the kernel before it in the stream releases it
+template <class... P, class... A>
+static void launch_dependent(void (*k)(P...), int grid, int block, size_t smem, cudaStream_t s, A... args)
+{
+    cudaLaunchConfig_t c = {};
+    cudaLaunchAttribute a = {};
+    a.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    a.val.programmaticStreamSerializationAllowed = 1;
+    c.gridDim = dim3((unsigned)grid); c.blockDim = dim3((unsigned)block);
+    c.dynamicSmemBytes = smem; c.stream = s;
+    c.attrs = &a; c.numAttrs = 1;
+    cudaLaunchKernelEx(&c, k, static_cast<P>(args)...);      // errors: cudaGetLastError by the caller, as for <<<>>>
+}
+
 void mel_launch_contact(const mel_dev& d, double law_dt_scale, cudaStream_t s)
 {
     int total = d.ncont + d.ne;
     if (total <= 0) return;
-    mel::contact_kernel<<<(total + 127) / 128, 128, 0, s>>>(d, law_dt_scale, 0);
+    launch_dependent(mel::contact_kernel, (total + 127) / 128, 128, 0, s, d, law_dt_scale, 0);
 }
 
 void mel_launch_czm_init(const mel_dev& d, cudaStream_t s)
@@ -2060,15 +2098,19 @@ size_t mel_body_smem_bytes(int max_nodes, size_t stage, int mixed)
 void mel_launch_batch_step(const mel_dev* devs, const int* thr0, int nthr, const int* cta0, int ncta_small, int ncta,
                            int nsamp, int mixed, size_t smem_small, size_t smem, cudaStream_t s)
 {
-    if (nthr > 0) mel::contact_kernel_batch<<<(nthr + 127) / 128, 128, 0, s>>>(devs, thr0, nsamp, 1.0);
+    if (nthr > 0) launch_dependent(mel::contact_kernel_batch, (nthr + 127) / 128, 128, 0, s, devs, thr0, nsamp, 1.0);
+    // the first body launch overlaps the contact pass; the second follows it in the ordinary way
+    auto body = mixed ? mel::body_kernel_batch<true> : mel::body_kernel_batch<false>;
+    bool after_contact = nthr > 0;
     // members whose bodies fit two CTAs per SM first, in their own launch, then the others
     if (ncta_small > 0) {
-        if (mixed) mel::body_kernel_batch<true><<<ncta_small, MEL_BODY_THREADS, smem_small, s>>>(devs, cta0, nsamp, 0);
-        else mel::body_kernel_batch<false><<<ncta_small, MEL_BODY_THREADS, smem_small, s>>>(devs, cta0, nsamp, 0);
+        if (after_contact) launch_dependent(body, ncta_small, MEL_BODY_THREADS, smem_small, s, devs, cta0, nsamp, 0);
+        else body<<<ncta_small, MEL_BODY_THREADS, smem_small, s>>>(devs, cta0, nsamp, 0);
+        after_contact = false;
     }
     if (ncta > ncta_small) {
-        if (mixed) mel::body_kernel_batch<true><<<ncta - ncta_small, MEL_BODY_THREADS, smem, s>>>(devs, cta0, nsamp, ncta_small);
-        else mel::body_kernel_batch<false><<<ncta - ncta_small, MEL_BODY_THREADS, smem, s>>>(devs, cta0, nsamp, ncta_small);
+        if (after_contact) launch_dependent(body, ncta - ncta_small, MEL_BODY_THREADS, smem, s, devs, cta0, nsamp, ncta_small);
+        else body<<<ncta - ncta_small, MEL_BODY_THREADS, smem, s>>>(devs, cta0, nsamp, ncta_small);
     }
     mel::advance_kernel<<<(nsamp + 127) / 128, 128, 0, s>>>(devs, nsamp);
 }
@@ -2076,8 +2118,11 @@ void mel_launch_batch_step(const mel_dev* devs, const int* thr0, int nthr, const
 void mel_launch_body(const mel_dev& d, int parity, int nblocks, size_t smem, cudaStream_t s, int nwide)
 {
     if (nblocks > 0) {
-        if (d.precision == MEL_PREC_MIXED) mel::body_kernel<true><<<nblocks, MEL_BODY_THREADS, smem, s>>>(d, parity);
-        else mel::body_kernel<false><<<nblocks, MEL_BODY_THREADS, smem, s>>>(d, parity);
+        auto body = d.precision == MEL_PREC_MIXED ? mel::body_kernel<true> : mel::body_kernel<false>;
+        // beside the contact pass where this step has one (without it the kernel before this one is
+        // the last step's body kernel, which lets its successor start at once)
+        if (d.ncont + d.ne > 0) launch_dependent(body, nblocks, MEL_BODY_THREADS, smem, s, d, parity);
+        else body<<<nblocks, MEL_BODY_THREADS, smem, s>>>(d, parity);
     }
     if (nwide > 0) {
         const int set_time = nblocks > 0 ? 0 : 1;
