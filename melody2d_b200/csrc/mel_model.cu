@@ -828,14 +828,11 @@ static mel_status build(mel_handle* h, const mel_model_desc* d, const mel_option
         }
     }
     P.b_inc0 = dalloc<int>(h, nb + 1);
-    P.tcnt = dalloc<int>(h, nb + 1);
+    P.inc_cnt = dalloc<int>(h, nb + 1);
     P.btask0 = dalloc<int>(h, nb + 2);
-    P.scnt = dalloc<int>(h, nb + 1);
+    P.ncand = dalloc<int>(h, 1);
     P.bslot0 = dalloc<int>(h, nb + 2);
     P.b_cont0 = dalloc<int>(h, nb + 1);
-    P.e_cnt = dalloc<int>(h, ne + 1);
-    P.e_ptr = dalloc<int>(h, ne + 2);
-    P.e_cur = dalloc<int>(h, ne + 2);
     size_t cb = sizeof(mel_contact) * 1024;
     if (cudaMalloc(&D.cont, cb) != cudaSuccess) return MEL_ERR_OOM;
     P.cont_bytes = cb;
@@ -1246,10 +1243,8 @@ mel_status mel_destroy(mel_handle* h)
     if (h->stream) cudaStreamSynchronize(h->stream);
     for (void* p : h->allocs) cudaFree(p);
     mel_prox_state& P = h->P;
-    for (void* p : { (void*)P.nbr, (void*)P.task, (void*)P.inc_task, (void*)P.slot_cnt, (void*)P.slot_off, (void*)P.tmap, (void*)P.nzoff, (void*)P.nzlist, (void*)P.inc_rng,
-                     (void*)P.scan_ws,
-                     (void*)P.tns, (void*)P.tslot, (void*)P.tkey,
-                     (void*)P.e_list, (void*)P.cont_alt, (void*)P.cont_w, (void*)P.cont_rt, (void*)h->d.cont })
+    for (void* p : { (void*)P.nbr, (void*)P.cand, (void*)P.tcand, (void*)P.toff, (void*)P.tkey, (void*)P.bucket, (void*)P.inc_task,
+                     (void*)P.inc_rng, (void*)P.scan_ws, (void*)P.cont_alt, (void*)P.cont_w, (void*)P.cont_rt, (void*)h->d.cont })
         if (p) cudaFree(p);
     mel_prox_stage_free(P.stage);
     if (h->ck.side) { cudaStreamSynchronize(h->ck.side); cudaStreamDestroy(h->ck.side); }

@@ -2,24 +2,32 @@
 // (the members of a batch) with the same launches.
 //
 // Stages (all integer bookkeeping deterministic, geometry bit-identical to the reference):
-//   aabb_kernel        border boxes inflated by the detection distance and their period shifts
-//                      (Code/Proximity.h:63-109), one warp per border; segment-block and
-//                      superblock boxes for pruning
-//   neighbour_kernel   all-pairs (body, border) overlap with periodic shifts and de-duplication
-//                      (Code/Proximity.h:112-169), one warp per body, lanes over candidate bodies
-//   task_count / scan / task_fill   task list: one task per (slave body, slave border, neighbour)
-//                      in the reference's loop order, then one self task per (slave body, border);
-//                      a slot per (task, slave border node)
+//   boxes_kernel       border boxes inflated by the detection distance and their period shifts
+//                      (Code/Proximity.h:63-109), one warp per border; segment-block and superblock
+//                      boxes for pruning, one warp per superblock
+//   neighbour_kernel or cl_*   (body, border) overlap with periodic shifts and de-duplication
+//                      (Code/Proximity.h:112-169), one warp per body
+//   tasks_kernel       tasks and slots per body and their offsets: one task per (slave body, slave
+//                      border, neighbour) in the reference's loop order, then one self task per (slave
+//                      body, border); a slot per (task, slave border node)
 //   [host read-back]   task and slot totals of every member
-//   count_kernel       accepted candidates per slot, one thread per slot (slot_task_kernel maps
-//                      slots to tasks)
-//   scan               slot offsets = the canonical position of every new contact element; the
-//                      slots with candidates are listed for the write pass
+//   find_kernel        accepted candidates: a thread per slot tests the master's boxes, then a warp per
+//                      slot that is near one tests the segments; candidates are listed in any order
+//                      and counted per task
+//   scan               task offsets in the new list
 //   [host read-back]   contact totals of every member
-//   write_kernel       writes the new list in the reference's order; history inheritance searches
-//                      the previous list of the same slave border node (Code/Proximity.h:269-284)
-//   incoming ranges, entry index, vgap carry   index structures for the next step and update
-// Every kernel reads a table of member jobs (mel_prox_job); the host driver is at the end.
+//   bucket_kernel, write_kernel   the candidates by task; one warp per candidate finds its place in
+//                      the task (slave border node, then segment order, the reference's) and writes the
+//                      contact element, with the history of the first matching old element of the
+//                      same slave border node (Code/Proximity.h:269-284)
+//   inc_fill_kernel, bodies_kernel   incoming ranges, contact ranges and the vgap carry per body
+// Every kernel reads a table of member jobs (mel_prox_job), or its own argument when there is one
+// member; the host driver is at the end.
+//
+// What bounds it: latency.  A run is some fifteen short launches, each a chain of dependent loads.
+// Measured on B200, an update with its launch gaps and read-backs: 4x4 lattice 370 -> 123 us, 50
+// grains 486 -> 166 us, 700 grains 582 -> 216 us, against forty launches in which a thread per slot
+// walked its segments itself, once to count (68 us) and once to write (155 us).
 #include <cstdio>
 #include <cstring>
 #include <utility>
@@ -34,10 +42,15 @@ struct mel_scan_job { const int* in; int* out; int n; int* sums; };
 namespace mel {
 
 // ---------------------------------------------------------------------------------------------
-// exclusive scans of int arrays, several per launch (three-phase, deterministic).  Job j scans
-// in[0..n) into out[0..n] (out[n] = total); blocks [bpre[j], bpre[j+1]) of a launch serve job j.
+// exclusive scans of int arrays, several per launch (deterministic; one launch up to SCAN_ITEMS
+// entries, three above).  Job j scans in[0..n) into out[0..n] (out[n] = total); blocks [bpre[j],
+// bpre[j+1]) of a launch serve job j.  A few jobs travel as the kernel's argument.
 // ---------------------------------------------------------------------------------------------
 #define SCAN_BLOCK 1024
+#define SCAN_PER 8
+#define SCAN_ITEMS (SCAN_BLOCK * SCAN_PER)
+#define SCAN_INLINE 4
+struct scan_args { const mel_scan_job* J; const int* bpre; int nj; mel_scan_job job[SCAN_INLINE]; int pre[SCAN_INLINE + 1]; };
 __device__ __forceinline__ int block_job(const int* bpre, int nj)
 {
     int lo = 0, hi = nj;                  // largest j with bpre[j] <= blockIdx.x
@@ -45,34 +58,46 @@ __device__ __forceinline__ int block_job(const int* bpre, int nj)
     return lo;
 }
 
-__global__ void __launch_bounds__(SCAN_BLOCK) scan_block_kernel(const mel_scan_job* J, const int* bpre, int nj)
+// exclusive prefix of v over the block and the block's total; s: one int per warp
+__device__ __forceinline__ int block_scan(int v, int* s, int& total)
 {
-    __shared__ int s[SCAN_BLOCK];
-    const int j = block_job(bpre, nj);
-    const int* in = J[j].in;
-    int* out = J[j].out;
-    const int n = J[j].n;
-    const int lb = blockIdx.x - bpre[j];
-    int i = lb * SCAN_BLOCK + threadIdx.x;
-    int v = (i < n) ? in[i] : 0;
-    s[threadIdx.x] = v;
-    __syncthreads();
-    for (int off = 1; off < SCAN_BLOCK; off <<= 1) {
-        int t = (threadIdx.x >= off) ? s[threadIdx.x - off] : 0;
-        __syncthreads();
-        s[threadIdx.x] += t;
-        __syncthreads();
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
+    int incl = v;
+    for (int o = 1; o < 32; o <<= 1) {
+        const int t = __shfl_up_sync(0xffffffffu, incl, o);
+        if (lane >= o) incl += t;
     }
-    if (i <= n) out[i] = s[threadIdx.x] - v;
-    if (threadIdx.x == SCAN_BLOCK - 1) J[j].sums[lb] = s[threadIdx.x];
+    __syncthreads();
+    if (lane == 31) s[warp] = incl;
+    __syncthreads();
+    int before = 0;
+    total = 0;
+    for (int w = 0; w < nw; w++) { if (w < warp) before += s[w]; total += s[w]; }
+    return before + incl - v;
+}
+
+__global__ void __launch_bounds__(SCAN_BLOCK) scan_block_kernel(const __grid_constant__ scan_args A)
+{
+    __shared__ int s[SCAN_BLOCK / 32];
+    const int j = block_job(A.J ? A.bpre : A.pre, A.nj);
+    const mel_scan_job job = A.J ? A.J[j] : A.job[j];
+    const int lb = blockIdx.x - (A.J ? A.bpre : A.pre)[j];
+    const int i0 = lb * SCAN_ITEMS + threadIdx.x * SCAN_PER;
+    int v[SCAN_PER], sum = 0;
+#pragma unroll
+    for (int k = 0; k < SCAN_PER; k++) { v[k] = i0 + k < job.n ? job.in[i0 + k] : 0; sum += v[k]; }
+    int total, at = block_scan(sum, s, total);
+#pragma unroll
+    for (int k = 0; k < SCAN_PER; k++) { if (i0 + k <= job.n) job.out[i0 + k] = at; at += v[k]; }
+    if (threadIdx.x == SCAN_BLOCK - 1) job.sums[lb] = total;
 }
 // adds the scanned block totals (in) to out[0..n) block by block
-__global__ void __launch_bounds__(SCAN_BLOCK) scan_add_kernel(const mel_scan_job* J, const int* bpre, int nj)
+__global__ void __launch_bounds__(SCAN_BLOCK) scan_add_kernel(const __grid_constant__ scan_args A)
 {
-    const int j = block_job(bpre, nj);
-    const int lb = blockIdx.x - bpre[j];
-    int i = lb * SCAN_BLOCK + threadIdx.x;
-    if (i < J[j].n) J[j].out[i] += J[j].in[lb];
+    const int j = block_job(A.J ? A.bpre : A.pre, A.nj);
+    const mel_scan_job job = A.J ? A.J[j] : A.job[j];
+    const int lb = blockIdx.x - (A.J ? A.bpre : A.pre)[j];
+    for (int i = lb * SCAN_ITEMS + threadIdx.x; i < min((lb + 1) * SCAN_ITEMS, job.n); i += SCAN_BLOCK) job.out[i] += job.in[lb];
 }
 
 } // namespace mel
@@ -89,13 +114,23 @@ __device__ __forceinline__ void aabb_item(const mel_dev& d, double* aabb, int* s
     int n0 = d.b_node0[b];
     double xmin = 1.e100, xmax = -1.e100, ymin = 1.e100, ymax = -1.e100;
     bool nonfinite = false;          // the comparisons below pass over NaN, so it is tested apart
-    for (int e = d.bd_e0[g] + lane; e < d.bd_e0[g + 1]; e += 32) {
-        double2 p = d.x[n0 + d.e_node[e]];
-        nonfinite |= !isfinite(p.x) || !isfinite(p.y);
-        if (p.x - dd < xmin) xmin = p.x - dd;
-        if (p.x + dd > xmax) xmax = p.x + dd;
-        if (p.y - dd < ymin) ymin = p.y - dd;
-        if (p.y + dd > ymax) ymax = p.y + dd;
+    const int e1 = d.bd_e0[g + 1];
+    for (int e = d.bd_e0[g] + lane; e < e1; e += 8 * 32) {      // eight entries in flight a lane
+        int nd[8];
+        double2 p[8];
+#pragma unroll
+        for (int k = 0; k < 8; k++) nd[k] = e + 32 * k < e1 ? d.e_node[e + 32 * k] : -1;
+#pragma unroll
+        for (int k = 0; k < 8; k++) p[k] = nd[k] >= 0 ? d.x[n0 + nd[k]] : make_double2(0., 0.);
+#pragma unroll
+        for (int k = 0; k < 8; k++) {
+            if (nd[k] < 0) continue;
+            nonfinite |= !isfinite(p[k].x) || !isfinite(p[k].y);
+            if (p[k].x - dd < xmin) xmin = p[k].x - dd;
+            if (p[k].x + dd > xmax) xmax = p[k].x + dd;
+            if (p[k].y - dd < ymin) ymin = p[k].y - dd;
+            if (p[k].y + dd > ymax) ymax = p[k].y + dd;
+        }
     }
     for (int o = 16; o > 0; o >>= 1) {
         xmin = fmin(xmin, __shfl_xor_sync(0xffffffffu, xmin, o));
@@ -427,43 +462,55 @@ __device__ __forceinline__ void cl_neighbour_item(const mel_prox_job& j, int b1,
 // Detect_Segment_Proximity; the boxes are widened by the detection distance plus a margin, so the
 // accepted candidates and their order are unchanged.
 // ---------------------------------------------------------------------------------------------
-__device__ __forceinline__ void segblock_item(const mel_dev& d, int k)
-{
-    if (k >= d.nblk) return;
-    int g = d.blk_border[k];
-    int b = d.bd_body[g];
-    int e0 = d.bd_e0[g];
-    int nseg = d.bd_e0[g + 1] - e0 - 1;
-    int s0 = (k - d.bd_blk0[g]) * MEL_SEGB;
-    int s1 = min(s0 + MEL_SEGB, nseg);
-    int n0 = d.b_node0[b];
-    double xmin = 1.e300, xmax = -1.e300, ymin = 1.e300, ymax = -1.e300;
-    for (int sg = s0; sg < s1; sg++) {
-        int e = e0 + sg;
-        for (int j = 1; j <= 2; j++) {
-            // shifted (regular search) and unshifted (self search) abscissae both count
-            double2 p = d.x[n0 + d.e_sn[4 * e + j]];
-            double x = p.x + d.period * d.e_ss[4 * e + j];
-            xmin = fmin(xmin, fmin(x, p.x)); xmax = fmax(xmax, fmax(x, p.x));
-            ymin = fmin(ymin, p.y); ymax = fmax(ymax, p.y);
-        }
-    }
-    d.seg_blk[k] = make_double4(xmin, xmax, ymin, ymax);
-}
-
-// superblock boxes: unions of MEL_SEGB2 consecutive block boxes of one border
-__device__ __forceinline__ void superblock_item(const mel_dev& d, int k)
+// Superblock boxes are unions of MEL_SEGB2 consecutive block boxes of one border.  One warp per
+// superblock, a half-warp per block and a lane per segment.
+static_assert(MEL_SEGB == 16 && MEL_SEGB2 == 16, "a half-warp serves a block of 16 segments, 16 blocks a superblock");
+__device__ __forceinline__ void superblock_item(const mel_dev& d, int k, int lane)
 {
     if (k >= d.nsblk) return;
-    int g = d.sblk_border[k];
-    int b0 = d.bd_blk0[g] + (k - d.bd_sblk0[g]) * MEL_SEGB2;
-    int b1 = min(b0 + MEL_SEGB2, d.bd_blk0[g + 1]);
-    double4 u = make_double4(1.e300, -1.e300, 1.e300, -1.e300);
-    for (int j = b0; j < b1; j++) {
-        double4 bb = d.seg_blk[j];
-        u.x = fmin(u.x, bb.x); u.y = fmax(u.y, bb.y); u.z = fmin(u.z, bb.z); u.w = fmax(u.w, bb.w);
+    const int g = d.sblk_border[k];
+    const int n0 = d.b_node0[d.bd_body[g]];
+    const int e0 = d.bd_e0[g], nseg = d.bd_e0[g + 1] - e0 - 1;
+    const int kb0 = (k - d.bd_sblk0[g]) * MEL_SEGB2, nb = min(MEL_SEGB2, d.bd_blk0[g + 1] - d.bd_blk0[g] - kb0);
+    double ux0 = 1.e300, ux1 = -1.e300, uy0 = 1.e300, uy1 = -1.e300;
+    for (int i = 0; i < nb; i += 8) {           // four blocks in flight a half-warp
+        double2 p[8];
+        double xs[8];
+        bool on[4];
+#pragma unroll
+        for (int q = 0; q < 4; q++) {
+            const int kb = i + 2 * q + (lane >> 4), sg = (kb0 + kb) * MEL_SEGB + (lane & 15);
+            on[q] = kb < nb && sg < nseg;
+#pragma unroll
+            for (int j = 0; j < 2; j++) {
+                // shifted (regular search) and unshifted (self search) abscissae both count
+                const int e = 4 * (e0 + sg) + 1 + j;
+                p[2 * q + j] = on[q] ? d.x[n0 + d.e_sn[e]] : make_double2(0., 0.);
+                xs[2 * q + j] = on[q] ? p[2 * q + j].x + d.period * d.e_ss[e] : 0.;
+            }
+        }
+#pragma unroll
+        for (int q = 0; q < 4; q++) {
+            double x0 = 1.e300, x1 = -1.e300, y0 = 1.e300, y1 = -1.e300;
+            if (on[q])
+#pragma unroll
+                for (int j = 0; j < 2; j++) {
+                    const double2 v = p[2 * q + j];
+                    x0 = fmin(x0, fmin(xs[2 * q + j], v.x)); x1 = fmax(x1, fmax(xs[2 * q + j], v.x));
+                    y0 = fmin(y0, v.y); y1 = fmax(y1, v.y);
+                }
+            for (int o = 8; o > 0; o >>= 1) {
+                x0 = fmin(x0, __shfl_xor_sync(0xffffffffu, x0, o)); x1 = fmax(x1, __shfl_xor_sync(0xffffffffu, x1, o));
+                y0 = fmin(y0, __shfl_xor_sync(0xffffffffu, y0, o)); y1 = fmax(y1, __shfl_xor_sync(0xffffffffu, y1, o));
+            }
+            const int kb = i + 2 * q + (lane >> 4);
+            if ((lane & 15) == 0 && kb < nb) d.seg_blk[d.bd_blk0[g] + kb0 + kb] = make_double4(x0, x1, y0, y1);
+            ux0 = fmin(ux0, x0); ux1 = fmax(ux1, x1); uy0 = fmin(uy0, y0); uy1 = fmax(uy1, y1);
+        }
     }
-    d.seg_sblk[k] = u;
+    ux0 = fmin(ux0, __shfl_xor_sync(0xffffffffu, ux0, 16)); ux1 = fmax(ux1, __shfl_xor_sync(0xffffffffu, ux1, 16));
+    uy0 = fmin(uy0, __shfl_xor_sync(0xffffffffu, uy0, 16)); uy1 = fmax(uy1, __shfl_xor_sync(0xffffffffu, uy1, 16));
+    if (lane == 0) d.seg_sblk[k] = make_double4(ux0, ux1, uy0, uy1);
 }
 
 __device__ __forceinline__ bool block_may_detect(const double4& bb, double xs, double ys, double m)
@@ -471,312 +518,303 @@ __device__ __forceinline__ bool block_may_detect(const double4& bb, double xs, d
     return !(xs < bb.x - m || xs > bb.y + m || ys < bb.z - m || ys > bb.w + m);
 }
 
-// Calls body(kb) for each block kb (border-local index) of border g whose superblock box and
-// block box both lie within `margin` of (x, y), in ascending block order.
-template <typename F>
-__device__ __forceinline__ void for_near_blocks(const mel_dev& d, int g, double x, double y, double margin, F&& body)
+// whether any block box of border g lies within `margin` of (x, y)
+__device__ __forceinline__ bool any_near_block(const mel_dev& d, int g, double x, double y, double margin)
 {
     const int blk0 = d.bd_blk0[g], blk1 = d.bd_blk0[g + 1];
     for (int ks = d.bd_sblk0[g]; ks < d.bd_sblk0[g + 1]; ks++) {
         if (!block_may_detect(d.seg_sblk[ks], x, y, margin)) continue;
-        const int k0 = blk0 + (ks - d.bd_sblk0[g]) * MEL_SEGB2;
-        const int k1 = min(k0 + MEL_SEGB2, blk1);
-        for (int k = k0; k < k1; k++)
-            if (block_may_detect(d.seg_blk[k], x, y, margin)) body(k - blk0);
-    }
-}
-
-// regular task: slave node kS of global border gS of body bS against neighbour (bM, rM, shM)
-template <typename F>
-__device__ __forceinline__ void enum_regular(const mel_dev& d, int bS, int gS, int kS, int bM, int rM, int shM, F&& f)
-{
-    int gM = d.b_bd0[bM] + rM;
-    int eM0 = d.bd_e0[gM], nM = d.bd_e0[gM + 1] - eM0;
-    int eS = d.bd_e0[gS] + kS;
-    double2 xs = d.x[d.b_node0[bS] + d.e_node[eS]];
-    double dd = d.b_dist[3 * bS + 1], cd = d.b_dist[3 * bS + 2];
-    double margin = dd * 1.0001 + 1e-12 * (fabs(xs.x) + fabs(xs.y) + fabs(d.period * shM)) + 1e-15;
-    double xrel = xs.x - d.period * shM;
-    int mb = d.b_node0[bM];
-    for_near_blocks(d, gM, xrel, xs.y, margin, [&](int kb) {
-        int s0 = kb * MEL_SEGB;
-        int s1 = min(s0 + MEL_SEGB, nM - 1);
-        for (int seg = s0; seg < s1; seg++) {
-            int e = eM0 + seg;
-            const int* sn = d.e_sn + 4 * e;
-            const int* ss = d.e_ss + 4 * e;
-            double2 p1 = d.x[mb + sn[1]], p2 = d.x[mb + sn[2]];
-            double X1 = p1.x + d.period * (shM + ss[1]), Y1 = p1.y;
-            double X2 = p2.x + d.period * (shM + ss[2]), Y2 = p2.y;
-            if (detect_proximity(xs.x, xs.y, X1, Y1, X2, Y2, dd) == 0) continue;
-            double2 p0 = d.x[mb + sn[0]], p3 = d.x[mb + sn[3]];
-            double X0 = p0.x + d.period * (shM + ss[0]), Y0 = p0.y;
-            double X3 = p3.x + d.period * (shM + ss[3]), Y3 = p3.y;
-            Proj p;
-            p.gap = 0.; p.xsi = 0.; p.xn = p.yn = p.xt = p.yt = 0.; p.N[0] = p.N[1] = p.N[2] = p.N[3] = 0.; p.flag = 0;
-            closest_linear(xs.x, xs.y, X0, Y0, X1, Y1, X2, Y2, X3, Y3, p);
-            if ((p.flag == -2 || p.flag == -1 || p.flag == 0) && (p.gap > -cd)) f(seg, e, p);
+        const int k0 = blk0 + (ks - d.bd_sblk0[g]) * MEL_SEGB2, k1 = min(k0 + MEL_SEGB2, blk1);
+        for (int k = k0; k < k1; k += 4) {
+            double4 bb[4];
+#pragma unroll
+            for (int q = 0; q < 4; q++) bb[q] = d.seg_blk[min(k + q, k1 - 1)];
+#pragma unroll
+            for (int q = 0; q < 4; q++) if (block_may_detect(bb[q], x, y, margin)) return true;
         }
-    });
+    }
+    return false;
 }
 
-// self task: slave node kS of global border gS of body bS against the body's own segments
-// (Code/Proximity.h:355-405); Closest_2_segment_self never yields flag 0, so those pairs are skipped
-template <typename F>
-__device__ __forceinline__ void enum_self(const mel_dev& d, int bS, int gS, int kS, F&& f)
+// Calls test(seg) in all lanes for the segments of border g's blocks that lie within `margin` of (x, y),
+// two blocks (32 segments, a lane each; seg -1: none) at a time in ascending order, and hit(accepted
+// lanes) after each.  One warp.
+template <typename T, typename H>
+__device__ __forceinline__ void for_near_segments(const mel_dev& d, int g, double x, double y, double margin, int lane, T&& test, H&& hit)
 {
-    int eS = d.bd_e0[gS] + kS;
-    int NodeS = d.e_node[eS];
-    int n0 = d.b_node0[bS];
-    double2 xs = d.x[n0 + NodeS];
-    double dd = d.b_dist[3 * bS + 1], cd = d.b_dist[3 * bS + 2];
-    double margin = dd * 1.0001 + 1e-12 * (fabs(xs.x) + fabs(xs.y)) + 1e-15;
-    for (int gM = d.b_bd0[bS]; gM < d.b_bd0[bS + 1]; gM++) {
-        int eM0 = d.bd_e0[gM], nM = d.bd_e0[gM + 1] - eM0;
-        for_near_blocks(d, gM, xs.x, xs.y, margin, [&](int kb) {
-            int s0 = kb * MEL_SEGB;
-            int s1 = min(s0 + MEL_SEGB, nM - 1);
-            for (int seg = s0; seg < s1; seg++) {
-                int e = eM0 + seg;
-                const int* sn = d.e_sn + 4 * e;
-                if (sn[1] == NodeS) continue;
-                if (sn[2] == NodeS) continue;
-                double2 p1 = d.x[n0 + sn[1]], p2 = d.x[n0 + sn[2]];
-                if (detect_proximity(xs.x, xs.y, p1.x, p1.y, p2.x, p2.y, dd) == 0) continue;
-                if (sn[0] == NodeS || sn[3] == NodeS) continue;
-                double2 p0 = d.x[n0 + sn[0]], p3 = d.x[n0 + sn[3]];
-                Proj p;
-                p.gap = 0.; p.xsi = 0.; p.xn = p.yn = p.xt = p.yt = 0.; p.N[0] = p.N[1] = p.N[2] = p.N[3] = 0.; p.flag = 0;
-                closest_linear(xs.x, xs.y, p0.x, p0.y, p1.x, p1.y, p2.x, p2.y, p3.x, p3.y, p);
-                if (p.flag == 0 && (p.gap > -cd)) f(seg, e, p, gM - d.b_bd0[bS]);
-            }
-        });
+    const int blk0 = d.bd_blk0[g], nblk = d.bd_blk0[g + 1] - blk0, nseg = d.bd_e0[g + 1] - d.bd_e0[g] - 1;
+    for (int ks = d.bd_sblk0[g]; ks < d.bd_sblk0[g + 1]; ks++) {
+        const int k0 = (ks - d.bd_sblk0[g]) * MEL_SEGB2;
+        const bool near = lane < 16 && k0 + lane < nblk && block_may_detect(d.seg_blk[blk0 + k0 + lane], x, y, margin);
+        unsigned m = __ballot_sync(0xffffffffu, near);
+        while (m) {
+            const int a = __ffs(m) - 1;
+            m &= m - 1;
+            const int b = m ? __ffs(m) - 1 : -1;
+            m &= m - 1;
+            const int kb = lane < 16 ? a : b;
+            int seg = kb >= 0 ? (k0 + kb) * MEL_SEGB + (lane & 15) : -1;
+            if (seg >= nseg) seg = -1;
+            const bool ok = seg >= 0 && test(seg);
+            hit(__ballot_sync(0xffffffffu, ok), seg);
+        }
     }
+}
+
+// projection of slave node (xs, ys) onto segment e of a master body (nodes from mb, shifted by shM): the
+// acceptance test of the regular search (Code/Proximity.h:221-270)
+__device__ __forceinline__ bool project_regular(const mel_dev& d, double2 xs, int mb, int shM, int e, double dd, double cd, Proj& p)
+{
+    const int* sn = d.e_sn + 4 * e;
+    const int* ss = d.e_ss + 4 * e;
+    const double2 p1 = d.x[mb + sn[1]], p2 = d.x[mb + sn[2]];
+    const double X1 = p1.x + d.period * (shM + ss[1]), Y1 = p1.y;
+    const double X2 = p2.x + d.period * (shM + ss[2]), Y2 = p2.y;
+    if (detect_proximity(xs.x, xs.y, X1, Y1, X2, Y2, dd) == 0) return false;
+    const double2 p0 = d.x[mb + sn[0]], p3 = d.x[mb + sn[3]];
+    const double X0 = p0.x + d.period * (shM + ss[0]), Y0 = p0.y;
+    const double X3 = p3.x + d.period * (shM + ss[3]), Y3 = p3.y;
+    p.gap = 0.; p.xsi = 0.; p.xn = p.yn = p.xt = p.yt = 0.; p.N[0] = p.N[1] = p.N[2] = p.N[3] = 0.; p.flag = 0;
+    closest_linear(xs.x, xs.y, X0, Y0, X1, Y1, X2, Y2, X3, Y3, p);
+    return (p.flag == -2 || p.flag == -1 || p.flag == 0) && (p.gap > -cd);
+}
+
+// the same against the body's own segment e (Code/Proximity.h:355-405); Closest_2_segment_self never
+// yields flag 0, so those pairs are skipped
+__device__ __forceinline__ bool project_self(const mel_dev& d, double2 xs, int NodeS, int n0, int e, double dd, double cd, Proj& p)
+{
+    const int* sn = d.e_sn + 4 * e;
+    if (sn[1] == NodeS) return false;
+    if (sn[2] == NodeS) return false;
+    const double2 p1 = d.x[n0 + sn[1]], p2 = d.x[n0 + sn[2]];
+    if (detect_proximity(xs.x, xs.y, p1.x, p1.y, p2.x, p2.y, dd) == 0) return false;
+    if (sn[0] == NodeS || sn[3] == NodeS) return false;
+    const double2 p0 = d.x[n0 + sn[0]], p3 = d.x[n0 + sn[3]];
+    p.gap = 0.; p.xsi = 0.; p.xn = p.yn = p.xt = p.yt = 0.; p.N[0] = p.N[1] = p.N[2] = p.N[3] = 0.; p.flag = 0;
+    closest_linear(xs.x, xs.y, p0.x, p0.y, p1.x, p1.y, p2.x, p2.y, p3.x, p3.y, p);
+    return p.flag == 0 && (p.gap > -cd);
+}
+
+// margin of the box tests around (x, y): the detection distance, widened past rounding
+__device__ __forceinline__ double near_margin(const mel_dev& d, double2 xs, double dd, int shM)
+{
+    return dd * 1.0001 + 1e-12 * (fabs(xs.x) + fabs(xs.y) + fabs(d.period * shM)) + 1e-15;
 }
 
 // ---------------------------------------------------------------------------------------------
-// task list on the device.  Task t: slave body, slave border (global), neighbour index q (-1: self),
-// slave border nodes; tasks of a body are contiguous: (border, neighbour) pairs in the reference's
-// loop order (Code/Proximity.h:207-212), then one self task per border (Code/Proximity.h:346-356).
+// tasks and slots.  A body's tasks are contiguous: (border, neighbour) pairs in the reference's loop
+// order (Code/Proximity.h:207-212), then one self task per border (Code/Proximity.h:346-356); its
+// slots likewise, a slot per slave border node of each task.
 // ---------------------------------------------------------------------------------------------
 __device__ __forceinline__ bool has_self(const mel_dev& d, int b)
 {
     return d.self_contact && d.b_type[b] == MEL_BODY_DEFORMABLE && !d.b_per[b];
 }
 
-// per body: task count and slot count (slave border nodes summed over its tasks)
-__device__ __forceinline__ void task_count_item(const mel_dev& d, const int* nbn, int* tcnt, int* scnt, int b)
+// a slot's slave body, slave border (global), neighbour (-1: self), slave border node and task
+struct slot_ref { int b, g, q, kS, t; };
+__device__ __forceinline__ slot_ref slot_of(const mel_prox_job& j, int s)
 {
-    if (b >= d.nb) return;
-    int nbd = d.b_bd0[b + 1] - d.b_bd0[b];
-    int nent = d.bd_e0[d.b_bd0[b + 1]] - d.bd_e0[d.b_bd0[b]];
-    int per = nbn[b] + (has_self(d, b) ? 1 : 0);
-    tcnt[b] = nbd * per;
-    scnt[b] = nent * per;
-}
-
-// task t = (slave body, slave border, neighbour q or -1 for self, first slot), its slave border node
-// count, its first slot and its master body; inc_cnt counts the tasks of each master body
-__device__ __forceinline__ void task_fill_item(const mel_dev& d, const int* nbr, const int* nbn, int cap, const int* btask0,
-                                               const int* bslot0, int4* task, int* tns, int* tslot, int* tkey, int* inc_cnt,
-                                               int b)
-{
-    if (b >= d.nb) return;
-    int t = btask0[b];
-    int slot = bslot0[b];
-    const int* nb = nbr + (size_t)3 * cap * b;
-    for (int g = d.b_bd0[b]; g < d.b_bd0[b + 1]; g++) {
-        int nS = d.bd_e0[g + 1] - d.bd_e0[g];
-        for (int q = 0; q < nbn[b]; q++) {
-            int key = nb[3 * q];
-            task[t] = make_int4(b, g, q, slot); tns[t] = nS; tslot[t] = slot; tkey[t] = key;
-            atomicAdd(&inc_cnt[key], 1);
-            t++; slot += nS;
-        }
+    const mel_dev& d = j.d;
+    int lo = 0, hi = d.nb;                   // largest b with bslot0[b] <= s that has slots
+    while (hi - lo > 1) { const int mid = (lo + hi) >> 1; if (j.bslot0[mid] <= s) lo = mid; else hi = mid; }
+    slot_ref r;
+    r.b = lo;
+    int at = s - j.bslot0[lo];
+    const int n = j.nbn[lo], g0 = d.b_bd0[lo], g1 = d.b_bd0[lo + 1];
+    int g = g0;
+    r.q = -1;
+    for (; g < g1; g++) {                    // regular tasks
+        const int nS = d.bd_e0[g + 1] - d.bd_e0[g];
+        if (at < n * nS) { r.q = at / nS; at -= r.q * nS; break; }
+        at -= n * nS;
     }
-    if (has_self(d, b))
-        for (int g = d.b_bd0[b]; g < d.b_bd0[b + 1]; g++) {
-            int nS = d.bd_e0[g + 1] - d.bd_e0[g];
-            task[t] = make_int4(b, g, -1, slot); tns[t] = nS; tslot[t] = slot; tkey[t] = b;
-            atomicAdd(&inc_cnt[b], 1);
-            t++; slot += nS;
+    if (g == g1)                             // self tasks
+        for (g = g0; g < g1 - 1; g++) {
+            const int nS = d.bd_e0[g + 1] - d.bd_e0[g];
+            if (at < nS) break;
+            at -= nS;
         }
+    r.g = g;
+    r.kS = at;
+    r.t = j.btask0[lo] + (r.q >= 0 ? (g - g0) * n + r.q : (g1 - g0) * n + (g - g0));
+    return r;
 }
 
-// slot -> task map: warp per task, lanes over its slots
-__device__ __forceinline__ void slot_task_item(const mel_dev& d, const int4* task, int ntask, int* tmap, int t, int lane)
+// A candidate: a = {task, slave border node, its number among the node's candidates, master entry},
+// b = {slave body, slave border (global), neighbour or -1, master border (global)}
+#define FIND_THREADS 128
+__global__ void __launch_bounds__(FIND_THREADS) find_kernel(const mel_prox_job* J, const int* bpre, int nj, const __grid_constant__ mel_prox_job one)
 {
-    if (t >= ntask) return;
-    const int4 tk = task[t];
-    const int nS = d.bd_e0[tk.y + 1] - d.bd_e0[tk.y];
-    for (int kS = lane; kS < nS; kS += 32) tmap[tk.w + kS] = t;
-}
-
-// candidates of slot s (one slave border node of one task); one thread per slot, so a task with a
-// long slave border (a plate or a wall) spreads over many warps
-__device__ __forceinline__ void count_item(const mel_dev& d, const int4* task, const int* tmap, int nslot, const int* nbr,
-                                           int cap, int* slot_cnt, int s)
-{
-    if (s >= nslot) return;
-    int t = tmap[s];
-    int4 tk = task[t];
-    int bS = tk.x, gS = tk.y, q = tk.z, slot0 = tk.w;
+    __shared__ mel_prox_job sj;
+    __shared__ slot_ref s_near[FIND_THREADS];
+    __shared__ int s_n;
+    const int jj = J ? block_job(bpre, nj) : 0;
     {
-        const int kS = s - slot0;
-        int cnt = 0;
-        if (q >= 0) {
-            const int* nb = nbr + (size_t)3 * cap * bS + 3 * q;
-            enum_regular(d, bS, gS, kS, nb[0], nb[1], nb[2], [&](int, int, const Proj&) { cnt++; });
-        } else {
-            enum_self(d, bS, gS, kS, [&](int, int, const Proj&, int) { cnt++; });
-        }
-        slot_cnt[slot0 + kS] = cnt;
+        const int* src = reinterpret_cast<const int*>(J ? J + jj : &one);
+        int* dst = reinterpret_cast<int*>(&sj);
+        for (int k = threadIdx.x; k < (int)(sizeof(mel_prox_job) / sizeof(int)); k += blockDim.x) dst[k] = src[k];
+    }
+    if (threadIdx.x == 0) s_n = 0;
+    __syncthreads();
+    const mel_prox_job& j = sj;
+    const mel_dev& d = sj.d;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int s = ((int)blockIdx.x - (J ? bpre[jj] : 0)) * FIND_THREADS + (int)threadIdx.x;
+    // a thread per slot: is the slave node near any block of the master?
+    if (s < j.nslot) {
+        const slot_ref r = slot_of(j, s);
+        const double2 xs = d.x[d.b_node0[r.b] + d.e_node[d.bd_e0[r.g] + r.kS]];
+        const double dd = d.b_dist[3 * r.b + 1];
+        bool near = false;
+        if (r.q >= 0) {
+            const int* nb = j.nbr + 3 * ((size_t)j.nbr_cap * r.b + r.q);
+            near = any_near_block(d, d.b_bd0[nb[0]] + nb[1], xs.x - d.period * nb[2], xs.y, near_margin(d, xs, dd, nb[2]));
+        } else
+            for (int g = d.b_bd0[r.b]; g < d.b_bd0[r.b + 1] && !near; g++)
+                near = any_near_block(d, g, xs.x, xs.y, near_margin(d, xs, dd, 0));
+        if (near) s_near[atomicAdd(&s_n, 1)] = r;
+    }
+    __syncthreads();
+    // a warp per near slot: its candidates, in segment order
+    for (int i = warp; i < s_n; i += FIND_THREADS / 32) {
+        const slot_ref r = s_near[i];
+        const int n0 = d.b_node0[r.b], NodeS = d.e_node[d.bd_e0[r.g] + r.kS];
+        const double2 xs = d.x[n0 + NodeS];
+        const double dd = d.b_dist[3 * r.b + 1], cd = d.b_dist[3 * r.b + 2];
+        int found = 0;
+        auto list = [&](unsigned m, int e, int gM) {
+            if (!m) return;
+            int at = 0;
+            if (lane == 0) at = atomicAdd(j.ncand, __popc(m));
+            at = __shfl_sync(0xffffffffu, at, 0);
+            if ((m >> lane) & 1u) {
+                const int k = __popc(m & ((1u << lane) - 1u));
+                if (at + k < j.cand_cap) {
+                    j.cand[2 * (size_t)(at + k)] = make_int4(r.t, r.kS, found + k, e);
+                    j.cand[2 * (size_t)(at + k) + 1] = make_int4(r.b, r.g, r.q, gM);
+                }
+            }
+            found += __popc(m);
+        };
+        Proj p;
+        if (r.q >= 0) {
+            const int* nb = j.nbr + 3 * ((size_t)j.nbr_cap * r.b + r.q);
+            const int bM = nb[0], shM = nb[2], gM = d.b_bd0[bM] + nb[1], mb = d.b_node0[bM], eM0 = d.bd_e0[gM];
+            for_near_segments(d, gM, xs.x - d.period * shM, xs.y, near_margin(d, xs, dd, shM), lane,
+                [&](int seg) { return project_regular(d, xs, mb, shM, eM0 + seg, dd, cd, p); },
+                [&](unsigned m, int seg) { list(m, eM0 + seg, gM); });
+        } else
+            for (int gM = d.b_bd0[r.b]; gM < d.b_bd0[r.b + 1]; gM++) {
+                const int eM0 = d.bd_e0[gM];
+                for_near_segments(d, gM, xs.x, xs.y, near_margin(d, xs, dd, 0), lane,
+                    [&](int seg) { return project_self(d, xs, NodeS, n0, eM0 + seg, dd, cd, p); },
+                    [&](unsigned m, int seg) { list(m, eM0 + seg, gM); });
+            }
+        if (lane == 0 && found) atomicAdd(&j.tcand[r.t], found);
     }
 }
 
-// writes the candidates of slot s at their canonical positions; one thread per slot
-__device__ __forceinline__ void write_item(const mel_dev& d, const int4* task, const int* tmap, const int* nzlist,
-                                           int nnz, const int* nbr, int cap, const int* slot_off, mel_contact* out,
-                                           const mel_contact* old, const int* old_eptr, const int* old_elist,
-                                           int have_old, int i)
+// candidate i into its task's bucket (any order); leaves tcand at zero
+__device__ __forceinline__ void bucket_item(const mel_prox_job& j, int i)
 {
-    if (i >= nnz) return;
-    const int s = nzlist[i];                 // slots with at least one candidate
-    int t = tmap[s];
-    int4 tk = task[t];
-    int bS = tk.x, gS = tk.y, q = tk.z, slot0 = tk.w;
-    int rS = gS - d.b_bd0[bS];
-    int eS0 = d.bd_e0[gS];
-    {
-        const int kS = s - slot0;
-        int pos = slot_off[slot0 + kS];
-        const int end = slot_off[slot0 + kS + 1];   // the count pass found end - pos candidates
-        int eS = eS0 + kS;
-        int NodeS = d.e_node[eS];
-        double length = d.e_len[eS];
-        if (q >= 0) {
-            const int* nb = nbr + (size_t)3 * cap * bS + 3 * q;
-            int bM = nb[0], rM = nb[1], shM = nb[2];
-            double effm;
-            const double* rgM = d.rg + MEL_RIGID_NF * bM;
-            const double* rgS = d.rg + MEL_RIGID_NF * bS;
-            if (rgM[MEL_RG_MASS] == 0.) effm = 0.;
-            else if (rgS[MEL_RG_MASS] == 0.) effm = 0.;
-            else effm = 1. / (rgM[MEL_RG_INV_MASS] + rgS[MEL_RG_INV_MASS]);
-            enum_regular(d, bS, gS, kS, bM, rM, shM, [&](int seg, int e, const Proj& p) {
-                mel_contact c;
-                bool found = false;
-                if (have_old) {
-                    for (int k = old_eptr[eS]; k < old_eptr[eS + 1]; k++) {
-                        const mel_contact& o = old[old_elist[k]];
-                        if (o.bodyM == bM && o.borderM == rM && abs(o.segmentM - seg) <= 1) { c = o; found = true; break; }
-                    }
-                }
-                if (!found) {
-                    c.bodyS = bS; c.borderS = rS; c.border_nodeS = kS; c.nodeS = NodeS;
-                    c.bodyM = bM; c.borderM = rM; c.shiftM = shM; c.segmentM = seg;
-                    for (int k = 0; k < 4; k++) { c.nodeM[k] = d.e_sn[4 * e + k]; c.shiftMk[k] = d.e_ss[4 * e + k]; c.shapeM[k] = p.N[k]; }
-                    c.gapn = p.gap; c.vgapn = 0.; c.gapt = 0.; c.vgapt = 0.; c.xsi = p.xsi;
-                    c.xnorm = p.xn; c.ynorm = p.yn; c.xtan = p.xt; c.ytan = p.yt;
-                    c.effective_mass = effm; c.length = length; c.fx = 0.; c.fy = 0.;
-                    c.nb_internal = 0; c.internal[0] = 0.; c.internal[1] = 0.; c.internal[2] = 0.;
-                }
-                c.bodyS = bS;
-                c.pad_ = found ? 0 : 1;      // new elements get vgapn/vgapt in carry_kernel
-                if (pos < end) out[pos] = c;
-                pos++;
-            });
-        } else {
-            double effm = d.rg[MEL_RIGID_NF * bS + MEL_RG_MASS];
-            enum_self(d, bS, gS, kS, [&](int seg, int e, const Proj& p, int rM) {
-                mel_contact c;
-                c.bodyS = bS; c.borderS = rS; c.border_nodeS = kS; c.nodeS = NodeS;
-                c.bodyM = bS; c.borderM = rM; c.shiftM = 0; c.segmentM = seg;
-                for (int k = 0; k < 4; k++) { c.nodeM[k] = d.e_sn[4 * e + k]; c.shiftMk[k] = 0; c.shapeM[k] = p.N[k]; }
-                c.gapn = p.gap; c.vgapn = 0.; c.gapt = 0.; c.vgapt = 0.; c.xsi = p.xsi;
-                c.xnorm = p.xn; c.ynorm = p.yn; c.xtan = p.xt; c.ytan = p.yt;
-                c.effective_mass = effm; c.length = length; c.fx = 0.; c.fy = 0.;
-                c.nb_internal = 0; c.pad_ = 1; c.internal[0] = 0.; c.internal[1] = 0.; c.internal[2] = 0.;
-                if (pos < end) out[pos] = c;
-                pos++;
-            });
-        }
-        if (pos != end) atomicOr(&d.err[MEL_E_BOUNDS], 4u);   // count and write passes disagree
+    if (i >= j.ncont_new) return;
+    const int t = j.cand[2 * (size_t)i].x;
+    j.bucket[j.toff[t] + atomicSub(&j.tcand[t], 1) - 1] = i;
+}
+
+// candidate i at its place in the new list; one warp
+__device__ __forceinline__ void write_item(const mel_prox_job& j, int i, int lane)
+{
+    if (i >= j.ncont_new) return;
+    const mel_dev& d = j.d;
+    const int4 a = j.cand[2 * (size_t)i], c4 = j.cand[2 * (size_t)i + 1];
+    const int t = a.x, kS = a.y, e = a.w, bS = c4.x, gS = c4.y, q = c4.z, gM = c4.w;
+    const int t0 = j.toff[t], t1 = j.toff[t + 1];
+    int rank = 0;
+    for (int k = t0 + lane; k < t1; k += 32) {
+        const int4 o = j.cand[2 * (size_t)j.bucket[k]];
+        rank += o.y < kS || (o.y == kS && o.z < a.z);
     }
+    for (int o = 16; o > 0; o >>= 1) rank += __shfl_xor_sync(0xffffffffu, rank, o);
+    const int pos = t0 + rank;
+    const int rS = gS - d.b_bd0[bS], eS = d.bd_e0[gS] + kS, NodeS = d.e_node[eS], n0 = d.b_node0[bS];
+    const int seg = e - d.bd_e0[gM];
+    int bM = bS, shM = 0;
+    if (q >= 0) {
+        const int* nb = j.nbr + 3 * ((size_t)j.nbr_cap * bS + q);
+        bM = nb[0];
+        shM = nb[2];
+    }
+    const int rM = gM - d.b_bd0[bM];
+    if (lane == 0) {
+        if (rank == 0) { j.tkey[t] = bM; atomicAdd(&j.inc_cnt[bM], 1); }
+        d.cont_w[pos] = 0.;
+    }
+    mel_contact* out = j.cont_new + pos;
+    // the first old element of this slave border node, in list order, on the same master border
+    // within one segment
+    if (q >= 0 && j.have_old) {
+        const int o1 = j.b_cont0[bS + 1];
+        for (int k = j.b_cont0[bS]; k < o1; k += 32) {
+            bool match = false;
+            if (k + lane < o1) {
+                const mel_contact& o = d.cont[k + lane];
+                match = o.border_nodeS == kS && o.borderS == rS && o.bodyM == bM && o.borderM == rM && abs(o.segmentM - seg) <= 1;
+            }
+            const unsigned m = __ballot_sync(0xffffffffu, match);
+            if (m) {
+                const int* src = reinterpret_cast<const int*>(d.cont + k + __ffs(m) - 1);
+                int* dst = reinterpret_cast<int*>(out);
+                for (int w = lane; w < (int)(sizeof(mel_contact) / sizeof(int)); w += 32) dst[w] = src[w];
+                __syncwarp();
+                if (lane == 0) { out->bodyS = bS; out->pad_ = 0; }
+                return;
+            }
+        }
+    }
+    if (lane) return;
+    const double2 xs = d.x[n0 + NodeS];
+    const double dd = d.b_dist[3 * bS + 1], cd = d.b_dist[3 * bS + 2];
+    Proj p;
+    const bool ok = q >= 0 ? project_regular(d, xs, d.b_node0[bM], shM, e, dd, cd, p) : project_self(d, xs, NodeS, n0, e, dd, cd, p);
+    if (!ok) atomicOr(&d.err[MEL_E_BOUNDS], 4u);         // both passes read the same positions
+    mel_contact c;
+    c.bodyS = bS; c.borderS = rS; c.border_nodeS = kS; c.nodeS = NodeS;
+    c.bodyM = bM; c.borderM = rM; c.shiftM = shM; c.segmentM = seg;
+    for (int k = 0; k < 4; k++) { c.nodeM[k] = d.e_sn[4 * e + k]; c.shiftMk[k] = q >= 0 ? d.e_ss[4 * e + k] : 0; c.shapeM[k] = p.N[k]; }
+    c.gapn = p.gap; c.vgapn = 0.; c.gapt = 0.; c.vgapt = 0.; c.xsi = p.xsi;
+    c.xnorm = p.xn; c.ynorm = p.yn; c.xtan = p.xt; c.ytan = p.yt;
+    if (q >= 0) {
+        const double* rgM = d.rg + MEL_RIGID_NF * bM;
+        const double* rgS = d.rg + MEL_RIGID_NF * bS;
+        if (rgM[MEL_RG_MASS] == 0.) c.effective_mass = 0.;
+        else if (rgS[MEL_RG_MASS] == 0.) c.effective_mass = 0.;
+        else c.effective_mass = 1. / (rgM[MEL_RG_INV_MASS] + rgS[MEL_RG_INV_MASS]);
+    } else c.effective_mass = d.rg[MEL_RIGID_NF * bS + MEL_RG_MASS];
+    c.length = d.e_len[eS]; c.fx = 0.; c.fy = 0.;
+    c.nb_internal = 0; c.internal[0] = 0.; c.internal[1] = 0.; c.internal[2] = 0.;
+    c.pad_ = 1;                                          // new elements get vgapn/vgapt in the carry
+    *out = c;
 }
 
 // ---------------------------------------------------------------------------------------------
 // incoming (master-side) contact ranges of each body in send order.  Send_contact_forces runs over
 // the sending bodies in index order (Code/Solver.h:61-62) and each sender over its contact list, so
-// the incoming ranges of master body B are the tasks whose master is B, in ascending task order.
-// Tasks are grouped by master with a counting pass and an atomic fill, then each group is put back
-// in ascending order by a rank sort (task ids are unique), one warp per master body.
+// the incoming ranges of master body B are the tasks whose master is B, in ascending task order; tasks
+// without contacts are left out.  Tasks are grouped by master with a counting pass and an atomic fill,
+// then each group is put back in ascending order by a rank sort (task ids are unique).
 // ---------------------------------------------------------------------------------------------
-__device__ __forceinline__ void inc_fill_item(const int* tkey, int ntask, int* cur, int* tmp, int t)
+__device__ __forceinline__ void inc_fill_item(const mel_prox_job& j, int t)
 {
-    if (t >= ntask) return;
-    tmp[atomicAdd(&cur[tkey[t]], 1)] = t;
+    if (t >= j.ntask || j.toff[t + 1] == j.toff[t]) return;
+    const int key = j.tkey[t];
+    j.inc_task[j.b_inc0[key] + atomicSub(&j.inc_cnt[key], 1) - 1] = t;
 }
 
-__device__ __forceinline__ void inc_sort_item(int nb, const int* inc0, const int* tmp, int* sorted, int B, int lane)
-{
-    if (B >= nb) return;
-    int i0 = inc0[B], n = inc0[B + 1] - i0;
-    for (int i = lane; i < n; i += 32) {
-        int t = tmp[i0 + i], r = 0;
-        for (int j = 0; j < n; j++) r += (tmp[i0 + j] < t);
-        sorted[i0 + r] = t;
-    }
-}
-
-__device__ __forceinline__ void inc_range_item(const int* sorted, int n, const int* tslot, const int* tns,
-                                               const int* slot_off, int2* rng, int i)
-{
-    if (i >= n) return;
-    int t = sorted[i];
-    rng[i] = make_int2(slot_off[tslot[t]], slot_off[tslot[t] + tns[t]]);
-}
-
-
-// per-body counting sort of a body-major contact list by slave border entry: one warp per body,
-// 32 contacts at a time in list order; lanes with the same entry take consecutive places in lane
-// order, so every entry lists its contacts in list order (as a serial pass would)
-__device__ __forceinline__ void entry_index_item(const mel_dev& d, const mel_contact* cont, const int* b_cont0,
-                                                 int* eptr_cnt, int* elist, int b, int lane)
-{
-    if (b >= d.nb) return;
-    const int e_lo = d.bd_e0[d.b_bd0[b]], e_hi = d.bd_e0[d.b_bd0[b + 1]];
-    const int c0 = b_cont0[b], c1 = b_cont0[b + 1];
-    // eptr_cnt holds the exclusive offsets of this body's entries (prepared by the caller) and is
-    // advanced as a cursor; only this warp touches the entries of body b
-    for (int base = c0; base < c1; base += 32) {
-        const int c = base + lane;
-        int e = -1;
-        if (c < c1) {
-            e = d.bd_e0[d.b_bd0[b] + cont[c].borderS] + cont[c].border_nodeS;
-            if (e < e_lo || e >= e_hi) { atomicOr(&d.err[MEL_E_BOUNDS], 2u); e = -1; }
-        }
-        const unsigned same = __match_any_sync(0xffffffffu, e);
-        const int leader = __ffs(same) - 1;
-        int pos = 0;
-        if (lane == leader && e >= 0) { pos = eptr_cnt[e]; eptr_cnt[e] = pos + __popc(same); }
-        pos = __shfl_sync(0xffffffffu, pos, leader) + __popc(same & ((1u << lane) - 1u));
-        if (e >= 0) elist[pos] = c;
-        __syncwarp();
-    }
-}
-
-__device__ __forceinline__ void entry_count_item(const mel_dev& d, const mel_contact* cont, int n, int* cnt, int c)
-{
-    if (c >= n) return;
-    int b = cont[c].bodyS;
-    int e = d.bd_e0[d.b_bd0[b] + cont[c].borderS] + cont[c].border_nodeS;
-    atomicAdd(&cnt[e], 1);
-}
-
+// first index with bodyS >= b of a body-major list
 __device__ __forceinline__ void body_range_item(const mel_contact* cont, int n, int nb, int* b_cont0, int b)
 {
-    // b_cont0[b] = first index with bodyS >= b (list is body-major)
     if (b > nb) return;
     int lo = 0, hi = n;
     while (lo < hi) { int mid = (lo + hi) >> 1; if (cont[mid].bodyS < b) lo = mid + 1; else hi = mid; }
@@ -788,11 +826,9 @@ __device__ __forceinline__ void body_range_item(const mel_contact* cont, int n, 
 // Code/Proximity.h:286-313); self contacts use a fresh variable (Code/Proximity.h:350).  One warp
 // per body, 32 contacts at a time: a new element takes the values of the last inherited non-self
 // element before it (found by ballot within the 32, else carried over from earlier ones).
-__device__ __forceinline__ void carry_item(const mel_dev& d, mel_contact* cont, const int* b_cont0, int b, int lane)
+__device__ __forceinline__ void carry_item(mel_contact* cont, int b, int c0, int c1, int lane)
 {
-    if (b >= d.nb) return;
     double vn = 0., vt = 0.;                 // carried value (equal in all lanes)
-    const int c0 = b_cont0[b], c1 = b_cont0[b + 1];
     for (int base = c0; base < c1; base += 32) {
         const int c = base + lane;
         const bool valid = c < c1;
@@ -821,6 +857,26 @@ __device__ __forceinline__ void carry_item(const mel_dev& d, mel_contact* cont, 
     }
 }
 
+// body b of the new list (one warp): its incoming ranges, its contact range and the carry
+__device__ __forceinline__ void body_item(const mel_prox_job& j, int b, int lane)
+{
+    const mel_dev& d = j.d;
+    if (b >= d.nb) return;
+    const int i0 = j.b_inc0[b], n = j.b_inc0[b + 1] - i0;
+    for (int i = lane; i < n; i += 32) {
+        const int t = j.inc_task[i0 + i];
+        int r = 0;
+        for (int k = 0; k < n; k++) r += j.inc_task[i0 + k] < t;
+        j.inc_rng[i0 + r] = make_int2(j.toff[t], j.toff[t + 1]);
+    }
+    const int c0 = j.toff[j.btask0[b]], c1 = j.toff[j.btask0[b + 1]];
+    if (lane == 0) {
+        j.b_cont0[b] = c0;
+        if (b == d.nb - 1) j.b_cont0[d.nb] = c1;
+    }
+    carry_item(d.cont, b, c0, c1, lane);
+}
+
 // ---------------------------------------------------------------------------------------------
 // job-table launches: blocks [bpre[j], bpre[j+1]) serve member j.  The block copies the member's
 // job into shared memory; item `it` of the member is handled by TPI consecutive threads (TPI 32:
@@ -829,17 +885,18 @@ __device__ __forceinline__ void carry_item(const mel_dev& d, mel_contact* cont, 
 #define PROX_THREADS 256
 static_assert(PROX_THREADS == PROX_THREADS_CL, "cell-list scratch is sized for the job kernels' block");
 #define JOB_KERNEL(name, TPI, ...)                                                                  \
-    __global__ void __launch_bounds__(PROX_THREADS) name(const mel_prox_job* J, const int* bpre, int nj) \
+    __global__ void __launch_bounds__(PROX_THREADS) name(const mel_prox_job* J, const int* bpre, int nj, \
+                                                         const __grid_constant__ mel_prox_job one)  \
     {                                                                                               \
         __shared__ mel_prox_job sj;                                                                 \
-        const int jj = block_job(bpre, nj);                                                         \
+        const int jj = J ? block_job(bpre, nj) : 0;                                                         \
         {                                                                                           \
-            const int* src = reinterpret_cast<const int*>(J + jj);                                  \
+            const int* src = reinterpret_cast<const int*>(J ? J + jj : &one);                                  \
             int* dst = reinterpret_cast<int*>(&sj);                                                 \
             for (int k = threadIdx.x; k < (int)(sizeof(mel_prox_job) / sizeof(int)); k += blockDim.x) dst[k] = src[k]; \
         }                                                                                           \
         __syncthreads();                                                                            \
-        const int it = (blockIdx.x - bpre[jj]) * (PROX_THREADS / (TPI)) + (int)threadIdx.x / (TPI); \
+        const int it = ((int)blockIdx.x - (J ? bpre[jj] : 0)) * (PROX_THREADS / (TPI)) + (int)threadIdx.x / (TPI); \
         const int lane = threadIdx.x & 31;                                                          \
         (void)lane;                                                                                 \
         const mel_prox_job& j = sj;                                                                 \
@@ -848,63 +905,77 @@ static_assert(PROX_THREADS == PROX_THREADS_CL, "cell-list scratch is sized for t
         __VA_ARGS__;                                                                                \
     }
 
-JOB_KERNEL(aabb_kernel, 32, aabb_item(d, j.aabb, j.shmin, j.shmax, it, lane))
-JOB_KERNEL(segblock_kernel, 1, segblock_item(d, it))
-JOB_KERNEL(superblock_kernel, 1, superblock_item(d, it))
+// the boxes, and what the first neighbour attempt starts from: cleared overflow words and buckets
+JOB_KERNEL(boxes_kernel, 32,
+    if (it < d.nbd) aabb_item(d, j.aabb, j.shmin, j.shmax, it, lane);
+    else if (it < d.nbd + d.nsblk) superblock_item(d, it - d.nbd, lane);
+    else if (j.cl_on) cl_zero_item(j, 32 * (it - d.nbd - d.nsblk) + lane);
+    if (it == 0 && lane == 0) { d.err[MEL_E_NBR_OVERFLOW] = 0u; d.err[MEL_E_NBR_NEED] = 0u; })
 JOB_KERNEL(neighbour_kernel, 32, neighbour_item(d, j.aabb, j.shmin, j.shmax, j.nbr, j.nbn, j.nbr_cap, it, lane))
 JOB_KERNEL(cl_zero_kernel, 1, cl_zero_item(j, it))
 JOB_KERNEL(cl_count_kernel, 1, cl_count_item(j, it))
 JOB_KERNEL(cl_fill_kernel, 1, cl_fill_item(j, it))
 JOB_KERNEL(cl_neighbour_kernel, 32, cl_neighbour_item(j, it, lane))
-JOB_KERNEL(task_count_kernel, 1, task_count_item(d, j.nbn, j.tcnt, j.scnt, it))
-JOB_KERNEL(zero_tcnt_kernel, 1, if (it <= d.nb) j.tcnt[it] = 0)
-JOB_KERNEL(task_fill_kernel, 1, task_fill_item(d, j.nbr, j.nbn, j.nbr_cap, j.btask0, j.bslot0, j.task, j.tns, j.tslot,
-                                               j.tkey, j.tcnt, it))
-JOB_KERNEL(slot_task_kernel, 32, slot_task_item(d, j.task, j.ntask, j.tmap, it, lane))
-JOB_KERNEL(count_kernel, 1, count_item(d, j.task, j.tmap, j.nslot, j.nbr, j.nbr_cap, j.slot_cnt, it))
-// slots with candidates: flags in place of the counts (after their scan), then their list
-JOB_KERNEL(nz_flag_kernel, 1, if (it < j.nslot) j.slot_cnt[it] = j.slot_cnt[it] > 0 ? 1 : 0)
-JOB_KERNEL(nz_list_kernel, 1, if (it < j.nslot && j.slot_cnt[it]) j.nzlist[j.nzoff[it]] = it)
-JOB_KERNEL(write_kernel, 1, write_item(d, j.task, j.tmap, j.nzlist, j.nnz, j.nbr, j.nbr_cap, j.slot_off, j.cont_new,
-                                       d.cont, j.e_ptr, j.e_list, j.have_old, it))
-JOB_KERNEL(zero_contw_kernel, 1, if (it <= d.ncont) d.cont_w[it] = 0.)
-JOB_KERNEL(copy_inc_kernel, 1, if (it < d.nb) j.tcnt[it] = j.b_inc0[it])
-JOB_KERNEL(inc_fill_kernel, 1, inc_fill_item(j.tkey, j.ntask, j.tcnt, j.inc_task, it))
-JOB_KERNEL(inc_sort_kernel, 32, inc_sort_item(d.nb, j.b_inc0, j.inc_task, j.inc_task + j.ntask, it, lane))
-JOB_KERNEL(inc_range_kernel, 1, inc_range_item(j.inc_task + j.ntask, j.ntask, j.tslot, j.tns, j.slot_off, j.inc_rng, it))
+JOB_KERNEL(clear_kernel, 1,
+    if (it <= j.ntask) j.tcand[it] = 0;
+    if (it <= d.nb) j.inc_cnt[it] = 0;
+    if (it == 0) *j.ncand = 0)
+JOB_KERNEL(bucket_kernel, 1, bucket_item(j, it))
+JOB_KERNEL(write_kernel, 32, write_item(j, it, lane))
+JOB_KERNEL(inc_fill_kernel, 1, inc_fill_item(j, it))
+JOB_KERNEL(bodies_kernel, 32, body_item(j, it, lane))
 JOB_KERNEL(body_range_kernel, 1, body_range_item(d.cont, d.ncont, d.nb, j.b_cont0, it))
-JOB_KERNEL(zero_ecnt_kernel, 1, if (it <= d.ne) j.e_cnt[it] = 0)
-JOB_KERNEL(entry_count_kernel, 1, entry_count_item(d, d.cont, d.ncont, j.e_cnt, it))
-JOB_KERNEL(copy_eptr_kernel, 1, if (it <= d.ne) j.e_cur[it] = j.e_ptr[it])
-JOB_KERNEL(entry_index_kernel, 32, entry_index_item(d, d.cont, j.b_cont0, j.e_cur, j.e_list, it, lane))
-JOB_KERNEL(carry_kernel, 32, carry_item(d, d.cont, j.b_cont0, it, lane))
 
-// one thread per member: clear the neighbour-overflow words before an attempt
-__global__ void nbr_clear_kernel(const mel_prox_job* J, int nj)
+// one block per member: tasks and slots of every body, their offsets (btask0, bslot0), and the words
+// the host needs after the neighbour stage (0-4)
+__global__ void __launch_bounds__(1024) tasks_kernel(const mel_prox_job* J, int nj, const __grid_constant__ mel_prox_job one)
 {
-    const int k = blockIdx.x * blockDim.x + threadIdx.x;
-    if (k >= nj) return;
-    J[k].d.err[MEL_E_NBR_OVERFLOW] = 0u;
-    J[k].d.err[MEL_E_NBR_NEED] = 0u;
-}
-// one thread per member: the words the host needs after the neighbour stage (0-4) or the count
-// stage (5)
-__global__ void readback_kernel(const mel_prox_job* J, int nj, int stage)
-{
-    const int k = blockIdx.x * blockDim.x + threadIdx.x;
-    if (k >= nj) return;
-    const mel_prox_job& j = J[k];
-    int* r = j.readback;
-    if (stage == 0) {
-        r[0] = (int)j.d.err[MEL_E_NAN];
-        r[1] = (int)j.d.err[MEL_E_NBR_OVERFLOW];
-        r[2] = (int)j.d.err[MEL_E_NBR_NEED];
-        r[3] = j.btask0[j.d.nb];
-        r[4] = j.bslot0[j.d.nb];
-    } else {
-        r[5] = j.slot_off[j.nslot];
-        r[6] = j.nzoff[j.nslot];
+    __shared__ int s[32];
+    const mel_prox_job& j = J ? J[blockIdx.x] : one;
+    const mel_dev& d = j.d;
+    int t0 = 0, s0 = 0;
+    for (int base = 0; base < d.nb; base += 1024) {
+        const int b = base + (int)threadIdx.x;
+        int tc = 0, sc = 0;
+        if (b < d.nb) {
+            const int g0 = d.b_bd0[b], g1 = d.b_bd0[b + 1], per = j.nbn[b] + (has_self(d, b) ? 1 : 0);
+            tc = (g1 - g0) * per;
+            sc = (d.bd_e0[g1] - d.bd_e0[g0]) * per;
+        }
+        int tt, st;
+        const int ta = block_scan(tc, s, tt), sa = block_scan(sc, s, st);
+        if (b < d.nb) { j.btask0[b] = t0 + ta; j.bslot0[b] = s0 + sa; }
+        t0 += tt;
+        s0 += st;
     }
+    if (threadIdx.x == 0) {
+        j.btask0[d.nb] = t0;
+        j.bslot0[d.nb] = s0;
+        int* r = j.readback;
+        r[0] = (int)d.err[MEL_E_NAN];
+        r[1] = (int)d.err[MEL_E_NBR_OVERFLOW];
+        r[2] = (int)d.err[MEL_E_NBR_NEED];
+        r[3] = t0;
+        r[4] = s0;
+    }
+}
+
+// one thread per member: clear the neighbour-overflow words before another attempt
+__global__ void nbr_clear_kernel(const mel_prox_job* J, int nj, const __grid_constant__ mel_prox_job one)
+{
+    const int k = blockIdx.x * blockDim.x + threadIdx.x;
+    if (k >= nj) return;
+    const mel_dev& d = J ? J[k].d : one.d;
+    d.err[MEL_E_NBR_OVERFLOW] = 0u;
+    d.err[MEL_E_NBR_NEED] = 0u;
+}
+// one thread per member: the new list's length, for the host (word 5)
+__global__ void readback_kernel(const mel_prox_job* J, int nj, const __grid_constant__ mel_prox_job one)
+{
+    const int k = blockIdx.x * blockDim.x + threadIdx.x;
+    if (k >= nj) return;
+    const mel_prox_job& j = J ? J[k] : one;
+    j.readback[5] = j.toff[j.ntask];
 }
 
 } // namespace mel
@@ -951,7 +1022,6 @@ static bool sync_failed(cudaStream_t s, int line)
 struct mel_prox_stage {
     char* h = nullptr; char* dv = nullptr; size_t cap = 0, used = 0;
     int* rb_h = nullptr; int* rb_d = nullptr; int rb_cap = 0;    // 8 words per member; rb_d[8 * rb_cap] = 0
-    const int* zero = nullptr;     // block prefix of a one-member launch (blocks start at 0)
     std::vector<std::pair<char*, char*>> retired;               // outgrown buffers, freed after a sync
 };
 
@@ -996,7 +1066,10 @@ static void* stage_upload(mel_prox_stage& S, const void* src, size_t bytes, cuda
 
 namespace {
 
-typedef void (*job_kernel_t)(const mel_prox_job*, const int*, int);
+typedef void (*job_kernel_t)(const mel_prox_job*, const int*, int, const mel_prox_job);
+
+// members of a launch: a table on the device, or the one member as the kernels' argument
+struct job_table { const mel_prox_job* J; mel_prox_job one; };
 
 struct run_ctx {
     mel_prox_stage& S;
@@ -1009,7 +1082,7 @@ size_t scan_scratch_ints(int n)
 {
     size_t t = 0;
     while (true) {
-        int nblk = (n + SCAN_BLOCK) / SCAN_BLOCK;
+        int nblk = (n + SCAN_ITEMS) / SCAN_ITEMS;
         t += (size_t)nblk + 1 + nblk + 2;
         if (nblk <= 1) break;
         n = nblk;
@@ -1017,23 +1090,39 @@ size_t scan_scratch_ints(int n)
     return t;
 }
 
-// kernel k over items[j] items of member j of the job table J (TPI threads per item)
-int launch_jobs(run_ctx& C, job_kernel_t k, const mel_prox_job* J, const std::vector<int>& items, int tpi)
+// kernel k over items[j] items of member j of the job table T (TPI threads per item)
+int launch_jobs(run_ctx& C, job_kernel_t k, const job_table& T, const std::vector<int>& items, int tpi, int threads = PROX_THREADS)
 {
     const int nj = (int)items.size();
-    const int per_block = PROX_THREADS / tpi;
+    const int per_block = threads / tpi;
     std::vector<int> bpre(nj + 1, 0);
     for (int j = 0; j < nj; j++) bpre[j + 1] = bpre[j] + (items[j] + per_block - 1) / per_block;
     if (bpre[nj] == 0) return MEL_OK;
-    const int* dp = nj == 1 ? C.S.zero : (const int*)stage_upload(C.S, bpre.data(), sizeof(int) * (nj + 1), C.s);
-    if (!dp) { mel_set_error("proximity staging upload failed"); return MEL_ERR_CUDA; }
-    k<<<bpre[nj], PROX_THREADS, 0, C.s>>>(J, dp, nj);
+    const int* dp = T.J ? (const int*)stage_upload(C.S, bpre.data(), sizeof(int) * (nj + 1), C.s) : nullptr;
+    if (T.J && !dp) { mel_set_error("proximity staging upload failed"); return MEL_ERR_CUDA; }
+    k<<<bpre[nj], threads, 0, C.s>>>(T.J, dp, nj, T.one);
     C.launches++;
     return MEL_OK;
 }
 
 // exclusive scans: req[j] scans in[0..n) into out[0..n] using the scratch ws (scan_scratch_ints(n))
 struct scan_req { const int* in; int* out; int n; int* ws; };
+// the jobs and block prefixes of a scan launch, as its argument or on the device
+bool scan_pack(run_ctx& C, const std::vector<mel_scan_job>& jobs, const std::vector<int>& bpre, mel::scan_args& A)
+{
+    memset(&A, 0, sizeof A);
+    A.nj = (int)jobs.size();
+    if (A.nj <= SCAN_INLINE) {
+        for (int j = 0; j < A.nj; j++) A.job[j] = jobs[j];
+        for (int j = 0; j <= A.nj; j++) A.pre[j] = bpre[j];
+        return true;
+    }
+    A.J = (const mel_scan_job*)stage_upload(C.S, jobs.data(), sizeof(mel_scan_job) * jobs.size(), C.s);
+    A.bpre = (const int*)stage_upload(C.S, bpre.data(), sizeof(int) * bpre.size(), C.s);
+    if (A.J && A.bpre) return true;
+    mel_set_error("proximity staging upload failed");
+    return false;
+}
 int scan_many(run_ctx& C, const std::vector<scan_req>& req)
 {
     if (req.empty()) return MEL_OK;
@@ -1042,7 +1131,7 @@ int scan_many(run_ctx& C, const std::vector<scan_req>& req)
     std::vector<int> bpre(nj + 1, 0), apre(1, 0);
     std::vector<scan_req> next;
     for (int j = 0; j < nj; j++) {
-        const int nblk = (req[j].n + SCAN_BLOCK) / SCAN_BLOCK;      // covers index n as well
+        const int nblk = (req[j].n + SCAN_ITEMS) / SCAN_ITEMS;      // covers index n as well
         jobs[j] = { req[j].in, req[j].out, req[j].n, req[j].ws };
         bpre[j + 1] = bpre[j] + nblk;
         if (nblk > 1) {                                              // block totals scanned the same way
@@ -1052,17 +1141,14 @@ int scan_many(run_ctx& C, const std::vector<scan_req>& req)
             apre.push_back(apre.back() + nblk);
         }
     }
-    const mel_scan_job* dj = (const mel_scan_job*)stage_upload(C.S, jobs.data(), sizeof(mel_scan_job) * nj, C.s);
-    const int* db = nj == 1 ? C.S.zero : (const int*)stage_upload(C.S, bpre.data(), sizeof(int) * (nj + 1), C.s);
-    if (!dj || !db) { mel_set_error("proximity staging upload failed"); return MEL_ERR_CUDA; }
-    mel::scan_block_kernel<<<bpre[nj], SCAN_BLOCK, 0, C.s>>>(dj, db, nj);
+    mel::scan_args A;
+    if (!scan_pack(C, jobs, bpre, A)) return MEL_ERR_CUDA;
+    mel::scan_block_kernel<<<bpre[nj], SCAN_BLOCK, 0, C.s>>>(A);
     C.launches++;
     if (next.empty()) return MEL_OK;
     if (int rc = scan_many(C, next)) return rc;
-    const mel_scan_job* da = (const mel_scan_job*)stage_upload(C.S, adds.data(), sizeof(mel_scan_job) * adds.size(), C.s);
-    const int* dap = adds.size() == 1 ? C.S.zero : (const int*)stage_upload(C.S, apre.data(), sizeof(int) * apre.size(), C.s);
-    if (!da || !dap) { mel_set_error("proximity staging upload failed"); return MEL_ERR_CUDA; }
-    mel::scan_add_kernel<<<apre.back(), SCAN_BLOCK, 0, C.s>>>(da, dap, (int)adds.size());
+    if (!scan_pack(C, adds, apre, A)) return MEL_ERR_CUDA;
+    mel::scan_add_kernel<<<apre.back(), SCAN_BLOCK, 0, C.s>>>(A);
     C.launches++;
     return MEL_OK;
 }
@@ -1076,12 +1162,11 @@ mel_prox_job make_job(const mel_prox_member& m, int* readback)
     j.aabb = P.aabb; j.shmin = P.shmin; j.shmax = P.shmax;
     j.nbr = P.nbr; j.nbn = P.nbn; j.nbr_cap = P.nbr_cap;
     j.ntask = P.ntask; j.nslot = P.nslot; j.have_old = m.d->ncont > 0 ? 1 : 0;
-    j.task = (int4*)P.task; j.tns = P.tns; j.tslot = P.tslot; j.tkey = P.tkey;
-    j.tcnt = P.tcnt; j.btask0 = P.btask0; j.scnt = P.scnt; j.bslot0 = P.bslot0;
-    j.slot_cnt = P.slot_cnt; j.slot_off = P.slot_off; j.inc_task = P.inc_task; j.tmap = P.tmap;
-    j.nzoff = P.nzoff; j.nzlist = P.nzlist; j.nnz = P.nnz;
+    j.btask0 = P.btask0; j.bslot0 = P.bslot0;
+    j.cand = (int4*)P.cand; j.cand_cap = P.cand_cap; j.ncand = P.ncand; j.ncont_new = P.ncont_new;
+    j.tcand = P.tcand; j.toff = P.toff; j.bucket = P.bucket; j.tkey = P.tkey;
+    j.inc_task = P.inc_task; j.inc_cnt = P.inc_cnt;
     j.inc_rng = P.inc_rng; j.b_inc0 = P.b_inc0; j.b_cont0 = P.b_cont0;
-    j.e_cnt = P.e_cnt; j.e_ptr = P.e_ptr; j.e_cur = P.e_cur; j.e_list = P.e_list;
     j.cont_new = P.cont_alt;
     j.readback = readback;
     j.cl_on = P.cl_on; j.cl_T = P.cl_T; j.cl_ncx = P.cl_ncx; j.cl_h = P.cl_h; j.cl_hx = P.cl_hx;
@@ -1089,15 +1174,17 @@ mel_prox_job make_job(const mel_prox_member& m, int* readback)
     return j;
 }
 
-// job table of the members idx (read-back words by member index) on the device
-const mel_prox_job* upload_jobs(run_ctx& C, mel_prox_member* m, const std::vector<int>& idx,
-                                std::vector<mel_prox_job>& hj)
+// job table of the members idx (read-back words by member index)
+bool make_jobs(run_ctx& C, mel_prox_member* m, const std::vector<int>& idx, std::vector<mel_prox_job>& hj, job_table& T)
 {
     hj.clear();
     for (int i : idx) hj.push_back(make_job(m[i], C.S.rb_d + 8 * i));
-    const mel_prox_job* J = (const mel_prox_job*)stage_upload(C.S, hj.data(), sizeof(mel_prox_job) * hj.size(), C.s);
-    if (!J) mel_set_error("proximity staging upload failed");
-    return J;
+    T.J = nullptr;
+    T.one = hj[0];
+    if (hj.size() == 1) return true;
+    T.J = (const mel_prox_job*)stage_upload(C.S, hj.data(), sizeof(mel_prox_job) * hj.size(), C.s);
+    if (!T.J) mel_set_error("proximity staging upload failed");
+    return T.J != nullptr;
 }
 
 template <typename F>
@@ -1106,24 +1193,6 @@ std::vector<int> items_of(const std::vector<mel_prox_job>& hj, F&& f)
     std::vector<int> v;
     for (const mel_prox_job& j : hj) v.push_back(f(j));
     return v;
-}
-
-// the per-entry index of each member's current list (d.cont, d.ncont) and b_cont0.  The members'
-// e_list must hold ncont + 1 entries and their scan scratch scan_scratch_ints(ne); J / hj is the
-// job table of the members idx.
-int index_stage(run_ctx& C, mel_prox_member* m, const std::vector<int>& idx, const mel_prox_job* J,
-                const std::vector<mel_prox_job>& hj)
-{
-    using namespace mel;
-    int rc;
-    if ((rc = launch_jobs(C, body_range_kernel, J, items_of(hj, [](const mel_prox_job& j) { return j.d.nb + 1; }), 1))) return rc;
-    if ((rc = launch_jobs(C, zero_ecnt_kernel, J, items_of(hj, [](const mel_prox_job& j) { return j.d.ne + 1; }), 1))) return rc;
-    if ((rc = launch_jobs(C, entry_count_kernel, J, items_of(hj, [](const mel_prox_job& j) { return j.d.ncont; }), 1))) return rc;
-    std::vector<scan_req> sc;
-    for (int i : idx) sc.push_back({ m[i].P->e_cnt, m[i].P->e_ptr, m[i].d->ne, m[i].P->scan_ws });
-    if ((rc = scan_many(C, sc))) return rc;
-    if ((rc = launch_jobs(C, copy_eptr_kernel, J, items_of(hj, [](const mel_prox_job& j) { return j.d.ne + 1; }), 1))) return rc;
-    return launch_jobs(C, entry_index_kernel, J, items_of(hj, [](const mel_prox_job& j) { return j.d.nb; }), 32);
 }
 
 bool stage_ready(mel_prox_stage*& stage, int n)
@@ -1138,7 +1207,6 @@ bool stage_ready(mel_prox_stage*& stage, int n)
     if (cudaMallocHost(&S.rb_h, sizeof(int) * 8 * (size_t)cap) != cudaSuccess) return false;
     if (cudaMalloc(&S.rb_d, sizeof(int) * (8 * (size_t)cap + 1)) != cudaSuccess) return false;
     if (cudaMemset(S.rb_d, 0, sizeof(int) * (8 * (size_t)cap + 1)) != cudaSuccess) return false;
-    S.zero = S.rb_d + 8 * (size_t)cap;
     S.rb_cap = cap;
     return true;
 }
@@ -1164,53 +1232,43 @@ int mel_run_proximity_many(mel_prox_member* m, int n, mel_prox_stage*& stage, in
     run_ctx C{ *stage, s, 0 };
     std::vector<mel_prox_job> hj;
     std::vector<int> act;
+    job_table T;
     int rc;
     for (int i = 0; i < n; i++) {
         m[i].rc = MEL_OK;
         m[i].msg.clear();
         mel_prox_state& P = *m[i].P;
-        const int nsc = std::max(m[i].d->nb, m[i].d->ne);
-        if (ensure((void**)&P.scan_ws, &P.scan_ws_bytes, sizeof(int) * scan_scratch_ints(std::max(nsc, P.cl_T)))) return MEL_ERR_OOM;
+        if (ensure((void**)&P.scan_ws, &P.scan_ws_bytes, sizeof(int) * scan_scratch_ints(std::max(m[i].d->nb, P.cl_T)))) return MEL_ERR_OOM;
         act.push_back(i);
     }
     // 1. border boxes and segment-block boxes
-    const mel_prox_job* J = upload_jobs(C, m, act, hj);
-    if (!J) return MEL_ERR_CUDA;
-    if ((rc = launch_jobs(C, aabb_kernel, J, items_of(hj, [](const mel_prox_job& j) { return j.d.nbd; }), 32))) return rc;
-    if ((rc = launch_jobs(C, segblock_kernel, J, items_of(hj, [](const mel_prox_job& j) { return j.d.nblk; }), 1))) return rc;
-    if ((rc = launch_jobs(C, superblock_kernel, J, items_of(hj, [](const mel_prox_job& j) { return j.d.nsblk; }), 1))) return rc;
+    if (!make_jobs(C, m, act, hj, T)) return MEL_ERR_CUDA;
+    if ((rc = launch_jobs(C, boxes_kernel, T, items_of(hj, [](const mel_prox_job& j) { return j.d.nbd + j.d.nsblk + (j.cl_on ? j.cl_T / 32 + 1 : 0); }), 32))) return rc;
     // 2. neighbours and the task counts; a member whose neighbour lists overflow grows them and
     //    repeats this stage (up to 4 attempts)
     std::vector<int> pend = act;
     for (int attempt = 0; attempt < 4 && !pend.empty(); attempt++) {
-        J = upload_jobs(C, m, pend, hj);
-        if (!J) return MEL_ERR_CUDA;
         const int np = (int)pend.size();
-        nbr_clear_kernel<<<(np + 127) / 128, 128, 0, s>>>(J, np); C.launches++;
         // members with the cell list: bucket the border boxes (counting sort), then query; the
         // others: all pairs of bodies
         bool any_cl = false, any_ap = false;
+        if (attempt > 0) {
+            if (!make_jobs(C, m, pend, hj, T)) return MEL_ERR_CUDA;
+            nbr_clear_kernel<<<(np + 127) / 128, 128, 0, s>>>(T.J, np, T.one); C.launches++;
+            if ((rc = launch_jobs(C, cl_zero_kernel, T, items_of(hj, [](const mel_prox_job& j) { return j.cl_on ? j.cl_T + 1 : 0; }), 1))) return rc;
+        }
         for (const mel_prox_job& jj : hj) { any_cl = any_cl || jj.cl_on; any_ap = any_ap || !jj.cl_on; }
         if (any_cl) {
-            if ((rc = launch_jobs(C, cl_zero_kernel, J, items_of(hj, [](const mel_prox_job& j) { return j.cl_on ? j.cl_T + 1 : 0; }), 1))) return rc;
-            if ((rc = launch_jobs(C, cl_count_kernel, J, items_of(hj, [](const mel_prox_job& j) { return j.cl_on ? j.d.nbd : 0; }), 1))) return rc;
+            if ((rc = launch_jobs(C, cl_count_kernel, T, items_of(hj, [](const mel_prox_job& j) { return j.cl_on ? j.d.nbd : 0; }), 1))) return rc;
             std::vector<scan_req> sc;
             for (int i : pend) if (m[i].P->cl_on) sc.push_back({ m[i].P->cl_cnt, m[i].P->cl_start, m[i].P->cl_T, m[i].P->scan_ws });
             if ((rc = scan_many(C, sc))) return rc;
-            if ((rc = launch_jobs(C, cl_fill_kernel, J, items_of(hj, [](const mel_prox_job& j) { return j.cl_on ? j.d.nbd : 0; }), 1))) return rc;
-            if ((rc = launch_jobs(C, cl_neighbour_kernel, J, items_of(hj, [](const mel_prox_job& j) { return j.cl_on ? j.d.nb : 0; }), 32))) return rc;
+            if ((rc = launch_jobs(C, cl_fill_kernel, T, items_of(hj, [](const mel_prox_job& j) { return j.cl_on ? j.d.nbd : 0; }), 1))) return rc;
+            if ((rc = launch_jobs(C, cl_neighbour_kernel, T, items_of(hj, [](const mel_prox_job& j) { return j.cl_on ? j.d.nb : 0; }), 32))) return rc;
         }
         if (any_ap)
-            if ((rc = launch_jobs(C, neighbour_kernel, J, items_of(hj, [](const mel_prox_job& j) { return j.cl_on ? 0 : j.d.nb; }), 32))) return rc;
-        if ((rc = launch_jobs(C, task_count_kernel, J, items_of(hj, [](const mel_prox_job& j) { return j.d.nb; }), 1))) return rc;
-        std::vector<scan_req> sc1, sc2;
-        for (int i : pend) {
-            sc1.push_back({ m[i].P->tcnt, m[i].P->btask0, m[i].d->nb, m[i].P->scan_ws });
-            sc2.push_back({ m[i].P->scnt, m[i].P->bslot0, m[i].d->nb, m[i].P->scan_ws });
-        }
-        if ((rc = scan_many(C, sc1))) return rc;
-        if ((rc = scan_many(C, sc2))) return rc;
-        readback_kernel<<<(np + 127) / 128, 128, 0, s>>>(J, np, 0); C.launches++;
+            if ((rc = launch_jobs(C, neighbour_kernel, T, items_of(hj, [](const mel_prox_job& j) { return j.cl_on ? 0 : j.d.nb; }), 32))) return rc;
+        tasks_kernel<<<np, 1024, 0, s>>>(T.J, np, T.one); C.launches++;
         if ((rc = launch_status(__LINE__))) return rc;
         if (!read_back(C, n)) return MEL_ERR_CUDA;
         std::vector<int> retry;
@@ -1245,89 +1303,74 @@ int mel_run_proximity_many(mel_prox_member* m, int n, mel_prox_stage*& stage, in
     act.clear();
     for (int i = 0; i < n; i++) if (m[i].rc == MEL_OK) act.push_back(i);
     if (act.empty()) { launches += C.launches; return launch_status(__LINE__); }
-    // 3. the task list and the candidate count of every slot
-    for (int i : act) {
-        mel_prox_state& P = *m[i].P;
-        const size_t nt = (size_t)P.ntask + 1, ns = (size_t)P.nslot + 1;
-        if (ensure((void**)&P.task, &P.task_bytes, sizeof(int4) * nt)) return MEL_ERR_OOM;
-        if (ensure((void**)&P.tns, &P.tns_bytes, sizeof(int) * nt)) return MEL_ERR_OOM;
-        if (ensure((void**)&P.tslot, &P.tslot_bytes, sizeof(int) * nt)) return MEL_ERR_OOM;
-        if (ensure((void**)&P.tkey, &P.tkey_bytes, sizeof(int) * nt)) return MEL_ERR_OOM;
-        if (ensure((void**)&P.inc_task, &P.inc_task_bytes, sizeof(int) * 2 * nt)) return MEL_ERR_OOM;
-        if (ensure((void**)&P.slot_cnt, &P.slot_bytes, sizeof(int) * ns)) return MEL_ERR_OOM;
-        if (ensure((void**)&P.slot_off, &P.slot_off_bytes, sizeof(int) * ns)) return MEL_ERR_OOM;
-        if (ensure((void**)&P.tmap, &P.tmap_bytes, sizeof(int) * ns)) return MEL_ERR_OOM;
-        if (ensure((void**)&P.nzoff, &P.nzoff_bytes, sizeof(int) * ns)) return MEL_ERR_OOM;
-        if (ensure((void**)&P.nzlist, &P.nzlist_bytes, sizeof(int) * ns)) return MEL_ERR_OOM;
-        const int nsc = std::max(std::max(m[i].d->nb, m[i].d->ne), P.nslot);
-        if (ensure((void**)&P.scan_ws, &P.scan_ws_bytes, sizeof(int) * scan_scratch_ints(std::max(nsc, P.cl_T)))) return MEL_ERR_OOM;
-    }
-    J = upload_jobs(C, m, act, hj);
-    if (!J) return MEL_ERR_CUDA;
-    if ((rc = launch_jobs(C, zero_tcnt_kernel, J, items_of(hj, [](const mel_prox_job& j) { return j.d.nb + 1; }), 1))) return rc;
-    if ((rc = launch_jobs(C, task_fill_kernel, J, items_of(hj, [](const mel_prox_job& j) { return j.ntask > 0 ? j.d.nb : 0; }), 1))) return rc;
-    if ((rc = launch_jobs(C, slot_task_kernel, J, items_of(hj, [](const mel_prox_job& j) { return j.ntask; }), 32))) return rc;
-    if ((rc = launch_jobs(C, count_kernel, J, items_of(hj, [](const mel_prox_job& j) { return j.ntask > 0 ? j.nslot : 0; }), 1))) return rc;
-    {
-        std::vector<scan_req> sc, sz;
-        for (int i : act) {
-            sc.push_back({ m[i].P->slot_cnt, m[i].P->slot_off, m[i].P->nslot, m[i].P->scan_ws });
-            sz.push_back({ m[i].P->slot_cnt, m[i].P->nzoff, m[i].P->nslot, m[i].P->scan_ws });
+    // 3. the candidates and the tasks' offsets in the new list; members whose candidates outgrow their
+    //    list grow it and repeat this stage
+    pend = act;
+    while (!pend.empty()) {
+        for (int i : pend) {
+            mel_prox_state& P = *m[i].P;
+            const size_t nt = (size_t)P.ntask + 2;
+            if (ensure((void**)&P.tcand, &P.tcand_bytes, sizeof(int) * nt)) return MEL_ERR_OOM;
+            if (ensure((void**)&P.toff, &P.toff_bytes, sizeof(int) * nt)) return MEL_ERR_OOM;
+            if (ensure((void**)&P.tkey, &P.tkey_bytes, sizeof(int) * nt)) return MEL_ERR_OOM;
+            if (ensure((void**)&P.cand, &P.cand_bytes, sizeof(int4) * 2 * 1024)) return MEL_ERR_OOM;
+            P.cand_cap = (int)std::min<size_t>(P.cand_bytes / (2 * sizeof(int4)), 0x7fffffff);
+            if (ensure((void**)&P.scan_ws, &P.scan_ws_bytes, sizeof(int) * scan_scratch_ints(std::max(std::max(m[i].d->nb, P.ntask), P.cl_T)))) return MEL_ERR_OOM;
         }
+        if (!make_jobs(C, m, pend, hj, T)) return MEL_ERR_CUDA;
+        if ((rc = launch_jobs(C, clear_kernel, T, items_of(hj, [](const mel_prox_job& j) { return std::max(j.ntask, j.d.nb) + 1; }), 1))) return rc;
+        if ((rc = launch_jobs(C, find_kernel, T, items_of(hj, [](const mel_prox_job& j) { return j.ntask > 0 ? j.nslot : 0; }), 1, FIND_THREADS))) return rc;
+        std::vector<scan_req> sc;
+        for (int i : pend) sc.push_back({ m[i].P->tcand, m[i].P->toff, m[i].P->ntask, m[i].P->scan_ws });
         if ((rc = scan_many(C, sc))) return rc;
-        // the write pass visits only the slots with candidates (a few in a thousand)
-        if ((rc = launch_jobs(C, nz_flag_kernel, J, items_of(hj, [](const mel_prox_job& j) { return j.ntask > 0 ? j.nslot : 0; }), 1))) return rc;
-        if ((rc = scan_many(C, sz))) return rc;
-        if ((rc = launch_jobs(C, nz_list_kernel, J, items_of(hj, [](const mel_prox_job& j) { return j.ntask > 0 ? j.nslot : 0; }), 1))) return rc;
+        readback_kernel<<<((int)pend.size() + 127) / 128, 128, 0, s>>>(T.J, (int)pend.size(), T.one); C.launches++;
+        if ((rc = launch_status(__LINE__))) return rc;
+        if (!read_back(C, n)) return MEL_ERR_CUDA;
+        std::vector<int> retry;
+        for (int i : pend) {
+            mel_prox_state& P = *m[i].P;
+            P.ncont_new = C.S.rb_h[8 * i + 5];
+            if (P.ncont_new <= P.cand_cap) continue;
+            if (ensure((void**)&P.cand, &P.cand_bytes, sizeof(int4) * 2 * (size_t)P.ncont_new)) return MEL_ERR_OOM;
+            retry.push_back(i);
+        }
+        pend = retry;
     }
-    readback_kernel<<<((int)act.size() + 127) / 128, 128, 0, s>>>(J, (int)act.size(), 1); C.launches++;
-    if ((rc = launch_status(__LINE__))) return rc;
-    if (!read_back(C, n)) return MEL_ERR_CUDA;
     // 4. the new list, written into the spare buffer with history inherited from the current one
     for (int i : act) {
         mel_prox_state& P = *m[i].P;
-        const size_t total = (size_t)C.S.rb_h[8 * i + 5];
-        P.nnz = C.S.rb_h[8 * i + 6];
+        const size_t total = (size_t)P.ncont_new;
         if (ensure((void**)&P.cont_alt, &P.cont_alt_bytes, sizeof(mel_contact) * (total + 1))) return MEL_ERR_OOM;
         if (ensure((void**)&P.cont_w, &P.cont_w_bytes, sizeof(double) * (total + 1))) return MEL_ERR_OOM;
         if (ensure((void**)&P.cont_rt, &P.cont_rt_bytes, 6 * sizeof(double) * (total + 1))) return MEL_ERR_OOM;
-        if (ensure((void**)&P.inc_rng, &P.inc_rng_bytes, sizeof(int2) * ((size_t)P.ntask + 1))) return MEL_ERR_OOM;
+        if (ensure((void**)&P.inc_rng, &P.inc_rng_bytes, sizeof(int2) * (total + 1))) return MEL_ERR_OOM;
+        if (ensure((void**)&P.inc_task, &P.inc_task_bytes, sizeof(int) * (total + 1))) return MEL_ERR_OOM;
+        if (ensure((void**)&P.bucket, &P.bucket_bytes, sizeof(int) * (total + 1))) return MEL_ERR_OOM;
+        m[i].d->cont_w = P.cont_w;
+        m[i].d->cont_rt = P.cont_rt;
+        m[i].d->inc_rng = P.inc_rng;
+        m[i].d->b_inc0 = P.b_inc0;
+        m[i].d->b_cont0 = P.b_cont0;
     }
-    J = upload_jobs(C, m, act, hj);
-    if (!J) return MEL_ERR_CUDA;
-    if ((rc = launch_jobs(C, write_kernel, J, items_of(hj, [](const mel_prox_job& j) { return j.ntask > 0 ? j.nnz : 0; }), 1))) return rc;
+    if (!make_jobs(C, m, act, hj, T)) return MEL_ERR_CUDA;
+    if ((rc = launch_jobs(C, bucket_kernel, T, items_of(hj, [](const mel_prox_job& j) { return j.ncont_new; }), 1))) return rc;
+    if ((rc = launch_jobs(C, write_kernel, T, items_of(hj, [](const mel_prox_job& j) { return j.ncont_new; }), 32))) return rc;
+    // 5. incoming ranges in send order, contact ranges, vgapn/vgapt carry of new elements
+    {
+        std::vector<scan_req> sc;
+        for (int i : act) sc.push_back({ m[i].P->inc_cnt, m[i].P->b_inc0, m[i].d->nb, m[i].P->scan_ws });
+        if ((rc = scan_many(C, sc))) return rc;
+    }
+    if ((rc = launch_jobs(C, inc_fill_kernel, T, items_of(hj, [](const mel_prox_job& j) { return j.ncont_new > 0 ? j.ntask : 0; }), 1))) return rc;
     for (int i : act) {
         mel_dev& d = *m[i].d;
         mel_prox_state& P = *m[i].P;
-        mel_contact* old = d.cont;
-        const size_t old_bytes = P.cont_bytes;
-        d.cont = P.cont_alt; P.cont_bytes = P.cont_alt_bytes;
-        P.cont_alt = old; P.cont_alt_bytes = old_bytes;
-        d.ncont = C.S.rb_h[8 * i + 5];
-        d.cont_w = P.cont_w;
-        d.cont_rt = P.cont_rt;
-        d.inc_rng = P.inc_rng;
-        d.b_inc0 = P.b_inc0;
-        d.b_cont0 = P.b_cont0;
-        // the old index is read by the write pass just launched; freeing it waits for that pass
-        if (ensure((void**)&P.e_list, &P.e_list_bytes, sizeof(int) * ((size_t)d.ncont + 1))) return MEL_ERR_OOM;
+        std::swap(d.cont, P.cont_alt);
+        std::swap(P.cont_bytes, P.cont_alt_bytes);
+        d.ncont = P.ncont_new;
     }
-    J = upload_jobs(C, m, act, hj);
-    if (!J) return MEL_ERR_CUDA;
-    if ((rc = launch_jobs(C, zero_contw_kernel, J, items_of(hj, [](const mel_prox_job& j) { return j.d.ncont + 1; }), 1))) return rc;
-    // 5. incoming ranges in send order
-    {
-        std::vector<scan_req> sc;
-        for (int i : act) sc.push_back({ m[i].P->tcnt, m[i].P->b_inc0, m[i].d->nb, m[i].P->scan_ws });
-        if ((rc = scan_many(C, sc))) return rc;
-    }
-    if ((rc = launch_jobs(C, copy_inc_kernel, J, items_of(hj, [](const mel_prox_job& j) { return j.ntask > 0 ? j.d.nb : 0; }), 1))) return rc;
-    if ((rc = launch_jobs(C, inc_fill_kernel, J, items_of(hj, [](const mel_prox_job& j) { return j.ntask; }), 1))) return rc;
-    if ((rc = launch_jobs(C, inc_sort_kernel, J, items_of(hj, [](const mel_prox_job& j) { return j.ntask > 0 ? j.d.nb : 0; }), 32))) return rc;
-    if ((rc = launch_jobs(C, inc_range_kernel, J, items_of(hj, [](const mel_prox_job& j) { return j.ntask; }), 1))) return rc;
-    // 6. per-entry index of the new list; vgapn/vgapt carry of new elements
-    if ((rc = index_stage(C, m, act, J, hj))) return rc;
-    if ((rc = launch_jobs(C, carry_kernel, J, items_of(hj, [](const mel_prox_job& j) { return j.d.nb; }), 32))) return rc;
+    if (!make_jobs(C, m, act, hj, T)) return MEL_ERR_CUDA;
+    if ((rc = launch_jobs(C, bodies_kernel, T, items_of(hj, [](const mel_prox_job& j) { return j.d.nb; }), 32))) return rc;
     launches += C.launches;
     return launch_status(__LINE__);
 }
@@ -1367,18 +1410,15 @@ int mel_index_external(mel_dev& d, mel_prox_state& P, const mel_contact* host_li
     d.inc_rng = P.inc_rng;
     d.b_inc0 = P.b_inc0;
     d.b_cont0 = P.b_cont0;
-    if (ensure((void**)&P.e_list, &P.e_list_bytes, sizeof(int) * ((size_t)d.ncont + 1))) return MEL_ERR_OOM;
-    if (ensure((void**)&P.scan_ws, &P.scan_ws_bytes, sizeof(int) * scan_scratch_ints(std::max(std::max(d.nb, d.ne), P.cl_T)))) return MEL_ERR_OOM;
     if (!stage_ready(P.stage, 1)) { mel_set_error("proximity read-back buffers could not be allocated"); return MEL_ERR_OOM; }
     mel_prox_member m;
     m.d = &d;
     m.P = &P;
     run_ctx C{ *P.stage, s, 0 };
     std::vector<mel_prox_job> hj;
-    const std::vector<int> idx{ 0 };
-    const mel_prox_job* J = upload_jobs(C, &m, idx, hj);
-    if (!J) return MEL_ERR_CUDA;
-    int rc = index_stage(C, &m, idx, J, hj);
+    job_table T;
+    if (!make_jobs(C, &m, std::vector<int>{ 0 }, hj, T)) return MEL_ERR_CUDA;
+    int rc = launch_jobs(C, mel::body_range_kernel, T, std::vector<int>{ d.nb + 1 }, 1);
     P.launches += C.launches;
     if (rc) return rc;
     if (sync_failed(s, __LINE__)) return MEL_ERR_CUDA;

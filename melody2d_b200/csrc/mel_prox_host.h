@@ -11,23 +11,18 @@ struct mel_prox_state {
     int nbr_cap = MEL_NBR_CAP_DEFAULT;
     int* nbr = nullptr; int* nbn = nullptr;
     double* aabb = nullptr; int* shmin = nullptr; int* shmax = nullptr;
-    void* task = nullptr; size_t task_bytes = 0;            // int4 per task
-    int* tns = nullptr; size_t tns_bytes = 0;               // slave border nodes per task
-    int* tslot = nullptr; size_t tslot_bytes = 0;           // first slot of each task
-    int* tkey = nullptr; size_t tkey_bytes = 0;             // master body of each task
-    int* tcnt = nullptr; int* btask0 = nullptr;             // per body: task count, first task
-    int* scnt = nullptr; int* bslot0 = nullptr;             // per body: slot count, first slot
-    int* inc_task = nullptr; size_t inc_task_bytes = 0;
-    int* slot_cnt = nullptr; size_t slot_bytes = 0;
-    int* slot_off = nullptr; size_t slot_off_bytes = 0;
-    int* tmap = nullptr; size_t tmap_bytes = 0;             // task of each slot
-    int* nzoff = nullptr; size_t nzoff_bytes = 0;           // slots with candidates: offsets, list
-    int* nzlist = nullptr; size_t nzlist_bytes = 0;
-    int nnz = 0;
+    int* btask0 = nullptr; int* bslot0 = nullptr;           // per body: first task, first slot
+    void* cand = nullptr; size_t cand_bytes = 0;            // two int4 per candidate, in any order
+    int cand_cap = 0, ncont_new = 0;                        // room for candidates, and how many were found
+    int* ncand = nullptr;
+    int* tcand = nullptr; size_t tcand_bytes = 0;           // candidates per task
+    int* toff = nullptr; size_t toff_bytes = 0;             // first contact of each task in the new list
+    int* tkey = nullptr; size_t tkey_bytes = 0;             // master body of each task with contacts
+    int* bucket = nullptr; size_t bucket_bytes = 0;         // candidates by task
+    int* inc_task = nullptr; size_t inc_task_bytes = 0;     // tasks by master body
+    int* inc_cnt = nullptr;                                 // per master body
     int2* inc_rng = nullptr; size_t inc_rng_bytes = 0;
     int* b_inc0 = nullptr; int* b_cont0 = nullptr;
-    int* e_cnt = nullptr; int* e_ptr = nullptr; int* e_cur = nullptr;
-    int* e_list = nullptr; size_t e_list_bytes = 0;
     size_t cont_bytes = 0;
     mel_contact* cont_alt = nullptr; size_t cont_alt_bytes = 0;
     double* cont_w = nullptr; size_t cont_w_bytes = 0;
@@ -55,12 +50,10 @@ struct mel_prox_job {
     double* aabb; int* shmin; int* shmax;
     int* nbr; int* nbn; int nbr_cap;
     int ntask, nslot, have_old;
-    int4* task; int* tns; int* tslot; int* tkey;
-    int* tcnt; int* btask0; int* scnt; int* bslot0;
-    int* slot_cnt; int* slot_off; int* inc_task; int* tmap;
-    int* nzoff; int* nzlist; int nnz;
+    int *btask0, *bslot0;
+    int4* cand; int cand_cap, ncont_new; int* ncand;
+    int *tcand, *toff, *tkey, *bucket, *inc_task, *inc_cnt;
     int2* inc_rng; int* b_inc0; int* b_cont0;
-    int* e_cnt; int* e_ptr; int* e_cur; int* e_list;
     mel_contact* cont_new;        // the list being written (write stage)
     int* readback;                // this member's words of the run's read-back array
     int cl_on, cl_T, cl_ncx;      // cell-list broad phase (mel_prox_state)
