@@ -235,8 +235,11 @@ void mel_launch_czm_init(const mel_dev& d, cudaStream_t s);
 void mel_launch_body(const mel_dev& d, int parity, int nblocks, size_t smem, cudaStream_t s, int nwide = 0);
 // one half-step of Solver_step (d.phase 1 or 2): T0 = Time, Tf = the time the forces see
 void mel_launch_body_adaptive(const mel_dev& d, double T0, double Tf, int nblocks, size_t smem, cudaStream_t s, int nwide = 0);
+// device-to-device copies of up to 16 arrays of 8-byte words by one launch
+struct mel_copy_list { int n; const void* src[16]; void* dst[16]; size_t words[16]; };
+void mel_launch_copy_many(const mel_copy_list& L, cudaStream_t s);
 // Solver_step's error and mass sums over the bodies in order (Code/Solver.h:289-331): out =
-// {mean_error, max_error, total_mass, max_mass}
+// {mean_error, max_error, total_mass, max_mass}, then the MEL_E_NWORDS error words
 void mel_launch_error_reduce(const mel_dev& d, double* out, cudaStream_t s);
 // Update_bc(T) of every body's driven degrees of freedom (mel_dev::drv)
 void mel_launch_drivendof(const mel_dev& d, double T, cudaStream_t s);

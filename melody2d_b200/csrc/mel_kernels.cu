@@ -13,6 +13,7 @@
 // internal forces, contact list order then send order for contact forces), so with identical inputs
 // the FP64 path reproduces the reference's values exactly; this file is compiled with
 // -fmad=false.
+#include <algorithm>
 #include <cstdio>
 #include <mutex>
 #include "mel_internal.h"
@@ -1783,6 +1784,7 @@ __global__ void __launch_bounds__(MEL_BODY_THREADS, 2) body_kernel_adaptive(cons
 {
     extern __shared__ __align__(16) char smem[];
     body_cta<MX, true>(d, blockIdx.x, Tf, smem, T0);
+    grid_wait();
 }
 
 // The wide bodies b_order[first + i]; the step's end time is written here when the launch above
@@ -1803,28 +1805,48 @@ __global__ void __launch_bounds__(MEL_BODY_THREADS, 2) body_kernel_adaptive_wide
     wide_body_cta<MX, true>(d, first + blockIdx.x, Tf, smem, T0);
 }
 
-// Solver_step's sums over bodies in body order (Code/Solver.h:289-331)
-__global__ void error_reduce_kernel(const __grid_constant__ mel_dev d, double* out)
+// Solver_step's sums over bodies in body order (Code/Solver.h:289-331): a warp reads 32 bodies at a
+// time, its first lanes add them up in order.  The device error words follow in out[4..]
+__global__ void __launch_bounds__(32) error_reduce_kernel(const __grid_constant__ mel_dev d, double* out)
 {
-    if (threadIdx.x != 0 || blockIdx.x != 0) return;
+    const int lane = threadIdx.x;
     double mean = 0., mx = 0., tm = 0., mm = 0.;
     int nnodes = 0;
     const bool ms = d.solver == MEL_SOLVER_MASS_SCALING || d.solver == MEL_SOLVER_ADAPTIVE_MASS_SCALING;
-    for (int i = 0; i < d.nb; i++) {
-        if (d.b_status[i] == MEL_STATUS_INACTIVE) continue;
-        mean += d.terr[i];
-        nnodes += d.b_node0[i + 1] - d.b_node0[i];
-        if (d.merr[i] > mx) mx = d.merr[i];
+    for (int base = 0; base < d.nb; base += 32) {
+        const int i = base + lane;
+        const bool on = i < d.nb && d.b_status[min(i, d.nb - 1)] != MEL_STATUS_INACTIVE;
+        double te = 0., me = 0., bm = 0., inv = 0.;
+        int nn = 0;
+        if (on) {
+            te = d.terr[i];
+            me = d.merr[i];
+            nn = d.b_node0[i + 1] - d.b_node0[i];
+            if (ms) { bm = d.bmms[i]; inv = d.rg[MEL_RIGID_NF * i + MEL_RG_INV_MASS]; }
+        }
+        for (unsigned m = __ballot_sync(0xffffffffu, on); m; m &= m - 1) {      // (equal in all lanes)
+            const int l = __ffs(m) - 1;
+            mean += __shfl_sync(0xffffffffu, te, l);
+            nnodes += __shfl_sync(0xffffffffu, nn, l);
+            const double e = __shfl_sync(0xffffffffu, me, l), w = __shfl_sync(0xffffffffu, bm, l);
+            const double wi = w * __shfl_sync(0xffffffffu, inv, l);
+            if (e > mx) mx = e;
+            if (ms) { tm += w; if (wi > mm) mm = wi; }
+        }
     }
     mean /= nnodes;
-    if (ms)
-        for (int i = 0; i < d.nb; i++) {
-            if (d.b_status[i] == MEL_STATUS_INACTIVE) continue;
-            tm += d.bmms[i];
-            const double inv = d.rg[MEL_RIGID_NF * i + MEL_RG_INV_MASS];
-            if (d.bmms[i] * inv > mm) mm = d.bmms[i] * inv;
-        }
-    out[0] = mean; out[1] = mx; out[2] = tm; out[3] = mm;
+    if (lane == 0) { out[0] = mean; out[1] = mx; out[2] = tm; out[3] = mm; }
+    if (lane < MEL_E_NWORDS) reinterpret_cast<unsigned*>(out + 4)[lane] = d.err[lane];
+}
+
+// copies of several arrays by one launch (8-byte words); a Solver_step snapshot is fifteen of them
+__global__ void __launch_bounds__(256) copy_many_kernel(const __grid_constant__ mel_copy_list L)
+{
+    for (int k = 0; k < L.n; k++) {
+        const unsigned long long* s = static_cast<const unsigned long long*>(L.src[k]);
+        unsigned long long* t = static_cast<unsigned long long*>(L.dst[k]);
+        for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < L.words[k]; i += (size_t)gridDim.x * blockDim.x) t[i] = s[i];
+    }
 }
 
 // ---- batches: several independent models (samples) advanced by the same launches -----------
@@ -2134,13 +2156,23 @@ void mel_launch_body(const mel_dev& d, int parity, int nblocks, size_t smem, cud
 void mel_launch_body_adaptive(const mel_dev& d, double T0, double Tf, int nblocks, size_t smem, cudaStream_t s, int nwide)
 {
     if (nblocks > 0) {
-        if (d.precision == MEL_PREC_MIXED) mel::body_kernel_adaptive<true><<<nblocks, MEL_BODY_THREADS, smem, s>>>(d, T0, Tf);
-        else mel::body_kernel_adaptive<false><<<nblocks, MEL_BODY_THREADS, smem, s>>>(d, T0, Tf);
+        auto body = d.precision == MEL_PREC_MIXED ? mel::body_kernel_adaptive<true> : mel::body_kernel_adaptive<false>;
+        if (d.ncont + d.ne > 0) launch_dependent(body, nblocks, MEL_BODY_THREADS, smem, s, d, T0, Tf);
+        else body<<<nblocks, MEL_BODY_THREADS, smem, s>>>(d, T0, Tf);
     }
     if (nwide > 0) {
         if (d.precision == MEL_PREC_MIXED) mel::body_kernel_adaptive_wide<true><<<nwide, MEL_BODY_THREADS, smem, s>>>(d, T0, Tf, nblocks);
         else mel::body_kernel_adaptive_wide<false><<<nwide, MEL_BODY_THREADS, smem, s>>>(d, T0, Tf, nblocks);
     }
+}
+
+void mel_launch_copy_many(const mel_copy_list& L, cudaStream_t s)
+{
+    size_t most = 0;
+    for (int k = 0; k < L.n; k++) most = std::max(most, L.words[k]);
+    if (most == 0) return;
+    const int grid = (int)std::min<size_t>((most + 255) / 256, 148 * 8);
+    mel::copy_many_kernel<<<grid, 256, 0, s>>>(L);
 }
 
 void mel_launch_error_reduce(const mel_dev& d, double* out, cudaStream_t s)

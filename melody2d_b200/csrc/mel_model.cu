@@ -882,10 +882,12 @@ static mel_status build(mel_handle* h, const mel_model_desc* d, const mel_option
 // ---------------------------------------------------------------------------------------------
 // set-up and stepping
 // ---------------------------------------------------------------------------------------------
-static mel_status check_errors(mel_handle* h)
+// the outcome that the device error words name; `words`: read already, else they are read here
+static mel_status check_errors(mel_handle* h, const unsigned* words = nullptr)
 {
     unsigned w[MEL_E_NWORDS];
-    if (cudaMemcpy(w, h->d.err, sizeof w, cudaMemcpyDeviceToHost) != cudaSuccess) { mel_set_cuda_error(cudaGetLastError(), "err", __FILE__, __LINE__); return MEL_ERR_CUDA; }
+    if (words) memcpy(w, words, sizeof w);
+    else if (cudaMemcpy(w, h->d.err, sizeof w, cudaMemcpyDeviceToHost) != cudaSuccess) { mel_set_cuda_error(cudaGetLastError(), "err", __FILE__, __LINE__); return MEL_ERR_CUDA; }
     if (w[MEL_E_BOUNDS]) { mel_set_error("device index check failed (code %u)", w[MEL_E_BOUNDS]); return MEL_ERR_BOUNDS; }
     if (w[MEL_E_WAIT]) { mel_set_error("a wait of the body kernel's pipeline gave up after %llu ns", h->d.wait_ns); return MEL_ERR_TIMEOUT; }
     if (w[MEL_E_DEACT]) {
@@ -1018,7 +1020,13 @@ static mel_status adaptive_store(mel_handle* h, bool restore)
     double2* nb_ = static_cast<double2*>(h->store_bufs[0]);
     double* bb = static_cast<double*>(h->store_bufs[1]);
     cudaStream_t s = h->stream;
-    const cudaMemcpyKind k = cudaMemcpyDeviceToDevice;
+    mel_copy_list L;
+    L.n = 0;
+    auto add = [&](void* stored, void* live, size_t bytes) {
+        L.dst[L.n] = restore ? live : stored;
+        L.src[L.n] = restore ? stored : live;
+        L.words[L.n++] = bytes / 8;
+    };
     if (!restore) {
         if ((size_t)D.ncont > h->store_cont_cap) {
             if (h->store_bufs[2]) cudaFree(h->store_bufs[2]);
@@ -1031,20 +1039,16 @@ static mel_status adaptive_store(mel_handle* h, bool restore)
             }
             h->store_cont_cap = cap;
         }
-        for (int a = 0; a < 11; a++) MEL_CUDA_OK(cudaMemcpyAsync(nb_ + a * nn, nodes[a], sizeof(double2) * nn, k, s));
-        MEL_CUDA_OK(cudaMemcpyAsync(bb, D.works, sizeof(double) * 7 * nb, k, s));
-        MEL_CUDA_OK(cudaMemcpyAsync(bb + 7 * nb, D.bdfms, sizeof(double) * nb, k, s));
-        MEL_CUDA_OK(cudaMemcpyAsync(bb + 8 * nb, D.rg, sizeof(double) * MEL_RIGID_NF * nb, k, s));
-        if (D.ncont) MEL_CUDA_OK(cudaMemcpyAsync(h->store_bufs[2], D.cont, sizeof(mel_contact) * D.ncont, k, s));
         h->store_ncont = D.ncont;
-    } else {
-        for (int a = 0; a < 11; a++) MEL_CUDA_OK(cudaMemcpyAsync(nodes[a], nb_ + a * nn, sizeof(double2) * nn, k, s));
-        MEL_CUDA_OK(cudaMemcpyAsync(D.works, bb, sizeof(double) * 7 * nb, k, s));
-        MEL_CUDA_OK(cudaMemcpyAsync(D.bdfms, bb + 7 * nb, sizeof(double) * nb, k, s));
-        mel_launch_rigid_restore(D, bb + 8 * nb, s);
-        MEL_CUDA_OK(cudaGetLastError());
-        if (h->store_ncont) MEL_CUDA_OK(cudaMemcpyAsync(D.cont, h->store_bufs[2], sizeof(mel_contact) * h->store_ncont, k, s));
     }
+    for (int a = 0; a < 11; a++) add(nb_ + a * nn, nodes[a], sizeof(double2) * nn);
+    add(bb, D.works, sizeof(double) * 7 * nb);
+    add(bb + 7 * nb, D.bdfms, sizeof(double) * nb);
+    if (!restore) add(bb + 8 * nb, D.rg, sizeof(double) * MEL_RIGID_NF * nb);
+    if (h->store_ncont) add(h->store_bufs[2], D.cont, sizeof(mel_contact) * h->store_ncont);
+    mel_launch_copy_many(L, s);
+    if (restore) mel_launch_rigid_restore(D, bb + 8 * nb, s);
+    MEL_CUDA_OK(cudaGetLastError());
     return MEL_OK;
 }
 
@@ -1063,8 +1067,8 @@ static void dt_law(mel_handle* h, double c1, double c2)
 static mel_status adaptive_step(mel_handle* h)
 {
     if (!h->h_red) {
-        if (cudaMallocHost(&h->h_red, 8 * sizeof(double)) != cudaSuccess) { h->h_red = nullptr; mel_set_error("pinned allocation failed"); return MEL_ERR_OOM; }
-        h->d_red = dalloc<double>(h, 8);
+        if (cudaMallocHost(&h->h_red, (8 + MEL_E_NWORDS) * sizeof(double)) != cudaSuccess) { h->h_red = nullptr; mel_set_error("pinned allocation failed"); return MEL_ERR_OOM; }
+        h->d_red = dalloc<double>(h, 8 + MEL_E_NWORDS);
         if (!h->d_red) { mel_set_error("device allocation failed"); return MEL_ERR_OOM; }
     }
     mel_status rc = adaptive_store(h, false);
@@ -1075,8 +1079,8 @@ static mel_status adaptive_step(mel_handle* h)
     double mean_error = 0., max_error = 0., total_mass = 0., max_mass = 0.;
     while (!ok) {
         neval++;
-        h->h_red[7] = h->dt;
-        MEL_CUDA_OK(cudaMemcpyAsync(h->d.dt, &h->h_red[7], sizeof(double), cudaMemcpyHostToDevice, h->stream));
+        h->h_red[0] = h->dt;
+        MEL_CUDA_OK(cudaMemcpyAsync(h->d.dt, &h->h_red[0], sizeof(double), cudaMemcpyHostToDevice, h->stream));
         mel_dev d = h->d;
         mel_launch_contact(d, 0.5, h->stream);                 // Update_contact_forces(Deltat*0.5)
         mel_launch_damping(d, h->stream);
@@ -1092,10 +1096,11 @@ static mel_status adaptive_step(mel_handle* h)
         mel_launch_error_reduce(d, h->d_red, h->stream);
         h->launches += 5 + (h->d.fdamp ? 2 : 0) + (h->d.falid ? 2 : 0) + (h->nwide && h->nblocks_body ? 2 : 0);
         MEL_CUDA_OK(cudaGetLastError());
-        MEL_CUDA_OK(cudaMemcpyAsync(h->h_red, h->d_red, 4 * sizeof(double), cudaMemcpyDeviceToHost, h->stream));
+        double* const red = h->h_red + 1;
+        MEL_CUDA_OK(cudaMemcpyAsync(red, h->d_red, 4 * sizeof(double) + MEL_E_NWORDS * sizeof(unsigned), cudaMemcpyDeviceToHost, h->stream));
         MEL_CUDA_OK(cudaStreamSynchronize(h->stream));
-        if ((rc = check_errors(h))) return rc;
-        mean_error = h->h_red[0]; max_error = h->h_red[1]; total_mass = h->h_red[2]; max_mass = h->h_red[3];
+        if ((rc = check_errors(h, reinterpret_cast<const unsigned*>(red + 4)))) return rc;
+        mean_error = red[0]; max_error = red[1]; total_mass = red[2]; max_mass = red[3];
         const double error = max_error;
         bool reject = false;
         switch (h->solver) {
@@ -1130,8 +1135,8 @@ static mel_status adaptive_step(mel_handle* h)
     }
     if (ok) {
         // Time += Deltat happened with the Deltat of the accepted attempt: recover it from the
-        // snapshot of the attempt (h_red[7]) before the law changed h->dt
-        h->time += h->h_red[7];
+        // copy of the attempt (h_red[0]) before the law changed h->dt
+        h->time += h->h_red[0];
         h->pressure_state = 1;
     }
     h->solver_stats[0] = neval; h->solver_stats[1] = max_error; h->solver_stats[2] = mean_error;
