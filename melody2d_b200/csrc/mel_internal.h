@@ -168,6 +168,7 @@ struct mel_dev {
     const int *bd_body, *bd_per, *bd_bef, *bd_aft, *bd_e0, *bd_bc, *bd_h0;
     const double *bd_bcp, *ht, *hv;
     const int *e_node, *e_sn, *e_ss;         // e_sn/e_ss: 4 per entry (node0..3, shift0..3)
+    const int* e_border;                      // border of each entry
     const double* e_len0;
     double* e_len;                            // lengths of the last Update_borders
     double2* e_bcp;                           // border-condition pressures of the last Update_bc_forces

@@ -43,10 +43,11 @@ __device__ __forceinline__ double border_length(const mel_dev& d, int b, int g, 
     int n0 = d.b_node0[b];
     const int* sn = d.e_sn + 4 * e;
     const int* ss = d.e_ss + 4 * e;
-    double2 p0 = d.x[n0 + sn[0]], p1 = d.x[n0 + sn[1]], p2 = d.x[n0 + sn[2]];
-    double x0 = p0.x + d.period * ss[0], y0 = p0.y;
-    double x1 = p1.x + d.period * ss[1], y1 = p1.y;
-    double x2 = p2.x + d.period * ss[2], y2 = p2.y;
+    const int4 a = *reinterpret_cast<const int4*>(sn), h = *reinterpret_cast<const int4*>(ss);
+    double2 p0 = d.x[n0 + a.x], p1 = d.x[n0 + a.y], p2 = d.x[n0 + a.z];
+    double x0 = p0.x + d.period * h.x, y0 = p0.y;
+    double x1 = p1.x + d.period * h.y, y1 = p1.y;
+    double x2 = p2.x + d.period * h.z, y2 = p2.y;
     bool simple = d.bd_per[g] == MEL_PER_SIMPLE;
     if (j == 0 && simple) return sqrt((x2 - x1) * (x2 - x1) + (y2 - y1) * (y2 - y1)) * 0.5;
     if (j == nbn - 1 && simple) return sqrt((x1 - x0) * (x1 - x0) + (y1 - y0) * (y1 - y0)) * 0.5;
@@ -72,9 +73,10 @@ __device__ __forceinline__ void seg_points(const mel_dev& d, int bodyM, int e, i
                                            double* X, double* Y)
 {
     int mb = d.b_node0[bodyM];
+    const int4 a = reinterpret_cast<const int4*>(d.e_sn)[e], h = reinterpret_cast<const int4*>(d.e_ss)[e];
+    nd[0] = a.x; nd[1] = a.y; nd[2] = a.z; nd[3] = a.w;
+    sh[0] = h.x; sh[1] = h.y; sh[2] = h.z; sh[3] = h.w;
     for (int k = 0; k < 4; k++) {
-        nd[k] = d.e_sn[4 * e + k];
-        sh[k] = d.e_ss[4 * e + k];
         double2 p = d.x[mb + nd[k]];
         X[k] = p.x + d.period * (shiftM + sh[k]);
         Y[k] = p.y;
@@ -119,9 +121,7 @@ __device__ void contact_thread(const mel_dev& d, int tid, double law_dt_scale, i
         // refresh stored border lengths (read by Update_proximity for new contacts)
         int e = tid - d.ncont;
         if (e >= d.ne) return;
-        // find the border of entry e: binary search on bd_e0
-        int lo = 0, hi = d.nbd;
-        while (hi - lo > 1) { int mid = (lo + hi) >> 1; if (d.bd_e0[mid] <= e) lo = mid; else hi = mid; }
+        const int lo = d.e_border[e];
         int b = d.bd_body[lo];
         if (d.b_status[b] == MEL_STATUS_INACTIVE) return;
         if (d.b_type[b] == MEL_BODY_DEFORMABLE) d.e_len[e] = border_length(d, b, lo, e - d.bd_e0[lo]);
@@ -134,6 +134,12 @@ __device__ void contact_thread(const mel_dev& d, int tid, double law_dt_scale, i
         if (!czm_init) rigid_terms(d, tid, c, d.x[d.b_node0[b] + c.nodeS]);
         return;
     }
+    // the slave border's length and the law, which do not depend on the projection: their loads go
+    // out with those of the projection instead of after it
+    const int gS = d.b_bd0[b] + c.borderS;
+    const double length = entry_length(d, b, gS, c.border_nodeS);
+    const double initial_length = d.e_len0[d.bd_e0[gS] + c.border_nodeS];
+    const int li = d.table[d.b_mat[b] * d.nmat + d.b_mat[c.bodyM]];
     // ---- Update_contacts (Code/Body.h:1352-1632) -----------------------------------------
     int bodyM = c.bodyM, borderM = c.borderM, shiftM = c.shiftM, segmentM = c.segmentM;
     int gM = d.b_bd0[bodyM] + borderM;
@@ -212,10 +218,9 @@ __device__ void contact_thread(const mel_dev& d, int tid, double law_dt_scale, i
     c.vgapn = vgapn; c.vgapt = vgapt;
     if (czm_init) {
         c.gapn = p.gap; c.gapt = gapt;
-        const int lb = d.table[d.b_mat[b] * d.nmat + d.b_mat[bodyM]];
-        if (lb > -1) {
-            const int t = d.law_type[lb];
-            const double* P = d.law_p + MEL_LAW_NPARAM * lb;
+        if (li > -1) {
+            const int t = d.law_type[li];
+            const double* P = d.law_p + MEL_LAW_NPARAM * li;
             if (t == MEL_LAW_CZM_LINEAR) { c.nb_internal = 1; c.internal[0] = (c.gapn < P[5]) ? 0. : 1.; }
             else if (t == MEL_LAW_CZM_FATIGUE || t == MEL_LAW_BONDED_MOHR_COULOMB) {
                 const double gi = (t == MEL_LAW_CZM_FATIGUE) ? P[8] : P[10];
@@ -226,11 +231,7 @@ __device__ void contact_thread(const mel_dev& d, int tid, double law_dt_scale, i
         return;
     }
     // ---- Update_contact_forces (Code/Body.h:1657-1849) ----------------------------------
-    int gS = d.b_bd0[b] + c.borderS;
-    double length = entry_length(d, b, gS, c.border_nodeS);
-    double initial_length = d.e_len0[d.bd_e0[gS] + c.border_nodeS];
     double gapn = p.gap;
-    int li = d.table[d.b_mat[b] * d.nmat + d.b_mat[bodyM]];
     if (li > -1) {
         double W = 0., Pn = 0., Pt = 0.;
         int nbi = c.nb_internal;
@@ -473,17 +474,34 @@ __device__ bool mbar_wait_bounded(uint64_t* bar, unsigned parity, unsigned long 
     }
 }
 
-// running sums of `n` terms t[k*stride] (k = 0..n-1) added in order to acc; loads batched so
-// that eight are in flight per round trip
+// running sums of `n` terms t[k*stride] (k = 0..n-1) added in order to acc, eight loads in flight
+// while eight are added
 __device__ __forceinline__ double ordered_sum(double acc, const double* t, int n, int stride)
 {
+    double v[8], w[8];
     int k = 0;
-    for (; k + 8 <= n; k += 8) {
-        double v[8];
+    if (n >= 8) {
 #pragma unroll
-        for (int j = 0; j < 8; j++) v[j] = t[(size_t)(k + j) * stride];
+        for (int j = 0; j < 8; j++) v[j] = t[(size_t)j * stride];
+        for (; k + 24 <= n; k += 16) {
+#pragma unroll
+            for (int j = 0; j < 8; j++) w[j] = t[(size_t)(k + 8 + j) * stride];
+#pragma unroll
+            for (int j = 0; j < 8; j++) acc += v[j];
+#pragma unroll
+            for (int j = 0; j < 8; j++) v[j] = t[(size_t)(k + 16 + j) * stride];
+#pragma unroll
+            for (int j = 0; j < 8; j++) acc += w[j];
+        }
 #pragma unroll
         for (int j = 0; j < 8; j++) acc += v[j];
+        k += 8;
+    }
+    for (; k + 4 <= n; k += 4) {
+#pragma unroll
+        for (int j = 0; j < 4; j++) w[j] = t[(size_t)(k + j) * stride];
+#pragma unroll
+        for (int j = 0; j < 4; j++) acc += w[j];
     }
     for (; k < n; k++) acc += t[(size_t)k * stride];
     return acc;
@@ -916,6 +934,12 @@ __device__ __forceinline__ void tile_forces(const mel_dev& d, int b, const typen
     const int mtype = d.mat_type[mat];
     const double Mu = d.mat_p[MEL_MAT_NPARAM * mat + 3];
     const double Lam = d.mat_p[MEL_MAT_NPARAM * mat + 4];
+    // point groups come sorted, the one with the most rows first: warp 3, which shares its scheduler
+    // with the contact warp alone, takes that one, and the warps that share one take a long and a
+    // short group (0: 1, 1: 2, 2: 3, 4: 6, 5: 5, 6: 4).  Against group w for warp w, B200: 50 grains
+    // FP64 69.7 -> 66.0 us a launch, 60 grains mixed 47.9 -> 46.9 us, 700 grains equal
+    const int group = (0x4560321 >> (4 * warp)) & 7;
+    const int pt = 32 * group + lane;
     const int t1 = d.b_tile0[b + 1];
     int t = d.b_tile0[b];
     if (t >= t1) return;
@@ -943,15 +967,15 @@ __device__ __forceinline__ void tile_forces(const mel_dev& d, int b, const typen
     struct lane_t { const load_t* dn; double c0; int ns, K, w; unsigned s0, i0, t0; };
     auto point = [&](const uint4& H) {
         const int last = (int)(H.z & 0xffffu) - 1;
-        return ld_quad(reinterpret_cast<const mel_point*>(d.timg + mel_tile_base(H.x) + mel_tile_o_rec(H.y)) + min(tid, last));
+        return ld_quad(reinterpret_cast<const mel_point*>(d.timg + mel_tile_base(H.x) + mel_tile_o_rec(H.y)) + min(pt, last));
     };
     auto take = [&](const uint4& r, const uint4& H) {
         lane_t L;
         const int np = (int)(H.z & 0xffffu);
         L.c0 = __hiloint2double((int)r.y, (int)r.x);
         L.w = 8 * (int)((r.w >> 14) & 3u) + 8;
-        L.ns = tid < np ? (int)((r.z >> 16) & 0xffu) : 0;
-        L.K = (warp << 5) < np ? (int)(r.z >> 24) : 0;
+        L.ns = pt < np ? (int)((r.z >> 16) & 0xffu) : 0;
+        L.K = 32 * group < np ? (int)(r.z >> 24) : 0;
         L.s0 = r.z & 0xffffu;
         L.i0 = r.w & 0x3fffu;
         L.t0 = r.w >> 16;
@@ -1192,6 +1216,7 @@ __device__ void deformable_body(const mel_dev& d, int b, double T, double T0, ch
     const int lane = tid & 31, warp = tid >> 5;
     const int n0 = d.b_node0[b];
     const int n = d.b_node0[b + 1] - n0;
+    if (n == 0) return;
     const double dt = d.dt[0];
     constexpr bool wide = WIDE;
     const long long go = WIDE ? d.b_gscr[b] : 0LL;
@@ -1243,6 +1268,13 @@ __device__ void deformable_body(const mel_dev& d, int b, double T, double T0, ch
             }
             __syncthreads();
         }
+        if (tid == MEL_BODY_THREADS - 32) {
+            // what the tail reads from global memory, on its way to L2
+            l2_prefetch(d.mass + n0, 16u * n); l2_prefetch(d.minv + n0, 16u * n);
+            l2_prefetch(d.vp + n0, 16u * n); l2_prefetch(d.X0 + n0, 16u * n);
+            const int k0 = d.kg_base[d.b_ks0[b] >> 5], k1 = d.kg_base[d.b_ks0[b + 1] >> 5];
+            if (k1 > k0) { l2_prefetch(d.ks_idx + k0, 2u * (k1 - k0)); l2_prefetch(d.ks_N + k0, 8u * (k1 - k0)); }
+        }
         if (warp < MEL_BODY_CTHREADS / 32) {
             if constexpr (MX) tile_forces<true>(d, b, s_upf, s_f, region, s_bar, s_abort, tid, lane, warp);
             else tile_forces<false>(d, b, s_up, s_f, region, s_bar, s_abort, tid, lane, warp);
@@ -1250,9 +1282,16 @@ __device__ void deformable_body(const mel_dev& d, int b, double T, double T0, ch
             grid_wait();
             contact_scatter(d, b, n0, s_fc, lane);
         }
-        __syncthreads();
-        if (*s_abort) return;
     }
+    // the first node's masses and velocity parameters and the first kinematics slot, asked for before
+    // the barrier
+    const int i0 = min(tid, n - 1), ki0 = tid >= 32 ? min(tid - 32, n - 1) : 0;
+    const int ks = d.b_ks0[b];
+    double2 m0 = d.mass[n0 + i0], im0 = d.minv[n0 + i0], vp0 = d.vp[n0 + i0];
+    unsigned krec = d.ks_rec[ks + ki0];
+    int kbase = d.kg_base[(ks + ki0) >> 5];
+    __syncthreads();
+    if (!wide && *reinterpret_cast<volatile int*>(reinterpret_cast<uint64_t*>(s_after) + 3)) return;
     double2* s_fn = reinterpret_cast<double2*>(wide ? d.gscr + go + mel_wide_pre_bytes(n) : region);
     double2* s_fd = s_fn + n;
     double2* s_vp = s_fd + n;
@@ -1323,7 +1362,8 @@ __device__ void deformable_body(const mel_dev& d, int b, double T, double T0, ch
     double2* s_upt = reinterpret_cast<double2*>(s_T + 6 * n);     // AD phase 1: temporary parameters
     for (int i = tid; i < n; i += blockDim.x) {
         int gi = n0 + i;
-        double2 m = d.mass[gi], im = d.minv[gi];
+        const double2 m = m0, im = im0, vp = vp0;
+        if (i + (int)blockDim.x < n) { m0 = d.mass[gi + blockDim.x]; im0 = d.minv[gi + blockDim.x]; vp0 = d.vp[gi + blockDim.x]; }
         double2 fb = make_double2(m.x * gx, m.y * gy);
         double2 fi = s_f[i], fc = s_fc[i];
         double2 fn = has_bc ? s_fn[i] : make_double2(0., 0.);
@@ -1336,7 +1376,6 @@ __device__ void deformable_body(const mel_dev& d, int b, double T, double T0, ch
         double2 ap;
         if (AD) { const double2 f = d.fms[gi]; ap = make_double2(ft.x * im.x / f.x, ft.y * im.y / f.y); }
         else ap = make_double2(ft.x * im.x / 1., ft.y * im.y / 1.);
-        double2 vp = d.vp[gi];
         s_ap[i] = ap;
         s_vp[i] = vp;
         if (d.record_forces) {
@@ -1356,67 +1395,79 @@ __device__ void deformable_body(const mel_dev& d, int b, double T, double T0, ch
         s_T[4 * n + i] = dte * (vx * fdp.x + vy * fdp.y);
         s_T[5 * n + i] = dte * (vx * fal.x + vy * fal.y);
     }
+    int* s_ticket = reinterpret_cast<int*>(s_after + 64);
+    if (tid == 0) *s_ticket = MEL_BODY_THREADS / 32 - 1;
     __syncthreads();
-    if (warp == 0) {
-        // works (internal, body, dirichlet, neumann, damping, alid), summed in node order; these
-        // serial sums are the body's last work for warp 0, and they overlap the kinematics below
-        if (lane < 6) {
-            const int w = lane == 0 ? 0 : lane + 1;       // works slots 0, 2, 3, 4, 5, 6
-            d.works[7 * b + w] = ordered_sum(d.works[7 * b + w], s_T + (size_t)lane * n, n, 1);
-        }
-        return;
-    } else {
-        // ---- Apply_Euler (Code/Node.h:239-245) ---------------------------------------------
-        for (int i = tid - 32; i < n; i += blockDim.x - 32) {
-            int gi = n0 + i;
-            double2 ap = s_ap[i], vp = s_vp[i], up = s_up[i];
-            vp.x = vp.x + dte * ap.x; vp.y = vp.y + dte * ap.y;
-            up.x = up.x + dte * vp.x; up.y = up.y + dte * vp.y;
-            s_vp[i] = vp; s_up[i] = up;
-            d.ap[gi] = ap; d.vp[gi] = vp; d.up[gi] = up;
-        }
+    // ---- Apply_Euler (Code/Node.h:239-245) -----------------------------------------------------
+    for (int i = tid; i < n; i += blockDim.x) {
+        int gi = n0 + i;
+        double2 ap = s_ap[i], vp = s_vp[i], up = s_up[i];
+        vp.x = vp.x + dte * ap.x; vp.y = vp.y + dte * ap.y;
+        up.x = up.x + dte * vp.x; up.y = up.y + dte * vp.y;
+        s_vp[i] = vp; s_up[i] = up;
+        d.ap[gi] = ap; d.vp[gi] = vp; d.up[gi] = up;
     }
-    tail_sync();      // warps 1-7: Euler done
+    __syncthreads();
+    // works (internal, body, dirichlet, neumann, damping, alid), summed in node order: serial sums of
+    // warp 0 beside the kinematics
+    if (warp == 0 && lane < 6) {
+        const int w = lane == 0 ? 0 : lane + 1;       // works slots 0, 2, 3, 4, 5, 6
+        d.works[7 * b + w] = ordered_sum(d.works[7 * b + w], s_T + (size_t)lane * n, n, 1);
+    }
+    __syncwarp();
     // ---- Update_kinematics + Update_current_positions (Code/Body.h:2176-2227, 2272-2283) --
-    // slot i of the body's kinematics layout is lane i & 31 of group i >> 5 (i = tid - 32 + 224 m
-    // keeps the lane); row k of a group is 32 consecutive entries, so the support loads of a warp
-    // are coalesced.  Each node sums its supports in their own order.
-    const int ks = d.b_ks0[b];
-    for (int i = tid - 32; i < n; i += blockDim.x - 32) {
-        const unsigned rec = d.ks_rec[ks + i];
-        const int node = (int)(rec & 0xffffu), cnt = (int)(rec >> 16);
-        const int* kb = d.kg_base + ((ks + i) >> 5);
-        const uint16_t* kidx = d.ks_idx + *kb + lane;
-        const double* kN = d.ks_N + *kb + lane;
+    // slot i of the body's kinematics layout is lane i & 31 of group i >> 5; row k of a group is 32
+    // consecutive entries, so the support loads of a warp are coalesced.  Each node sums its supports
+    // in their own order.  Groups are sorted by support count; warps 1-7 begin with the first seven,
+    // then every warp takes the next one, warp 0 after its sums.  The loads come from L2, some 600
+    // cycles away: the next group's records and eight rows are always in flight.
+    auto ticket = [&]() {
+        int t = 0;
+        if (lane == 0) t = atomicAdd(s_ticket, 1);
+        return __shfl_sync(0xffffffffu, t, 0);
+    };
+    int next = warp - 1;
+    if (warp == 0) {
+        next = ticket();
+        if (32 * next < n) { krec = d.ks_rec[ks + min(32 * next + lane, n - 1)]; kbase = d.kg_base[(ks >> 5) + next]; }
+    }
+    while (32 * next < n) {
+        const int i = 32 * next + lane;
+        const int node = (int)(krec & 0xffffu), cnt = i < n ? (int)(krec >> 16) : 0;
+        const uint16_t* kidx = d.ks_idx + kbase + lane;
+        const double* kN = d.ks_N + kbase + lane;
+        next = ticket();
+        if (32 * next < n) { krec = d.ks_rec[ks + min(32 * next + lane, n - 1)]; kbase = d.kg_base[(ks >> 5) + next]; }
+        const double2 X = d.X0[n0 + node];
         double dx = 0., dy = 0., vx = 0., vy = 0., ax = 0., ay = 0.;
-        int k = 0;
-        for (; k + 4 <= cnt; k += 4) {
-            int t[4];
-            double sN[4];
+        struct rows8 { int t[8]; double N[8]; } ra, rb;
+        auto get = [&](rows8& r, int k) {
 #pragma unroll
-            for (int q = 0; q < 4; q++) { t[q] = kidx[32 * (k + q)]; sN[q] = kN[32 * (k + q)]; }
+            for (int q = 0; q < 8; q++) if (k + q < cnt) { r.t[q] = kidx[32 * (k + q)]; r.N[q] = kN[32 * (k + q)]; }
+        };
+        auto add = [&](const rows8& r, int k) {
 #pragma unroll
-            for (int q = 0; q < 4; q++) {
-                double2 up = s_up[t[q]], vp = s_vp[t[q]], ap = s_ap[t[q]];
-                double sv = sN[q];
-                dx += sv * up.x; dy += sv * up.y;
-                vx += sv * vp.x; vy += sv * vp.y;
-                ax += sv * ap.x; ay += sv * ap.y;
-            }
+            for (int q = 0; q < 8; q++)
+                if (k + q < cnt) {
+                    const double2 up = s_up[r.t[q]], vp = s_vp[r.t[q]], ap = s_ap[r.t[q]];
+                    const double sv = r.N[q];
+                    dx += sv * up.x; dy += sv * up.y;
+                    vx += sv * vp.x; vy += sv * vp.y;
+                    ax += sv * ap.x; ay += sv * ap.y;
+                }
+        };
+        get(ra, 0);
+        for (int k = 0; k < cnt; k += 16) {
+            get(rb, k + 8);
+            add(ra, k);
+            get(ra, k + 16);
+            add(rb, k + 8);
         }
-        for (; k < cnt; k++) {
-            const int t = kidx[32 * k];
-            const double sv = kN[32 * k];
-            double2 up = s_up[t], vp = s_vp[t], ap = s_ap[t];
-            dx += sv * up.x; dy += sv * up.y;
-            vx += sv * vp.x; vy += sv * vp.y;
-            ax += sv * ap.x; ay += sv * ap.y;
-        }
+        if (i >= n) continue;
         const int gi = n0 + node;
         d.u[gi] = make_double2(dx, dy);
         d.v[gi] = make_double2(vx, vy);
         d.a[gi] = make_double2(ax, ay);
-        double2 X = d.X0[gi];
         d.x[gi] = make_double2(X.x + dx, X.y + dy);
         if (AD && d.phase == 1) {      // Update_kinematics_temporary (Code/Body.h:2235-2253)
             double tx = 0., ty = 0.;
@@ -1432,6 +1483,8 @@ __device__ void deformable_body(const mel_dev& d, int b, double T, double T0, ch
         // ---- Update_bc(Time+Deltat) of the body's driven borders, Compute_error and
         // Compute_mass_scaling (Code/Body.h:2528-2594, Code/Node.h:253-320): nodal terms in
         // parallel, the body's sums and maximum in node order --------------------------------------
+        __syncthreads();
+        if (warp == 0) return;
         double* drv = d.drv + 8 * b;
         if (tid == 32) body_drivendof(d, b, T0 + dt, drv);
         tail_sync();

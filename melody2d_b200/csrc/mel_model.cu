@@ -619,7 +619,8 @@ static mel_status build(mel_handle* h, const mel_model_desc* d, const mel_option
             if (kidx.size() > (size_t)INT32_MAX) { mel_set_error("node supports above 2^31 entries"); return MEL_ERR_UNSUPPORTED; }
         }
         ks0[nb] = (int)rec.size();
-        if (rec.empty()) { rec.push_back(0u); kgb.push_back(0); kidx.push_back(0); kN.push_back(0.); }
+        kgb.push_back((int)kidx.size());               // the end of the last group
+        if (rec.empty()) { rec.push_back(0u); kidx.push_back(0); kN.push_back(0.); }
         D.b_ks0 = dupload(h, ks0);
         D.ks_rec = dupload(h, rec);
         D.kg_base = dupload(h, kgb);
@@ -649,6 +650,9 @@ static mel_status build(mel_handle* h, const mel_model_desc* d, const mel_option
     for (int b = 0; b < nb; b++) initialize_segments(d, b, sn, ss, len0);
     D.e_sn = dupload(h, sn);
     D.e_ss = dupload(h, ss);
+    std::vector<int> eb(ne, 0);
+    for (int g = 0; g < nbd; g++) for (int e = d->border_node_ptr[g]; e < d->border_node_ptr[g + 1]; e++) eb[e] = g;
+    D.e_border = dupload(h, eb);
     D.e_len0 = dupload(h, len0);
     std::vector<double> len(len0);
     D.e_len = dupload(h, len);
