@@ -19,6 +19,7 @@
 #include "mel_internal.h"
 #include "mel_geometry.cuh"
 #include "mel_sincos.h"
+#include "mel_sums.cuh"
 
 namespace mel {
 
@@ -472,39 +473,6 @@ __device__ bool mbar_wait_bounded(uint64_t* bar, unsigned parity, unsigned long 
             if (mbar_try_wait(bar, parity)) return true;
         if (global_ns() - t0 > limit_ns) return false;
     }
-}
-
-// running sums of `n` terms t[k*stride] (k = 0..n-1) added in order to acc, eight loads in flight
-// while eight are added
-__device__ __forceinline__ double ordered_sum(double acc, const double* t, int n, int stride)
-{
-    double v[8], w[8];
-    int k = 0;
-    if (n >= 8) {
-#pragma unroll
-        for (int j = 0; j < 8; j++) v[j] = t[(size_t)j * stride];
-        for (; k + 24 <= n; k += 16) {
-#pragma unroll
-            for (int j = 0; j < 8; j++) w[j] = t[(size_t)(k + 8 + j) * stride];
-#pragma unroll
-            for (int j = 0; j < 8; j++) acc += v[j];
-#pragma unroll
-            for (int j = 0; j < 8; j++) v[j] = t[(size_t)(k + 16 + j) * stride];
-#pragma unroll
-            for (int j = 0; j < 8; j++) acc += w[j];
-        }
-#pragma unroll
-        for (int j = 0; j < 8; j++) acc += v[j];
-        k += 8;
-    }
-    for (; k + 4 <= n; k += 4) {
-#pragma unroll
-        for (int j = 0; j < 4; j++) w[j] = t[(size_t)(k + j) * stride];
-#pragma unroll
-        for (int j = 0; j < 4; j++) acc += w[j];
-    }
-    for (; k < n; k++) acc += t[(size_t)k * stride];
-    return acc;
 }
 
 // Gauss-point pass of one chunk held in shared memory (Body::Update_internal_forces,
@@ -1975,20 +1943,23 @@ __global__ void monitor_partial_kernel(const __grid_constant__ mel_dev d, double
     if (threadIdx.x < 5) part[threadIdx.x * MON_BLOCKS + blockIdx.x] = s[threadIdx.x][0];
 }
 
-__global__ void monitor_final_kernel(const __grid_constant__ mel_dev d, const double* part, const int* rigid_ids, int nrigid, double* out)
+// a lane per sum (added block by block, in order) and per rigid body
+__global__ void __launch_bounds__(32) monitor_final_kernel(const __grid_constant__ mel_dev d, const double* part, const int* rigid_ids, int nrigid, double* out)
 {
-    if (threadIdx.x == 0) {
-        double t[5] = { 0., 0., 0., 0., 0. };
-        for (int k = 0; k < 5; k++)
-            for (int b = 0; b < MON_BLOCKS; b++) t[k] += part[k * MON_BLOCKS + b];
-        out[0] = t[0];
-        out[1] = t[3] > 0 ? t[1] / t[3] : 0.;
-        out[2] = t[3] > 0 ? t[2] / t[3] : 0.;
-        out[3] = t[4];
-        for (int r = 0; r < nrigid && r < 4; r++) {
-            const double* rf = d.rf + 15 * rigid_ids[r];
-            out[4 + 4 * r] = rf[0]; out[5 + 4 * r] = rf[1]; out[6 + 4 * r] = rf[6]; out[7 + 4 * r] = rf[7];
-        }
+    const int lane = threadIdx.x;
+    const double t = lane < 5 ? ordered_sum(0., part + lane * MON_BLOCKS, MON_BLOCKS, 1) : 0.;
+    const double ux = __shfl_sync(0xffffffffu, t, 1), uy = __shfl_sync(0xffffffffu, t, 2);
+    const double mt = __shfl_sync(0xffffffffu, t, 3), act = __shfl_sync(0xffffffffu, t, 4);
+    if (lane == 0) {
+        out[0] = t;
+        out[1] = mt > 0 ? ux / mt : 0.;
+        out[2] = mt > 0 ? uy / mt : 0.;
+        out[3] = act;
+    }
+    const int r = lane - 8;
+    if (r >= 0 && r < min(nrigid, 4)) {
+        const double* rf = d.rf + 15 * rigid_ids[r];
+        out[4 + 4 * r] = rf[0]; out[5 + 4 * r] = rf[1]; out[6 + 4 * r] = rf[6]; out[7 + 4 * r] = rf[7];
     }
 }
 
@@ -2007,12 +1978,6 @@ __device__ __forceinline__ void pressure_push(const mel_dev& d, int e, int v)
     else set_err(d, MEL_E_PRESSURE);
 }
 
-__global__ void pressure_clear_kernel(const __grid_constant__ mel_dev d)
-{
-    const int e = blockIdx.x * blockDim.x + threadIdx.x;
-    if (e < d.ne) d.cp_cnt[e] = 0;
-}
-
 __global__ void pressure_push_kernel(const __grid_constant__ mel_dev d)
 {
     const int c = blockIdx.x * blockDim.x + threadIdx.x;
@@ -2026,29 +1991,35 @@ __global__ void pressure_push_kernel(const __grid_constant__ mel_dev d)
     pressure_push(d, eM + 1, (c << 2) | 2);
 }
 
-__global__ void pressure_sum_kernel(const __grid_constant__ mel_dev d)
+// contribution v = (contact << 2 | role) to a border entry's pressure
+__device__ __forceinline__ void pressure_add(const mel_dev& d, int v, double& px, double& py)
+{
+    const mel_contact& k = d.cont[v >> 2];
+    const int role = v & 3;
+    const double il = 1. / k.length;
+    if (role == 0) { px += k.fx * il; py += k.fy * il; }
+    else {
+        const double sh = k.shapeM[role];
+        px -= k.fx * il * sh;
+        py -= k.fy * il * sh;
+    }
+}
+
+// leaves the counts at zero for the next gather
+__global__ void __launch_bounds__(128) pressure_sum_kernel(const __grid_constant__ mel_dev d)
 {
     const int e = blockIdx.x * blockDim.x + threadIdx.x;
     if (e >= d.ne) return;
     const int n = min(d.cp_cnt[e], MEL_PRESSURE_CAP);
-    int v[MEL_PRESSURE_CAP];
-    for (int i = 0; i < n; i++) {                         // insertion sort: a handful of items
-        const int x = d.cp_item[(size_t)e * MEL_PRESSURE_CAP + i];
-        int j = i;
-        while (j > 0 && v[j - 1] > x) { v[j] = v[j - 1]; j--; }
-        v[j] = x;
-    }
     double px = 0., py = 0.;
-    for (int i = 0; i < n; i++) {
-        const mel_contact& k = d.cont[v[i] >> 2];
-        const int role = v[i] & 3;
-        const double il = 1. / k.length;
-        if (role == 0) { px += k.fx * il; py += k.fy * il; }
-        else {
-            const double sh = k.shapeM[role];
-            px -= k.fx * il * sh;
-            py -= k.fy * il * sh;
-        }
+    if (n > 0) d.cp_cnt[e] = 0;
+    const int* item = d.cp_item + (size_t)e * MEL_PRESSURE_CAP;
+    int last = -1;                                        // the items in ascending order, one at a time:
+    for (int i = 0; i < n; i++) {                         // a handful, each listed once
+        int v = 0x7fffffff;
+        for (int j = 0; j < n; j++) { const int x = item[j]; if (x > last && x < v) v = x; }
+        pressure_add(d, v, px, py);
+        last = v;
     }
     d.cpx[e] = px;
     d.cpy[e] = py;
@@ -2059,7 +2030,6 @@ __global__ void pressure_sum_kernel(const __grid_constant__ mel_dev d)
 void mel_launch_contact_pressures(const mel_dev& d, cudaStream_t s)
 {
     if (d.ne <= 0) return;
-    mel::pressure_clear_kernel<<<(d.ne + 255) / 256, 256, 0, s>>>(d);
     if (d.ncont > 0) mel::pressure_push_kernel<<<(d.ncont + 127) / 128, 128, 0, s>>>(d);
     mel::pressure_sum_kernel<<<(d.ne + 127) / 128, 128, 0, s>>>(d);
 }

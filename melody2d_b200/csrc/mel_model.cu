@@ -92,6 +92,7 @@ struct mel_handle {
     int store_ncont = 0;
     double t_bc = 0.;
     double solver_stats[5] = { 0., 0., 0., 0., 0. };
+    unsigned* h_err = nullptr;  // error words read with a call's last synchronisation (pinned)
     double* h_red = nullptr;
     double* d_red = nullptr;
     int* d_rigid_ids = nullptr;
@@ -783,6 +784,7 @@ static mel_status build(mel_handle* h, const mel_model_desc* d, const mel_option
     }
     // contacts and proximity buffers
     D.err = dalloc<unsigned>(h, MEL_E_NWORDS);
+    if (cudaMallocHost(&h->h_err, MEL_E_NWORDS * sizeof(unsigned)) != cudaSuccess) { h->h_err = nullptr; mel_set_error("pinned allocation failed"); return MEL_ERR_OOM; }
     D.ncont = 0;
     mel_prox_state& P = h->P;
     P.nbr_cap = MEL_NBR_CAP_DEFAULT;
@@ -1154,7 +1156,7 @@ static void update_pressures(mel_handle* h)
     if (h->pressure_state != 1) return;
     cudaMemsetAsync(h->d.err + MEL_E_PRESSURE, 0, sizeof(unsigned), h->stream);
     mel_launch_contact_pressures(h->d, h->stream);
-    h->launches += 3;
+    h->launches += 2;
     h->pressure_state = 0;
 }
 
@@ -1263,6 +1265,7 @@ mel_status mel_destroy(mel_handle* h)
     if (h->d_state) cudaFree(h->d_state);
     for (void* p : h->store_bufs) cudaFree(p);
     if (h->h_red) cudaFreeHost(h->h_red);
+    if (h->h_err) cudaFreeHost(h->h_err);
     for (void* p : { (void*)h->mon_ops, (void*)h->mon_part, (void*)h->mon_rows }) if (p) cudaFree(p);
     if (h->ck.h_stage) cudaFreeHost(h->ck.h_stage);
     for (auto e : h->ev_pool) cudaEventDestroy(e);
@@ -1329,7 +1332,7 @@ mel_status mel_step(mel_handle* h, mel_step_io* io)
             cudaError_t le = cudaGetLastError();
             if (le != cudaSuccess) { mel_set_cuda_error(le, "monitoring launch", __FILE__, __LINE__); return MEL_ERR_CUDA; }
             h->mon_count++;
-            h->launches += 2;
+            h->launches += 1;
         }
         if (io->run_proximity && h->time > h->next_cup - 1.e-6 * h->dt) {   // Code/main.cpp:191-196
             h->next_cup = h->next_cup + h->cup;
@@ -1352,6 +1355,7 @@ mel_status mel_step(mel_handle* h, mel_step_io* io)
         MEL_CUDA_OK(cudaMemcpyAsync(h->d.dt, &h->dt, sizeof(double), cudaMemcpyHostToDevice, h->stream));
     }
     cudaEventRecord(h->ev_end, h->stream);
+    MEL_CUDA_OK(cudaMemcpyAsync(h->h_err, h->d.err, MEL_E_NWORDS * sizeof(unsigned), cudaMemcpyDeviceToHost, h->stream));
     cudaError_t e = cudaStreamSynchronize(h->stream);
     if (e != cudaSuccess) { mel_set_cuda_error(e, "mel_step", __FILE__, __LINE__); return MEL_ERR_CUDA; }
     {
@@ -1372,7 +1376,7 @@ mel_status mel_step(mel_handle* h, mel_step_io* io)
             h->t_prox += ms;
         }
     }
-    mel_status rc = check_errors(h);
+    mel_status rc = check_errors(h, h->h_err);
     if (rc) return rc;
     io->time = h->time; io->dt = h->dt; io->next_contact_update = h->next_cup;
     io->n_contacts = h->d.ncont; io->n_proximity = nprox;
@@ -1791,6 +1795,7 @@ mel_status mel_monitor_setup(mel_handle* h, const double* monitored, int n_monit
         mel_set_error("monitoring buffers (%d rows of %d values) could not be allocated", ring_rows, row);
         return MEL_ERR_OOM;
     }
+    MEL_CUDA_OK(cudaMemsetAsync(h->mon_part, 0, sizeof(double) * 3 * ((size_t)h->nb + 1), h->stream));
     if (!ops.empty()) MEL_CUDA_OK(cudaMemcpy(h->mon_ops, ops.data(), sizeof(mel_mon_op) * ops.size(), cudaMemcpyHostToDevice));
     h->mon_nops = (int)ops.size();
     h->mon_energy = monitor_energy ? 1 : 0;
@@ -2355,7 +2360,7 @@ mel_status mel_batch_step(mel_batch* b, int nsteps, int run_proximity)
             if (run_proximity && h->time > h->next_cup - 1.e-6 * h->dt) {   // Code/main.cpp:191-196
                 h->next_cup = h->next_cup + h->cup;
                 due.push_back(h);
-                if (h->d.record_forces) { mel_launch_contact_pressures(h->d, b->stream); b->launches += 3; h->pressure_state = 0; }
+                if (h->d.record_forces) { mel_launch_contact_pressures(h->d, b->stream); b->launches += 2; h->pressure_state = 0; }
                 else h->pressure_state = 2;
             }
         }
@@ -2367,13 +2372,15 @@ mel_status mel_batch_step(mel_batch* b, int nsteps, int run_proximity)
         }
     }
     cudaEventRecord(b->e1, b->stream);
+    for (mel_handle* h : b->members)
+        MEL_CUDA_OK(cudaMemcpyAsync(h->h_err, h->d.err, MEL_E_NWORDS * sizeof(unsigned), cudaMemcpyDeviceToHost, b->stream));
     cudaError_t e = cudaStreamSynchronize(b->stream);
     if (e != cudaSuccess) { mel_set_cuda_error(e, "mel_batch_step", __FILE__, __LINE__); return MEL_ERR_CUDA; }
     float ms = 0.f;
     cudaEventElapsedTime(&ms, b->e0, b->e1);
     b->ms_last = ms;
     for (mel_handle* h : b->members) {
-        mel_status rc = check_errors(h);
+        mel_status rc = check_errors(h, h->h_err);
         if (rc == MEL_ERR_BOUNDS) { h->failed = rc; h->failed_msg = mel_last_error_string(); }
         else if (rc) return rc;
     }

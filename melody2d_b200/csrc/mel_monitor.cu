@@ -1,8 +1,8 @@
 // Monitoring (Code/Monitoring.h:8-559) on the device: after every accepted step the solver's stream
-// runs mon_body_kernel (one warp per body: the body's sums that the whole-sample quantities add up)
-// and mon_row_kernel (one thread: the monitored entries in list order, then the energy and boundary
-// blocks), which appends the row to a device buffer that the host drains at save time
-// (Write_monitoring, Code/IO.h:2644-2668).  No host download happens per step.
+// runs monitor_kernel: one warp per body for the body's sums that the whole-sample quantities add up,
+// then, in the block that ends last, one warp for the row: the monitored entries in list order, then
+// the energy and boundary blocks.  It appends the row to a device buffer that the host drains at save
+// time (Write_monitoring, Code/IO.h:2644-2668).  No host download happens per step.
 //
 // Exactness: every quantity of one node, one body or one border is computed in the reference's
 // operation order (a single thread walks the body's nodes in index order), so it equals the
@@ -11,6 +11,7 @@
 // which changes the association of the reference's single running sum: they agree with it to a
 // few units in the last place, far inside the 10 significant digits MONITORING.asc keeps.
 #include "mel_internal.h"
+#include "mel_sums.cuh"
 
 namespace mel {
 
@@ -18,7 +19,7 @@ namespace mel {
 // Monitoring.h:528-531), part[3b+1] = the body's Energy Kinetic term (Monitoring.h:398-412:
 // velocity parameters of a deformable body's nodes, or the rigid body's translation and rotation),
 // part[3b+2] = the body's Dwork terms (Monitoring.h:516-526) with Deltat = dt
-__global__ void __launch_bounds__(256) mon_body_kernel(mel_dev d, double dt, double* part)
+__device__ __forceinline__ void mon_body(const mel_dev& d, double dt, double* part)
 {
     const int b = (int)((blockIdx.x * blockDim.x + threadIdx.x) >> 5);
     const int lane = threadIdx.x & 31;
@@ -26,20 +27,36 @@ __global__ void __launch_bounds__(256) mon_body_kernel(mel_dev d, double dt, dou
     const int n0 = d.b_node0[b], n1 = d.b_node0[b + 1];
     const bool def = d.b_type[b] == MEL_BODY_DEFORMABLE;
     double ke = 0., kp = 0., dw = 0.;
-    for (int i = n0 + lane; i < n1; i += 32) {
-        const double2 v = d.v[i], m = d.mass[i];
-        ke += 0.5 * v.x * v.x * m.x;
-        ke += 0.5 * v.y * v.y * m.y;
-        if (def) {
-            const double2 w = d.vp[i];
-            kp += 0.5 * w.x * w.x * m.x;
-            kp += 0.5 * w.y * w.y * m.y;
+    // four nodes or entries of a lane in flight: a plate's border is hundreds of entries long
+    for (int i = n0 + lane; i < n1; i += 128) {
+        double2 v[4], m[4], w[4];
+#pragma unroll
+        for (int k = 0; k < 4; k++) {
+            const int q = min(i + 32 * k, n1 - 1);
+            v[k] = d.v[q]; m[k] = d.mass[q]; w[k] = d.vp[q];
+        }
+#pragma unroll
+        for (int k = 0; k < 4; k++) {
+            if (i + 32 * k >= n1) continue;
+            ke += 0.5 * v[k].x * v[k].x * m[k].x;
+            ke += 0.5 * v[k].y * v[k].y * m[k].y;
+            if (def) {
+                kp += 0.5 * w[k].x * w[k].x * m[k].x;
+                kp += 0.5 * w[k].y * w[k].y * m[k].y;
+            }
         }
     }
     const int e0 = d.bd_e0[d.b_bd0[b]], e1 = d.bd_e0[d.b_bd0[b + 1]];
-    for (int e = e0 + lane; e < e1; e += 32) {
-        const double2 p = d.e_bcp[e], v = d.v[n0 + d.e_node[e]];
-        dw += (p.x * v.x + p.y * v.y) * d.e_len[e] * dt;
+    for (int e = e0 + lane; e < e1; e += 256) {
+        double2 p[8], v[8];
+        double len[8];
+        int nd[8];
+#pragma unroll
+        for (int k = 0; k < 8; k++) { const int q = min(e + 32 * k, e1 - 1); nd[k] = d.e_node[q]; p[k] = d.e_bcp[q]; len[k] = d.e_len[q]; }
+#pragma unroll
+        for (int k = 0; k < 8; k++) v[k] = d.v[n0 + nd[k]];
+#pragma unroll
+        for (int k = 0; k < 8; k++) if (e + 32 * k < e1) dw += (p[k].x * v[k].x + p[k].y * v[k].y) * len[k] * dt;
     }
     for (int o = 16; o; o >>= 1) {
         ke += __shfl_xor_sync(0xffffffffu, ke, o);
@@ -113,126 +130,155 @@ __device__ double body_damage(const mel_dev& d, int b)
     return dmg;
 }
 
-// one row of Monitoring (Code/Monitoring.h:8-559) into row[1..], its length into row[0]
-__global__ void mon_row_kernel(mel_dev d, const mel_mon_op* ops, int nops, int energy, int boundaries,
-                               const double* part, double* row, mel_mon_head hd)
+// What one entry reads, found by a lane of its own: the values it assigns to the running x, y, r of
+// the entry list (has bits 1, 2, 4) and the value of entries that append one without them (has bit 8)
+struct mon_value { double x, y, r, v; int has; };
+__device__ __forceinline__ mon_value mon_entry(const mel_dev& d, const mel_mon_op& o, const double* part)
 {
-    if (threadIdx.x != 0) return;
-    int c = 1;
-    row[c++] = hd.iteration; row[c++] = hd.time; row[c++] = hd.dt;
-    row[c++] = hd.neval; row[c++] = hd.max_error; row[c++] = hd.mean_error;
-    // x, y, r and m live across entries as in the reference, where an entry that does not assign
-    // one of them reads the value the previous entry left (never-assigned values start at 0)
-    double x = 0., y = 0., r = 0., m = 0.;
-    for (int k = 0; k < nops; k++) {
-        const mel_mon_op o = ops[k];
-        if (o.type <= 3) {
-            // Position, Displacement, Velocity, Acceleration (Monitoring.h:33-192)
-            const double2* a = o.type == 0 ? d.x : o.type == 1 ? d.u : o.type == 2 ? d.v : d.a;
-            const int rx = o.type == 0 ? MEL_RG_XC : o.type == 1 ? MEL_RG_XD : o.type == 2 ? MEL_RG_XV : MEL_RG_XA;
-            const int n0 = d.b_node0[o.body];
-            if (o.node >= 0) {
-                const double2 p = a[n0 + o.node];
-                x = p.x; y = p.y;
-            } else if (d.b_type[o.body] == MEL_BODY_DEFORMABLE) {
-                x = 0.; y = 0.; m = 0.;
-                for (int j = n0; j < d.b_node0[o.body + 1]; j++) {
-                    const double2 p = a[j], w = d.mass[j];
-                    x += p.x * w.x;
-                    y += p.y * w.y;
-                    m += w.x;
-                }
-                x /= m;
-                y /= m;
-            } else {
-                const double* rg = d.rg + (size_t)MEL_RIGID_NF * o.body;
-                x = rg[rx]; y = rg[rx + 1]; r = rg[rx + 2];
+    mon_value q = { 0., 0., 0., 0., 0 };
+    if (o.type <= 3) {
+        // Position, Displacement, Velocity, Acceleration (Monitoring.h:33-192)
+        const double2* a = o.type == 0 ? d.x : o.type == 1 ? d.u : o.type == 2 ? d.v : d.a;
+        const int rx = o.type == 0 ? MEL_RG_XC : o.type == 1 ? MEL_RG_XD : o.type == 2 ? MEL_RG_XV : MEL_RG_XA;
+        const int n0 = d.b_node0[o.body];
+        q.has = 3;
+        if (o.node >= 0) {
+            const double2 p = a[n0 + o.node];
+            q.x = p.x; q.y = p.y;
+        } else if (d.b_type[o.body] == MEL_BODY_DEFORMABLE) {
+            double m = 0.;
+            for (int j = n0; j < d.b_node0[o.body + 1]; j++) {
+                const double2 p = a[j], w = d.mass[j];
+                q.x += p.x * w.x;
+                q.y += p.y * w.y;
+                m += w.x;
             }
-            if (o.kind == 0) row[c++] = x;
-            else if (o.kind == 1) row[c++] = y;
-            else if (o.type == 0) { if (o.kind == 2) row[c++] = r; }
-            else if (o.kind == 2) row[c++] = sqrt(x * x + y * y);   // pow(.,0.5): both correctly rounded
-            else if (o.kind == 3) row[c++] = r;
-        } else if (o.type == 4) {
-            // Force (Monitoring.h:193-338): o.sub = force kind, o.body, o.node
-            const int b = o.body;
-            if (o.node >= 0) {
-                const double2 f = node_force(d, b, d.b_node0[b] + o.node, o.sub);
-                x = f.x; y = f.y;
-            } else if (d.b_type[b] == MEL_BODY_DEFORMABLE) {
-                // the reference bounds this loop by the node count of body number o.sub
-                // (Monitoring.h:232); the host checked that it stays inside body b
-                x = 0.; y = 0.;
-                const int n0 = d.b_node0[b], cnt = d.b_node0[o.sub + 1] - d.b_node0[o.sub];
-                for (int j = 0; j < cnt; j++) {
-                    const double2 f = node_force(d, b, n0 + j, o.sub);
-                    x += f.x;
-                    y += f.y;
-                }
-            } else {
-                const double* rf = d.rf + 15 * b;
-                const int s = o.sub;
-                if (s == 0) { x = d.rtot[3 * b]; y = d.rtot[3 * b + 1]; r = d.rtot[3 * b + 2]; }
-                else if (s >= 2 && s <= 6) { const int q = 3 * (s - 2); x = rf[q]; y = rf[q + 1]; r = rf[q + 2]; }
+            q.x /= m;
+            q.y /= m;
+        } else {
+            const double* rg = d.rg + (size_t)MEL_RIGID_NF * o.body;
+            q.x = rg[rx]; q.y = rg[rx + 1]; q.r = rg[rx + 2];
+            q.has = 7;
+        }
+    } else if (o.type == 4) {
+        // Force (Monitoring.h:193-338): o.sub = force kind, o.body, o.node
+        const int b = o.body;
+        if (o.node >= 0) {
+            const double2 f = node_force(d, b, d.b_node0[b] + o.node, o.sub);
+            q.x = f.x; q.y = f.y; q.has = 3;
+        } else if (d.b_type[b] == MEL_BODY_DEFORMABLE) {
+            // the reference bounds this loop by the node count of body number o.sub
+            // (Monitoring.h:232); the host checked that it stays inside body b
+            const int n0 = d.b_node0[b], cnt = d.b_node0[o.sub + 1] - d.b_node0[o.sub];
+            for (int j = 0; j < cnt; j++) {
+                const double2 f = node_force(d, b, n0 + j, o.sub);
+                q.x += f.x;
+                q.y += f.y;
             }
-            if (o.kind == 0) row[c++] = x;
-            else if (o.kind == 1) row[c++] = y;
-            else if (o.kind == 2) row[c++] = sqrt(x * x + y * y);
-            else if (o.kind == 3) row[c++] = r;
-        } else if (o.type == 7) {
-            // Contact (Monitoring.h:362-382): the body's first contact element of that slave node
-            for (int j = d.b_cont0[o.body]; j < d.b_cont0[o.body + 1]; j++) {
-                const mel_contact& e = d.cont[j];
-                if (e.borderS == o.border && e.border_nodeS == o.bnode) {
-                    if (o.kind == 0) row[c++] = e.gapn;
-                    else if (o.kind == 1) row[c++] = e.gapt;
-                    else if (o.kind == 2) row[c++] = e.xsi;
-                    else if (o.kind == 3) row[c++] = e.xnorm;
-                    else if (o.kind == 4) row[c++] = e.ynorm;
-                    else if (o.kind == 5) row[c++] = e.internal[0];
-                    break;
-                }
-            }
-        } else if (o.type == 8) {
-            // Damage (Monitoring.h:385-390): Update_damage of the body, then its damage
-            row[c++] = body_damage(d, o.body);
-        } else if (o.type == 9) {
-            // Energy (Monitoring.h:390-458); the elastic energy of both material laws is zero
-            // (Code/Model.h:19-73 set energy = 0), so Deformation entries read +0
-            x = 0.;
-            if (o.body >= 0) {
-                if (o.kind == 0) {
-                    if (d.b_type[o.body] == MEL_BODY_DEFORMABLE) {
-                        for (int j = d.b_node0[o.body]; j < d.b_node0[o.body + 1]; j++) {
-                            const double2 w = d.vp[j], ms = d.mass[j];
-                            x += 0.5 * w.x * w.x * ms.x;
-                            x += 0.5 * w.y * w.y * ms.y;
-                        }
-                    } else {
-                        x = part[3 * o.body + 1];
-                    }
-                }
-            } else if (o.body == -1 && o.kind == 0) {
-                for (int b = 0; b < d.nb; b++) x += part[3 * b + 1];
-            }
-            row[c++] = x;
-        } else if (o.type == 10) {
-            // Work (Monitoring.h:459-503)
-            if (o.body >= 0) {
-                if (o.kind >= 0 && o.kind < 7) row[c++] = d.works[7 * o.body + o.kind];
-            } else if (o.body == -1) {
-                x = 0.;
-                if (o.kind >= 0 && o.kind < 7)
-                    for (int b = 0; b < d.nb; b++) x += d.works[7 * b + o.kind];
-                row[c++] = x;
+            q.has = 3;
+        } else {
+            const double* rf = d.rf + 15 * b;
+            const int s = o.sub;
+            if (s == 0) { q.x = d.rtot[3 * b]; q.y = d.rtot[3 * b + 1]; q.r = d.rtot[3 * b + 2]; q.has = 7; }
+            else if (s >= 2 && s <= 6) { const int k = 3 * (s - 2); q.x = rf[k]; q.y = rf[k + 1]; q.r = rf[k + 2]; q.has = 7; }
+        }
+    } else if (o.type == 7) {
+        // Contact (Monitoring.h:362-382): the body's first contact element of that slave node
+        for (int j = d.b_cont0[o.body]; j < d.b_cont0[o.body + 1]; j++) {
+            const mel_contact& e = d.cont[j];
+            if (e.borderS == o.border && e.border_nodeS == o.bnode) {
+                q.has = 8;
+                if (o.kind == 0) q.v = e.gapn;
+                else if (o.kind == 1) q.v = e.gapt;
+                else if (o.kind == 2) q.v = e.xsi;
+                else if (o.kind == 3) q.v = e.xnorm;
+                else if (o.kind == 4) q.v = e.ynorm;
+                else if (o.kind == 5) q.v = e.internal[0];
+                else q.has = 0;
+                break;
             }
         }
-        // other entry types add no column (Monitoring.h handles types 0-10 only)
+    } else if (o.type == 9) {
+        // Energy (Monitoring.h:390-458); the elastic energy of both material laws is zero
+        // (Code/Model.h:19-73 set energy = 0), so Deformation entries read +0
+        q.has = 9;
+        if (o.body >= 0) {
+            if (o.kind == 0) {
+                if (d.b_type[o.body] == MEL_BODY_DEFORMABLE) {
+                    for (int j = d.b_node0[o.body]; j < d.b_node0[o.body + 1]; j++) {
+                        const double2 w = d.vp[j], ms = d.mass[j];
+                        q.x += 0.5 * w.x * w.x * ms.x;
+                        q.x += 0.5 * w.y * w.y * ms.y;
+                    }
+                } else {
+                    q.x = part[3 * o.body + 1];
+                }
+            }
+        } else if (o.body == -1 && o.kind == 0) {
+            q.x = ordered_sum(0., part + 1, d.nb, 3);
+        }
+        q.v = q.x;
+    } else if (o.type == 10) {
+        // Work (Monitoring.h:459-503)
+        if (o.body >= 0) {
+            if (o.kind >= 0 && o.kind < 7) { q.v = d.works[7 * o.body + o.kind]; q.has = 8; }
+        } else if (o.body == -1) {
+            if (o.kind >= 0 && o.kind < 7) q.x = ordered_sum(0., d.works + o.kind, d.nb, 7);
+            q.v = q.x;
+            q.has = 9;
+        }
     }
+    // Damage entries change the body's running value and wait for their turn; other entry types add
+    // no column (Monitoring.h handles types 0-10 only)
+    return q;
+}
+
+// one row of Monitoring (Code/Monitoring.h:8-559) into row[1..], its length into row[0].  One warp: a
+// lane per entry reads what the entry needs (a few dependent loads each, which one thread after
+// another would wait for in turn), then lane 0 goes through the entries in order.
+__device__ void mon_row(const mel_dev& d, const mel_mon_op* ops, int nops, int energy, int boundaries, const double* part, double* row,
+                        const mel_mon_head& hd)
+{
+    __shared__ mon_value s_q[32];
+    const int lane = threadIdx.x & 31;
+    // MONITOR_ENERGY (Monitoring.h:508-537): Dwork, elastic energy (zero), kinetic energy
+    double en = 0.;
+    if (energy && lane >= 30) en = ordered_sum(0., part + (lane == 30 ? 2 : 0), d.nb, 3);
+    const double dw = __shfl_sync(0xffffffffu, en, 30), ke = __shfl_sync(0xffffffffu, en, 31);
+    int c = 1;
+    if (lane == 0) {
+        row[c++] = hd.iteration; row[c++] = hd.time; row[c++] = hd.dt;
+        row[c++] = hd.neval; row[c++] = hd.max_error; row[c++] = hd.mean_error;
+    }
+    // x, y and r live across entries as in the reference, where an entry that does not assign
+    // one of them reads the value the previous entry left (never-assigned values start at 0)
+    double x = 0., y = 0., r = 0.;
+    for (int base = 0; base < nops; base += 32) {
+        if (base + lane < nops) s_q[lane] = mon_entry(d, ops[base + lane], part);
+        __syncwarp();
+        if (lane == 0)
+            for (int k = base; k < min(base + 32, nops); k++) {
+                const mel_mon_op o = ops[k];
+                const mon_value q = s_q[k - base];
+                if (q.has & 1) x = q.x;
+                if (q.has & 2) y = q.y;
+                if (q.has & 4) r = q.r;
+                if (q.has & 8) row[c++] = q.v;
+                else if (o.type <= 4) {
+                    if (o.kind == 0) row[c++] = x;
+                    else if (o.kind == 1) row[c++] = y;
+                    else if (o.type == 0) { if (o.kind == 2) row[c++] = r; }
+                    else if (o.kind == 2) row[c++] = sqrt(x * x + y * y);   // pow(.,0.5): both correctly rounded
+                    else if (o.kind == 3) row[c++] = r;
+                } else if (o.type == 8) {
+                    // Damage (Monitoring.h:385-390): Update_damage of the body, then its damage
+                    row[c++] = body_damage(d, o.body);
+                }
+            }
+        __syncwarp();
+    }
+    if (lane) return;
     if (energy) {
-        // MONITOR_ENERGY (Monitoring.h:508-537): Dwork, elastic energy (zero), kinetic energy
-        double dw = 0., ke = 0.;
-        for (int b = 0; b < d.nb; b++) { dw += part[3 * b + 2]; ke += part[3 * b]; }
         row[c++] = dw;
         row[c++] = 0.;
         row[c++] = ke;
@@ -252,6 +298,23 @@ __global__ void mon_row_kernel(mel_dev d, const mel_mon_op* ops, int nops, int e
         for (int k = 0; k < 4; k++) row[c++] = f[k];
     }
     row[0] = (double)(c - 1);
+}
+
+// the bodies' sums by all blocks, then the row by the block that ends last
+__global__ void __launch_bounds__(256) monitor_kernel(const __grid_constant__ mel_dev d, const mel_mon_op* ops, int nops, int energy,
+                                                      int boundaries, double* part, double* row, const __grid_constant__ mel_mon_head hd)
+{
+    mon_body(d, hd.dt, part);
+    unsigned* done = reinterpret_cast<unsigned*>(part + 3 * (size_t)d.nb);      // zero between launches
+    __shared__ bool s_last;
+    __threadfence();
+    __syncthreads();
+    if (threadIdx.x == 0) s_last = atomicAdd(done, 1u) == gridDim.x - 1;
+    __syncthreads();
+    if (!s_last || threadIdx.x >= 32) return;
+    __threadfence();
+    if (threadIdx.x == 0) *done = 0u;
+    mon_row(d, ops, nops, energy, boundaries, part, row, hd);
 }
 
 // Update_status (Code/Proximity.h:550-1007), one thread, entries in order.  e = the entry (type,
@@ -363,6 +426,5 @@ void mel_launch_status(const mel_dev& d, const double* entries, int n, cudaStrea
 void mel_launch_monitor(const mel_dev& d, const mel_mon_op* ops, int nops, int energy, int boundaries,
                         double* part, double* row, const mel_mon_head& hd, cudaStream_t s)
 {
-    if (d.nb > 0) mel::mon_body_kernel<<<(d.nb + 7) / 8, 256, 0, s>>>(d, hd.dt, part);
-    mel::mon_row_kernel<<<1, 32, 0, s>>>(d, ops, nops, energy, boundaries, part, row, hd);
+    mel::monitor_kernel<<<(d.nb + 7) / 8, 256, 0, s>>>(d, ops, nops, energy, boundaries, part, row, hd);
 }
