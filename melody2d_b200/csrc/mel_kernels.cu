@@ -20,6 +20,7 @@
 #include "mel_geometry.cuh"
 #include "mel_sincos.h"
 #include "mel_sums.cuh"
+#include "mel_dependent.cuh"
 
 namespace mel {
 
@@ -60,12 +61,6 @@ __device__ __forceinline__ double entry_length(const mel_dev& d, int b, int g, i
     if (d.b_type[b] == MEL_BODY_DEFORMABLE) return border_length(d, b, g, j);
     return d.e_len0[d.bd_e0[g] + j];
 }
-
-// Programmatic dependent launch of the step's kernels.  grid_wait: what the kernels before this one
-// wrote is there from here on (nothing to wait for in an ordinary launch); grid_release: the next
-// kernel of the stream may start.
-__device__ __forceinline__ void grid_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
-__device__ __forceinline__ void grid_release() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 
 // ------------------------------------------------------------------------------------------
 // contact kernel
@@ -2101,20 +2096,6 @@ void mel_launch_damping(const mel_dev& d, cudaStream_t s)
 {
     if (!d.fdamp || d.nn == 0) return;
     mel::damping_kernel<<<(2 * d.nn + 255) / 256, 256, 0, s>>>(d);
-}
-
-// launch that may start as soon as the kernel before it in the stream releases it
-template <class... P, class... A>
-static void launch_dependent(void (*k)(P...), int grid, int block, size_t smem, cudaStream_t s, A... args)
-{
-    cudaLaunchConfig_t c = {};
-    cudaLaunchAttribute a = {};
-    a.id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    a.val.programmaticStreamSerializationAllowed = 1;
-    c.gridDim = dim3((unsigned)grid); c.blockDim = dim3((unsigned)block);
-    c.dynamicSmemBytes = smem; c.stream = s;
-    c.attrs = &a; c.numAttrs = 1;
-    cudaLaunchKernelEx(&c, k, static_cast<P>(args)...);      // errors: cudaGetLastError by the caller, as for <<<>>>
 }
 
 void mel_launch_contact(const mel_dev& d, double law_dt_scale, cudaStream_t s)

@@ -36,8 +36,10 @@
 #include "mel_internal.h"
 #include "mel_geometry.cuh"
 #include "mel_prox_host.h"
+#include "mel_dependent.cuh"
 
-struct mel_scan_job { const int* in; int* out; int n; int* sums; };
+// total: where the sum of all entries goes as well (a pinned host word), or NULL
+struct mel_scan_job { const int* in; int* out; int n; int* sums; int* total; };
 
 namespace mel {
 
@@ -79,6 +81,8 @@ __device__ __forceinline__ int block_scan(int v, int* s, int& total)
 __global__ void __launch_bounds__(SCAN_BLOCK) scan_block_kernel(const __grid_constant__ scan_args A)
 {
     __shared__ int s[SCAN_BLOCK / 32];
+    grid_wait();
+    grid_release();
     const int j = block_job(A.J ? A.bpre : A.pre, A.nj);
     const mel_scan_job job = A.J ? A.J[j] : A.job[j];
     const int lb = blockIdx.x - (A.J ? A.bpre : A.pre)[j];
@@ -89,11 +93,16 @@ __global__ void __launch_bounds__(SCAN_BLOCK) scan_block_kernel(const __grid_con
     int total, at = block_scan(sum, s, total);
 #pragma unroll
     for (int k = 0; k < SCAN_PER; k++) { if (i0 + k <= job.n) job.out[i0 + k] = at; at += v[k]; }
-    if (threadIdx.x == SCAN_BLOCK - 1) job.sums[lb] = total;
+    if (threadIdx.x == SCAN_BLOCK - 1) {
+        job.sums[lb] = total;
+        if (job.total) *job.total = total;
+    }
 }
 // adds the scanned block totals (in) to out[0..n) block by block
 __global__ void __launch_bounds__(SCAN_BLOCK) scan_add_kernel(const __grid_constant__ scan_args A)
 {
+    grid_wait();
+    grid_release();
     const int j = block_job(A.J ? A.bpre : A.pre, A.nj);
     const mel_scan_job job = A.J ? A.J[j] : A.job[j];
     const int lb = blockIdx.x - (A.J ? A.bpre : A.pre)[j];
@@ -657,6 +666,8 @@ __global__ void __launch_bounds__(FIND_THREADS) find_kernel(const mel_prox_job* 
     }
     if (threadIdx.x == 0) s_n = 0;
     __syncthreads();
+    grid_wait();
+    grid_release();
     const mel_prox_job& j = sj;
     const mel_dev& d = sj.d;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -896,6 +907,8 @@ static_assert(PROX_THREADS == PROX_THREADS_CL, "cell-list scratch is sized for t
             for (int k = threadIdx.x; k < (int)(sizeof(mel_prox_job) / sizeof(int)); k += blockDim.x) dst[k] = src[k]; \
         }                                                                                           \
         __syncthreads();                                                                            \
+        grid_wait();                                                                                \
+        grid_release();                                                                             \
         const int it = ((int)blockIdx.x - (J ? bpre[jj] : 0)) * (PROX_THREADS / (TPI)) + (int)threadIdx.x / (TPI); \
         const int lane = threadIdx.x & 31;                                                          \
         (void)lane;                                                                                 \
@@ -916,14 +929,15 @@ JOB_KERNEL(cl_zero_kernel, 1, cl_zero_item(j, it))
 JOB_KERNEL(cl_count_kernel, 1, cl_count_item(j, it))
 JOB_KERNEL(cl_fill_kernel, 1, cl_fill_item(j, it))
 JOB_KERNEL(cl_neighbour_kernel, 32, cl_neighbour_item(j, it, lane))
+// (a run leaves these at zero; cleared for new buffers and after a run that stopped half way)
 JOB_KERNEL(clear_kernel, 1,
-    if (it <= j.ntask) j.tcand[it] = 0;
+    if (it < j.tcand_n) j.tcand[it] = 0;
     if (it <= d.nb) j.inc_cnt[it] = 0;
     if (it == 0) *j.ncand = 0)
 JOB_KERNEL(bucket_kernel, 1, bucket_item(j, it))
 JOB_KERNEL(write_kernel, 32, write_item(j, it, lane))
 JOB_KERNEL(inc_fill_kernel, 1, inc_fill_item(j, it))
-JOB_KERNEL(bodies_kernel, 32, body_item(j, it, lane))
+JOB_KERNEL(bodies_kernel, 32, body_item(j, it, lane); if (it == 0 && lane == 0) *j.ncand = 0)
 JOB_KERNEL(body_range_kernel, 1, body_range_item(d.cont, d.ncont, d.nb, j.b_cont0, it))
 
 // one block per member: tasks and slots of every body, their offsets (btask0, bslot0), and the words
@@ -931,6 +945,8 @@ JOB_KERNEL(body_range_kernel, 1, body_range_item(d.cont, d.ncont, d.nb, j.b_cont
 __global__ void __launch_bounds__(1024) tasks_kernel(const mel_prox_job* J, int nj, const __grid_constant__ mel_prox_job one)
 {
     __shared__ int s[32];
+    grid_wait();
+    grid_release();
     const mel_prox_job& j = J ? J[blockIdx.x] : one;
     const mel_dev& d = j.d;
     int t0 = 0, s0 = 0;
@@ -969,15 +985,6 @@ __global__ void nbr_clear_kernel(const mel_prox_job* J, int nj, const __grid_con
     d.err[MEL_E_NBR_OVERFLOW] = 0u;
     d.err[MEL_E_NBR_NEED] = 0u;
 }
-// one thread per member: the new list's length, for the host (word 5)
-__global__ void readback_kernel(const mel_prox_job* J, int nj, const __grid_constant__ mel_prox_job one)
-{
-    const int k = blockIdx.x * blockDim.x + threadIdx.x;
-    if (k >= nj) return;
-    const mel_prox_job& j = J ? J[k] : one;
-    j.readback[5] = j.toff[j.ntask];
-}
-
 } // namespace mel
 
 // =============================================================================================
@@ -1021,7 +1028,7 @@ static bool sync_failed(cudaStream_t s, int line)
 // each synchronisation of the stream.  The read-back words of the members live apart.
 struct mel_prox_stage {
     char* h = nullptr; char* dv = nullptr; size_t cap = 0, used = 0;
-    int* rb_h = nullptr; int* rb_d = nullptr; int rb_cap = 0;    // 8 words per member; rb_d[8 * rb_cap] = 0
+    int* rb = nullptr; int rb_cap = 0;       // 8 words per member, pinned host memory the kernels write to
     std::vector<std::pair<char*, char*>> retired;               // outgrown buffers, freed after a sync
 };
 
@@ -1037,8 +1044,7 @@ void mel_prox_stage_free(mel_prox_stage* S)
     stage_release_retired(*S);
     if (S->h) cudaFreeHost(S->h);
     if (S->dv) cudaFree(S->dv);
-    if (S->rb_h) cudaFreeHost(S->rb_h);
-    if (S->rb_d) cudaFree(S->rb_d);
+    if (S->rb) cudaFreeHost(S->rb);
     delete S;
 }
 
@@ -1100,13 +1106,13 @@ int launch_jobs(run_ctx& C, job_kernel_t k, const job_table& T, const std::vecto
     if (bpre[nj] == 0) return MEL_OK;
     const int* dp = T.J ? (const int*)stage_upload(C.S, bpre.data(), sizeof(int) * (nj + 1), C.s) : nullptr;
     if (T.J && !dp) { mel_set_error("proximity staging upload failed"); return MEL_ERR_CUDA; }
-    k<<<bpre[nj], threads, 0, C.s>>>(T.J, dp, nj, T.one);
+    launch_dependent(k, bpre[nj], threads, 0, C.s, T.J, dp, nj, T.one);
     C.launches++;
     return MEL_OK;
 }
 
 // exclusive scans: req[j] scans in[0..n) into out[0..n] using the scratch ws (scan_scratch_ints(n))
-struct scan_req { const int* in; int* out; int n; int* ws; };
+struct scan_req { const int* in; int* out; int n; int* ws; int* total = nullptr; };
 // the jobs and block prefixes of a scan launch, as its argument or on the device
 bool scan_pack(run_ctx& C, const std::vector<mel_scan_job>& jobs, const std::vector<int>& bpre, mel::scan_args& A)
 {
@@ -1132,23 +1138,23 @@ int scan_many(run_ctx& C, const std::vector<scan_req>& req)
     std::vector<scan_req> next;
     for (int j = 0; j < nj; j++) {
         const int nblk = (req[j].n + SCAN_ITEMS) / SCAN_ITEMS;      // covers index n as well
-        jobs[j] = { req[j].in, req[j].out, req[j].n, req[j].ws };
+        jobs[j] = { req[j].in, req[j].out, req[j].n, req[j].ws, nblk > 1 ? nullptr : req[j].total };
         bpre[j + 1] = bpre[j] + nblk;
         if (nblk > 1) {                                              // block totals scanned the same way
             int* soff = req[j].ws + nblk + 1;
-            next.push_back({ req[j].ws, soff, nblk, soff + nblk + 2 });
-            adds.push_back({ soff, req[j].out, req[j].n + 1, nullptr });
+            next.push_back({ req[j].ws, soff, nblk, soff + nblk + 2, req[j].total });
+            adds.push_back({ soff, req[j].out, req[j].n + 1, nullptr, nullptr });
             apre.push_back(apre.back() + nblk);
         }
     }
     mel::scan_args A;
     if (!scan_pack(C, jobs, bpre, A)) return MEL_ERR_CUDA;
-    mel::scan_block_kernel<<<bpre[nj], SCAN_BLOCK, 0, C.s>>>(A);
+    launch_dependent(mel::scan_block_kernel, bpre[nj], SCAN_BLOCK, 0, C.s, A);
     C.launches++;
     if (next.empty()) return MEL_OK;
     if (int rc = scan_many(C, next)) return rc;
     if (!scan_pack(C, adds, apre, A)) return MEL_ERR_CUDA;
-    mel::scan_add_kernel<<<apre.back(), SCAN_BLOCK, 0, C.s>>>(A);
+    launch_dependent(mel::scan_add_kernel, apre.back(), SCAN_BLOCK, 0, C.s, A);
     C.launches++;
     return MEL_OK;
 }
@@ -1164,7 +1170,7 @@ mel_prox_job make_job(const mel_prox_member& m, int* readback)
     j.ntask = P.ntask; j.nslot = P.nslot; j.have_old = m.d->ncont > 0 ? 1 : 0;
     j.btask0 = P.btask0; j.bslot0 = P.bslot0;
     j.cand = (int4*)P.cand; j.cand_cap = P.cand_cap; j.ncand = P.ncand; j.ncont_new = P.ncont_new;
-    j.tcand = P.tcand; j.toff = P.toff; j.bucket = P.bucket; j.tkey = P.tkey;
+    j.tcand = P.tcand; j.tcand_n = (int)(P.tcand_bytes / sizeof(int)); j.toff = P.toff; j.bucket = P.bucket; j.tkey = P.tkey;
     j.inc_task = P.inc_task; j.inc_cnt = P.inc_cnt;
     j.inc_rng = P.inc_rng; j.b_inc0 = P.b_inc0; j.b_cont0 = P.b_cont0;
     j.cont_new = P.cont_alt;
@@ -1178,7 +1184,7 @@ mel_prox_job make_job(const mel_prox_member& m, int* readback)
 bool make_jobs(run_ctx& C, mel_prox_member* m, const std::vector<int>& idx, std::vector<mel_prox_job>& hj, job_table& T)
 {
     hj.clear();
-    for (int i : idx) hj.push_back(make_job(m[i], C.S.rb_d + 8 * i));
+    for (int i : idx) hj.push_back(make_job(m[i], C.S.rb + 8 * i));
     T.J = nullptr;
     T.one = hj[0];
     if (hj.size() == 1) return true;
@@ -1200,22 +1206,18 @@ bool stage_ready(mel_prox_stage*& stage, int n)
     if (!stage) stage = new mel_prox_stage();
     mel_prox_stage& S = *stage;
     if (S.rb_cap >= n) return true;
-    if (S.rb_h) { cudaFreeHost(S.rb_h); S.rb_h = nullptr; }
-    if (S.rb_d) { cudaFree(S.rb_d); S.rb_d = nullptr; }
+    if (S.rb) { cudaFreeHost(S.rb); S.rb = nullptr; }
     S.rb_cap = 0;
     const int cap = std::max(n, 16);
-    if (cudaMallocHost(&S.rb_h, sizeof(int) * 8 * (size_t)cap) != cudaSuccess) return false;
-    if (cudaMalloc(&S.rb_d, sizeof(int) * (8 * (size_t)cap + 1)) != cudaSuccess) return false;
-    if (cudaMemset(S.rb_d, 0, sizeof(int) * (8 * (size_t)cap + 1)) != cudaSuccess) return false;
+    if (cudaMallocHost(&S.rb, sizeof(int) * 8 * (size_t)cap) != cudaSuccess) return false;
+    memset(S.rb, 0, sizeof(int) * 8 * (size_t)cap);
     S.rb_cap = cap;
     return true;
 }
 
-// read-back words of members 0..n-1 to the host (one copy, one synchronisation); the stage space is
-// free again afterwards
-bool read_back(run_ctx& C, int n)
+// waits until the members' read-back words are there; the stage space is free again afterwards
+bool read_back(run_ctx& C)
 {
-    if (cudaMemcpyAsync(C.S.rb_h, C.S.rb_d, sizeof(int) * 8 * (size_t)n, cudaMemcpyDeviceToHost, C.s) != cudaSuccess) return false;
     if (sync_failed(C.s, __LINE__)) return false;
     C.S.used = 0;
     stage_release_retired(C.S);
@@ -1268,12 +1270,12 @@ int mel_run_proximity_many(mel_prox_member* m, int n, mel_prox_stage*& stage, in
         }
         if (any_ap)
             if ((rc = launch_jobs(C, neighbour_kernel, T, items_of(hj, [](const mel_prox_job& j) { return j.cl_on ? 0 : j.d.nb; }), 32))) return rc;
-        tasks_kernel<<<np, 1024, 0, s>>>(T.J, np, T.one); C.launches++;
+        launch_dependent(tasks_kernel, np, 1024, 0, s, T.J, np, T.one); C.launches++;
         if ((rc = launch_status(__LINE__))) return rc;
-        if (!read_back(C, n)) return MEL_ERR_CUDA;
+        if (!read_back(C)) return MEL_ERR_CUDA;
         std::vector<int> retry;
         for (int i : pend) {
-            const int* r = C.S.rb_h + 8 * i;
+            const int* r = C.S.rb + 8 * i;
             mel_prox_state& P = *m[i].P;
             if (r[0]) {
                 m[i].rc = MEL_ERR_NAN;
@@ -1310,7 +1312,9 @@ int mel_run_proximity_many(mel_prox_member* m, int n, mel_prox_stage*& stage, in
         for (int i : pend) {
             mel_prox_state& P = *m[i].P;
             const size_t nt = (size_t)P.ntask + 2;
+            const size_t had = P.tcand_bytes;
             if (ensure((void**)&P.tcand, &P.tcand_bytes, sizeof(int) * nt)) return MEL_ERR_OOM;
+            if (P.tcand_bytes != had) P.clear = true;
             if (ensure((void**)&P.toff, &P.toff_bytes, sizeof(int) * nt)) return MEL_ERR_OOM;
             if (ensure((void**)&P.tkey, &P.tkey_bytes, sizeof(int) * nt)) return MEL_ERR_OOM;
             if (ensure((void**)&P.cand, &P.cand_bytes, sizeof(int4) * 2 * 1024)) return MEL_ERR_OOM;
@@ -1318,18 +1322,25 @@ int mel_run_proximity_many(mel_prox_member* m, int n, mel_prox_stage*& stage, in
             if (ensure((void**)&P.scan_ws, &P.scan_ws_bytes, sizeof(int) * scan_scratch_ints(std::max(std::max(m[i].d->nb, P.ntask), P.cl_T)))) return MEL_ERR_OOM;
         }
         if (!make_jobs(C, m, pend, hj, T)) return MEL_ERR_CUDA;
-        if ((rc = launch_jobs(C, clear_kernel, T, items_of(hj, [](const mel_prox_job& j) { return std::max(j.ntask, j.d.nb) + 1; }), 1))) return rc;
+        bool any_clear = false;
+        std::vector<int> clear;
+        for (int i : pend) {
+            mel_prox_state& P = *m[i].P;
+            any_clear = any_clear || P.clear;
+            clear.push_back(P.clear ? std::max((int)(P.tcand_bytes / sizeof(int)) - 1, m[i].d->nb) + 1 : 0);
+            P.clear = true;                              // until the run is through
+        }
+        if (any_clear && (rc = launch_jobs(C, clear_kernel, T, clear, 1))) return rc;
         if ((rc = launch_jobs(C, find_kernel, T, items_of(hj, [](const mel_prox_job& j) { return j.ntask > 0 ? j.nslot : 0; }), 1, FIND_THREADS))) return rc;
         std::vector<scan_req> sc;
-        for (int i : pend) sc.push_back({ m[i].P->tcand, m[i].P->toff, m[i].P->ntask, m[i].P->scan_ws });
+        for (int i : pend) sc.push_back({ m[i].P->tcand, m[i].P->toff, m[i].P->ntask, m[i].P->scan_ws, C.S.rb + 8 * i + 5 });
         if ((rc = scan_many(C, sc))) return rc;
-        readback_kernel<<<((int)pend.size() + 127) / 128, 128, 0, s>>>(T.J, (int)pend.size(), T.one); C.launches++;
         if ((rc = launch_status(__LINE__))) return rc;
-        if (!read_back(C, n)) return MEL_ERR_CUDA;
+        if (!read_back(C)) return MEL_ERR_CUDA;
         std::vector<int> retry;
         for (int i : pend) {
             mel_prox_state& P = *m[i].P;
-            P.ncont_new = C.S.rb_h[8 * i + 5];
+            P.ncont_new = C.S.rb[8 * i + 5];
             if (P.ncont_new <= P.cand_cap) continue;
             if (ensure((void**)&P.cand, &P.cand_bytes, sizeof(int4) * 2 * (size_t)P.ncont_new)) return MEL_ERR_OOM;
             retry.push_back(i);
@@ -1368,6 +1379,7 @@ int mel_run_proximity_many(mel_prox_member* m, int n, mel_prox_stage*& stage, in
         std::swap(d.cont, P.cont_alt);
         std::swap(P.cont_bytes, P.cont_alt_bytes);
         d.ncont = P.ncont_new;
+        P.clear = false;                                 // bucket, inc_fill and bodies leave zeros
     }
     if (!make_jobs(C, m, act, hj, T)) return MEL_ERR_CUDA;
     if ((rc = launch_jobs(C, bodies_kernel, T, items_of(hj, [](const mel_prox_job& j) { return j.d.nb; }), 32))) return rc;

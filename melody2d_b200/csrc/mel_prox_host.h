@@ -15,6 +15,7 @@ struct mel_prox_state {
     void* cand = nullptr; size_t cand_bytes = 0;            // two int4 per candidate, in any order
     int cand_cap = 0, ncont_new = 0;                        // room for candidates, and how many were found
     int* ncand = nullptr;
+    bool clear = true;                                      // counters not known to be zero
     int* tcand = nullptr; size_t tcand_bytes = 0;           // candidates per task
     int* toff = nullptr; size_t toff_bytes = 0;             // first contact of each task in the new list
     int* tkey = nullptr; size_t tkey_bytes = 0;             // master body of each task with contacts
@@ -52,10 +53,10 @@ struct mel_prox_job {
     int ntask, nslot, have_old;
     int *btask0, *bslot0;
     int4* cand; int cand_cap, ncont_new; int* ncand;
-    int *tcand, *toff, *tkey, *bucket, *inc_task, *inc_cnt;
+    int *tcand, *toff, *tkey, *bucket, *inc_task, *inc_cnt; int tcand_n;
     int2* inc_rng; int* b_inc0; int* b_cont0;
     mel_contact* cont_new;        // the list being written (write stage)
-    int* readback;                // this member's words of the run's read-back array
+    int* readback;                // this member's words of the run's read-back array (host memory)
     int cl_on, cl_T, cl_ncx;      // cell-list broad phase (mel_prox_state)
     double cl_h, cl_hx;
     int *cl_cnt, *cl_cur, *cl_start, *cl_idx;
