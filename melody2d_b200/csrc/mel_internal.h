@@ -16,7 +16,7 @@
 #define MEL_CHUNK_GP_FP64 224     // Gauss points per chunk of a wide body: one point thread each
 #define MEL_PULL_WARPS 7          // warps 0-6 of the chunk loop: point pass, then pull
 #define MEL_PIECE 8               // entries of one node a lane of the mixed pull sums before the warp combines
-#define MEL_BAR_BYTES 128         // mbarriers and the abort flag
+#define MEL_BAR_BYTES 128         // mbarriers, the abort flag and the tail's ticket (at byte 64)
 #define MEL_PLACES(mixed) ((mixed) ? 16 : 8)      // slots of one shared-memory wavefront (8 or 16 bytes each)
 // head rows: derivative pairs of a point that its thread holds in registers (the rest are tail rows).
 // Measured on B200, body kernel of 700 grains of 384 nodes: FP64 with 16 / 12 / 8 / 4 head rows 237 /
@@ -246,11 +246,11 @@ void mel_launch_error_reduce(const mel_dev& d, double* out, cudaStream_t s);
 void mel_launch_drivendof(const mel_dev& d, double T, cudaStream_t s);
 // Body::Restore of the rigid bodies' kinematics from a copy of the rigid records
 void mel_launch_rigid_restore(const mel_dev& d, const double* rg_snap, cudaStream_t s);
-// one step of a batch: the contact pass over thr0[nsamp] threads, the body pass over cta0[nsamp]
-// CTAs and the per-sample time advance (devs, thr0, cta0 in device memory).  The body pass is two
+// one step of a batch: the contact pass over thr0[nsamp] threads, the body pass over the ncta
+// CTAs of cta (sample, CTA of the sample) and the per-sample time advance (devs, thr0, cta in device memory).  The body pass is two
 // launches: CTAs [0, ncta_small) with smem_small bytes (members whose bodies fit two CTAs per SM,
 // ordered first), then the rest with smem bytes
-void mel_launch_batch_step(const mel_dev* devs, const int* thr0, int nthr, const int* cta0, int ncta_small, int ncta,
+void mel_launch_batch_step(const mel_dev* devs, const int* thr0, int nthr, const int2* cta, int ncta_small, int ncta,
                            int nsamp, int mixed, size_t smem_small, size_t smem, cudaStream_t s);
 // shared memory of a body CTA: node arrays of max_nodes nodes beside `stage` bytes of Gauss-point
 // contributions or the post-loop arrays, whichever are larger

@@ -1164,7 +1164,7 @@ __device__ __forceinline__ void tile_forces(const mel_dev& d, int b, const typen
 //   s_up                   n + 1 double2       displacements (and a zero that padded rows name)
 //   s_f, s_fc              2 x n double2       internal forces, contact forces
 //   s_upf (mixed only)     n2 x float2         displacements relative to node 0 (n2 = n + 1 rounded to 2)
-//   mbarriers + abort flag                     MEL_BAR_BYTES
+//   mbarriers, abort flag, ticket              MEL_BAR_BYTES
 //   region                 a tile's contributions, index words and pull slots during the Gauss-point
 //                          pass, then s_fn, s_fd, s_vp, s_ap (n double2 each), the six work terms per
 //                          node (6 x n double) and, in the first half-step of Solver_step, the
@@ -1866,8 +1866,8 @@ __global__ void __launch_bounds__(256) copy_many_kernel(const __grid_constant__ 
 }
 
 // ---- batches: several independent models (samples) advanced by the same launches -----------
-// devs[s] is the descriptor of sample s; cta0 / thr0 are prefix sums of the samples' bodies and of
-// their contact-pass threads (contacts + border entries).  A sample's time lives in time2[0] and is
+// devs[s] is the descriptor of sample s; cta lists the samples' body CTAs (sample, CTA of the sample),
+// thr0 is a prefix sum of their contact-pass threads (contacts + border entries).  A sample's time lives in time2[0] and is
 // advanced by advance_kernel after each step.  Every sample runs exactly the code of a one-model
 // launch on its own arrays, so its results do not depend on the rest of the batch.
 __device__ __forceinline__ int batch_member(const int* prefix, int nsamp, int i)
@@ -1889,20 +1889,18 @@ __global__ void __launch_bounds__(128) contact_kernel_batch(const mel_dev* devs,
 }
 
 template <bool MX>
-__global__ void __launch_bounds__(MEL_BODY_THREADS, 2) body_kernel_batch(const mel_dev* devs, const int* cta0, int nsamp,
-                                                                         int cta_base)
+__global__ void __launch_bounds__(MEL_BODY_THREADS, 2) body_kernel_batch(const mel_dev* devs, const int2* cta, int cta_base)
 {
     extern __shared__ __align__(16) char smem[];
     __shared__ mel_dev sd;                   // the sample's descriptor, read once per CTA
-    const int c = (int)blockIdx.x + cta_base;
-    const int s = batch_member(cta0, nsamp, c);
+    const int2 c = cta[(int)blockIdx.x + cta_base];
     {
-        const int* src = reinterpret_cast<const int*>(devs + s);
+        const int* src = reinterpret_cast<const int*>(devs + c.x);
         int* dst = reinterpret_cast<int*>(&sd);
         for (int k = threadIdx.x; k < (int)(sizeof(mel_dev) / sizeof(int)); k += blockDim.x) dst[k] = src[k];
     }
     __syncthreads();
-    body_cta<MX>(sd, c - cta0[s], sd.time2[0], smem);
+    body_cta<MX>(sd, c.y, sd.time2[0], smem);
     grid_wait();
 }
 
@@ -2121,7 +2119,7 @@ size_t mel_body_smem_bytes(int max_nodes, size_t stage, int mixed)
     return r > rigid ? r : rigid;
 }
 
-void mel_launch_batch_step(const mel_dev* devs, const int* thr0, int nthr, const int* cta0, int ncta_small, int ncta,
+void mel_launch_batch_step(const mel_dev* devs, const int* thr0, int nthr, const int2* cta, int ncta_small, int ncta,
                            int nsamp, int mixed, size_t smem_small, size_t smem, cudaStream_t s)
 {
     if (nthr > 0) launch_dependent(mel::contact_kernel_batch, (nthr + 127) / 128, 128, 0, s, devs, thr0, nsamp, 1.0);
@@ -2130,13 +2128,13 @@ void mel_launch_batch_step(const mel_dev* devs, const int* thr0, int nthr, const
     bool after_contact = nthr > 0;
     // members whose bodies fit two CTAs per SM first, in their own launch, then the others
     if (ncta_small > 0) {
-        if (after_contact) launch_dependent(body, ncta_small, MEL_BODY_THREADS, smem_small, s, devs, cta0, nsamp, 0);
-        else body<<<ncta_small, MEL_BODY_THREADS, smem_small, s>>>(devs, cta0, nsamp, 0);
+        if (after_contact) launch_dependent(body, ncta_small, MEL_BODY_THREADS, smem_small, s, devs, cta, 0);
+        else body<<<ncta_small, MEL_BODY_THREADS, smem_small, s>>>(devs, cta, 0);
         after_contact = false;
     }
     if (ncta > ncta_small) {
-        if (after_contact) launch_dependent(body, ncta - ncta_small, MEL_BODY_THREADS, smem, s, devs, cta0, nsamp, ncta_small);
-        else body<<<ncta - ncta_small, MEL_BODY_THREADS, smem, s>>>(devs, cta0, nsamp, ncta_small);
+        if (after_contact) launch_dependent(body, ncta - ncta_small, MEL_BODY_THREADS, smem, s, devs, cta, ncta_small);
+        else body<<<ncta - ncta_small, MEL_BODY_THREADS, smem, s>>>(devs, cta, ncta_small);
     }
     mel::advance_kernel<<<(nsamp + 127) / 128, 128, 0, s>>>(devs, nsamp);
 }

@@ -5,6 +5,7 @@
 #include <cstdlib>
 #include <cstdio>
 #include <cstring>
+#include <climits>
 #include <cmath>
 #include <string>
 #include <numeric>
@@ -71,6 +72,7 @@ struct mel_handle {
     int parity = 0;
     size_t body_smem = 0;
     int nblocks_body = 0;     // body-kernel CTAs, and the wide bodies' CTAs after them
+    std::vector<int> cta_work; // their support entries (rigid bodies INT_MAX), in CTA order: what a batch sorts by
     int nwide = 0;
     int chunk_cap = 0;          // slots per tile chosen at build time
     double img_bytes = 0.;      // bytes of all chunk images
@@ -369,12 +371,19 @@ static mel_status build(mel_handle* h, const mel_model_desc* d, const mel_option
     for (int g = 0; g < nbd; g++)
         if (d->border_bc_type[2 * g] != MEL_BC_NONE || d->border_bc_type[2 * g + 1] != MEL_BC_NONE) has_bc[d->border_body[g]] = 1;
     D.b_has_bc = dupload(h, has_bc);
-    // CTA order of the body kernel: rigid bodies, deformable bodies, then the deformable bodies above
-    // MEL_MAX_BODY_NODES nodes, which run in a launch of their own (body_kernel_wide)
+    // CTA order of the body kernel: rigid bodies (they wait for the contact pass, and their sums are
+    // serial), deformable bodies from the most support entries to the fewest, so that the last wave of
+    // an uneven sample is of short CTAs, then the deformable bodies above MEL_MAX_BODY_NODES nodes, which
+    // run in a launch of their own (body_kernel_wide)
     std::vector<int> order;
     auto is_wide = [&](int b) { return d->body_type[b] != MEL_BODY_RIGID && d->body_node_ptr[b + 1] - d->body_node_ptr[b] > MEL_MAX_BODY_NODES; };
     for (int b = 0; b < nb; b++) if (d->body_type[b] == MEL_BODY_RIGID) order.push_back(b);
+    const size_t nrigid = order.size();
     for (int b = 0; b < nb; b++) if (d->body_type[b] != MEL_BODY_RIGID && !is_wide(b)) order.push_back(b);
+    auto entries = [&](int b) { return d->gp_sup_ptr[d->body_gp_ptr[b + 1]] - d->gp_sup_ptr[d->body_gp_ptr[b]]; };
+    std::stable_sort(order.begin() + nrigid, order.end(), [&](int x, int y) { return entries(x) > entries(y); });
+    h->cta_work.assign(nrigid, INT_MAX);
+    for (size_t i = nrigid; i < order.size(); i++) h->cta_work.push_back(entries(order[i]));
     h->nwide = 0;
     for (int b = 0; b < nb; b++) if (is_wide(b)) { order.push_back(b); h->nwide++; }
     D.b_order = dupload(h, order);
@@ -724,7 +733,8 @@ static mel_status build(mel_handle* h, const mel_model_desc* d, const mel_option
     cudaDeviceGetAttribute(&smem_sm, cudaDevAttrMaxSharedMemoryPerMultiprocessor, h->device);
     cudaDeviceGetAttribute(&smem_blk, cudaDevAttrMaxSharedMemoryPerBlockOptin, h->device);
     cudaDeviceGetAttribute(&smem_res, cudaDevAttrReservedSharedMemoryPerBlock, h->device);
-    const size_t two_per_sm = (size_t)(smem_sm / 2 - smem_res);
+    // (a batch's CTAs hold a member's descriptor beside it)
+    const size_t two_per_sm = (size_t)(smem_sm / 2 - smem_res) - sizeof(mel_dev);
     const bool mixed = h->precision == MEL_PREC_MIXED;
     {
         // slots per tile: MEL_TILE_SLOTS hold a full tile's points; fewer where the node arrays leave
@@ -765,7 +775,7 @@ static mel_status build(mel_handle* h, const mel_model_desc* d, const mel_option
         for (int ecap : { MEL_CHUNK_E_MAX, 1792, 1536, 1280, 1024, 768, 512, 256 }) {
             mel_status rc = mel_build_chunks(d, ecap, CS, mixed, 0, MEL_MAX_BODY_NODES);
             if (rc) return rc;
-            if (MEL_BAR_BYTES + 2 * (size_t)CS.img_max <= two_per_sm) break;
+            if (MEL_BAR_BYTES + 2 * (size_t)CS.img_max <= two_per_sm + sizeof(mel_dev)) break;    // (not in batches)
         }
         h->body_smem = std::max(h->body_smem, MEL_BAR_BYTES + 2 * (size_t)CS.img_max);
     }
@@ -2181,12 +2191,16 @@ struct mel_batch {
     cudaStream_t stream = nullptr;
     std::vector<mel_handle*> members;
     std::vector<mel_dev> h_devs;         // member descriptors as last uploaded
-    std::vector<int> h_thr0, h_cta0;     // prefix sums: contact-pass threads, body CTAs
+    std::vector<int> h_thr0;             // prefix sums: contact-pass threads
+    std::vector<int2> h_cta;             // the body launches' CTAs: member and its CTA
     mel_dev* d_devs = nullptr;
     int* d_thr0 = nullptr;
-    int* d_cta0 = nullptr;
+    int2* d_cta = nullptr;
     size_t cap = 0;                      // members the device arrays hold
+    size_t cta_cap = 0;                  // CTAs d_cta holds
+    int ncta_small = 0;                  // CTAs of the members that fit two per SM, listed first
     bool dirty = true;                   // descriptors changed (admission, retirement, proximity)
+    bool relist = true;                  // members changed (admission, retirement)
     size_t smem = 0;                     // largest body-kernel shared memory of the members
     size_t smem_small = 0;               // the same over the members that fit two CTAs per SM
     int nsmall = 0;                      // those members, ordered first
@@ -2204,11 +2218,10 @@ static mel_status batch_refresh(mel_batch* b)
     MEL_CUDA_OK(cudaStreamSynchronize(b->stream));
     if ((size_t)n > b->cap) {
         size_t cap = std::max((size_t)n, 2 * b->cap);
-        cudaFree(b->d_devs); cudaFree(b->d_thr0); cudaFree(b->d_cta0);
-        b->d_devs = nullptr; b->d_thr0 = nullptr; b->d_cta0 = nullptr;
+        cudaFree(b->d_devs); cudaFree(b->d_thr0);
+        b->d_devs = nullptr; b->d_thr0 = nullptr; b->cap = 0;
         if (cudaMalloc(&b->d_devs, sizeof(mel_dev) * cap) != cudaSuccess ||
-            cudaMalloc(&b->d_thr0, sizeof(int) * (cap + 1)) != cudaSuccess ||
-            cudaMalloc(&b->d_cta0, sizeof(int) * (cap + 1)) != cudaSuccess) {
+            cudaMalloc(&b->d_thr0, sizeof(int) * (cap + 1)) != cudaSuccess) {
             mel_set_error("batch descriptor allocation failed");
             return MEL_ERR_OOM;
         }
@@ -2218,7 +2231,7 @@ static mel_status batch_refresh(mel_batch* b)
         int smem_sm = 0, smem_res = 0;
         cudaDeviceGetAttribute(&smem_sm, cudaDevAttrMaxSharedMemoryPerMultiprocessor, b->device);
         cudaDeviceGetAttribute(&smem_res, cudaDevAttrReservedSharedMemoryPerBlock, b->device);
-        b->two_per_sm = (size_t)(smem_sm / 2 - smem_res);
+        b->two_per_sm = (size_t)(smem_sm / 2 - smem_res) - sizeof(mel_dev);
     }
     // members whose body kernel fits two CTAs per SM first: one launch of the body pass runs them
     // at that occupancy, a second the members that need more shared memory (one launch sized for
@@ -2227,20 +2240,41 @@ static mel_status batch_refresh(mel_batch* b)
                           [&](const mel_handle* h) { return h->body_smem <= b->two_per_sm; });
     b->h_devs.resize(n);
     b->h_thr0.assign(n + 1, 0);
-    b->h_cta0.assign(n + 1, 0);
     b->smem = 0; b->smem_small = 0; b->nsmall = 0;
     for (int i = 0; i < n; i++) {
         mel_handle* h = b->members[i];
         b->h_devs[i] = h->d;
         b->h_thr0[i + 1] = b->h_thr0[i] + h->d.ncont + h->d.ne;
-        b->h_cta0[i + 1] = b->h_cta0[i] + h->nblocks_body;
         b->smem = std::max(b->smem, h->body_smem);
         if (h->body_smem <= b->two_per_sm) { b->smem_small = std::max(b->smem_small, h->body_smem); b->nsmall = i + 1; }
     }
     if (n > 0) {
         MEL_CUDA_OK(cudaMemcpy(b->d_devs, b->h_devs.data(), sizeof(mel_dev) * n, cudaMemcpyHostToDevice));
         MEL_CUDA_OK(cudaMemcpy(b->d_thr0, b->h_thr0.data(), sizeof(int) * (n + 1), cudaMemcpyHostToDevice));
-        MEL_CUDA_OK(cudaMemcpy(b->d_cta0, b->h_cta0.data(), sizeof(int) * (n + 1), cudaMemcpyHostToDevice));
+    }
+    if (b->relist) {
+        // each launch's CTAs from the most work to the least over all its members, whose sizes differ
+        // (members one after the other: 8 samples of 100 grains of 64 to 576 nodes, mixed, 245 us a step, so 221)
+        std::vector<int2> l;
+        auto work = [&](const int2& x) { return b->members[x.x]->cta_work[x.y]; };
+        auto longer = [&](const int2& x, const int2& y) { return work(x) > work(y); };
+        for (int i = 0; i < n; i++) {
+            for (int c = 0; c < b->members[i]->nblocks_body; c++) l.push_back(make_int2(i, c));
+            if (i + 1 == b->nsmall) b->ncta_small = (int)l.size();
+        }
+        if (!b->nsmall) b->ncta_small = 0;
+        std::stable_sort(l.begin(), l.begin() + b->ncta_small, longer);
+        std::stable_sort(l.begin() + b->ncta_small, l.end(), longer);
+        if (l.size() > b->cta_cap) {
+            const size_t cap = std::max(l.size(), 2 * b->cta_cap);
+            cudaFree(b->d_cta);
+            b->d_cta = nullptr; b->cta_cap = 0;
+            if (cudaMalloc(&b->d_cta, sizeof(int2) * cap) != cudaSuccess) { mel_set_error("batch CTA list allocation failed"); return MEL_ERR_OOM; }
+            b->cta_cap = cap;
+        }
+        if (!l.empty()) MEL_CUDA_OK(cudaMemcpy(b->d_cta, l.data(), sizeof(int2) * l.size(), cudaMemcpyHostToDevice));
+        b->h_cta.swap(l);
+        b->relist = false;
     }
     b->dirty = false;
     return MEL_OK;
@@ -2274,7 +2308,7 @@ static void batch_drop_failed(mel_batch* b)
 {
     for (size_t i = 0; i < b->members.size();) {
         mel_handle* h = b->members[i];
-        if (h->failed) { b->members.erase(b->members.begin() + i); h->batch = nullptr; b->dirty = true; }
+        if (h->failed) { b->members.erase(b->members.begin() + i); h->batch = nullptr; b->dirty = b->relist = true; }
         else i++;
     }
 }
@@ -2323,7 +2357,7 @@ mel_status mel_batch_admit(mel_batch* b, mel_handle* h)
     }
     h->batch = b;
     b->members.push_back(h);
-    b->dirty = true;
+    b->dirty = b->relist = true;
     return MEL_OK;
 }
 
@@ -2334,7 +2368,7 @@ mel_status mel_batch_retire(mel_batch* b, mel_handle* h)
     MEL_CUDA_OK(cudaStreamSynchronize(b->stream));
     b->members.erase(std::find(b->members.begin(), b->members.end(), h));
     h->batch = nullptr;
-    b->dirty = true;
+    b->dirty = b->relist = true;
     return MEL_OK;
 }
 
@@ -2348,7 +2382,7 @@ mel_status mel_batch_step(mel_batch* b, int nsteps, int run_proximity)
         if (b->dirty) { mel_status rc = batch_refresh(b); if (rc) return rc; }
         const int n = (int)b->members.size();
         if (n == 0) break;
-        mel_launch_batch_step(b->d_devs, b->d_thr0, b->h_thr0[n], b->d_cta0, b->h_cta0[b->nsmall], b->h_cta0[n], n,
+        mel_launch_batch_step(b->d_devs, b->d_thr0, b->h_thr0[n], b->d_cta, b->ncta_small, (int)b->h_cta.size(), n,
                               b->precision == MEL_PREC_MIXED, b->smem_small, b->smem, b->stream);
         b->launches += 2 + (b->nsmall > 0) + (b->nsmall < n);
         cudaError_t le = cudaGetLastError();
@@ -2411,7 +2445,7 @@ mel_status mel_batch_destroy(mel_batch* b)
     cudaSetDevice(b->device);
     cudaStreamSynchronize(b->stream);
     for (mel_handle* h : b->members) h->batch = nullptr;
-    cudaFree(b->d_devs); cudaFree(b->d_thr0); cudaFree(b->d_cta0);
+    cudaFree(b->d_devs); cudaFree(b->d_thr0); cudaFree(b->d_cta);
     cudaEventDestroy(b->e0); cudaEventDestroy(b->e1);
     mel_prox_stage_free(b->pstage);
     cudaStreamDestroy(b->stream);

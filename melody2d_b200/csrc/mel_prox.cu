@@ -25,8 +25,8 @@
 // member; the host driver is at the end.
 //
 // What bounds it: latency.  A run is some fifteen short launches, each a chain of dependent loads.
-// Measured on B200, an update with its launch gaps and read-backs: 4x4 lattice 370 -> 123 us, 50
-// grains 486 -> 166 us, 700 grains 582 -> 216 us, against forty launches in which a thread per slot
+// Measured on B200, an update with its launch gaps and read-backs: 4x4 lattice 370 -> 95 us, 50
+// grains 486 -> 135 us, 700 grains 582 -> 175 us, against forty launches in which a thread per slot
 // walked its segments itself, once to count (68 us) and once to write (155 us).
 #include <cstdio>
 #include <cstring>
