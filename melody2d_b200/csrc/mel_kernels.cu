@@ -365,7 +365,8 @@ __device__ __forceinline__ void scatter_pairs(const mel_dev& d, int n0, int node
 // range, supports: about 2 us a pair, and a body in a compressed sample has 20 contacts of its own
 // and as many incoming ones with four master nodes each, so that this warp outlasted the
 // Gauss-point pass).  Here the lanes read 32 pairs at a time and only the pairs that carry
-// force are walked.
+// force are walked.  Measured on B200 with the staging of rigid bodies' contacts, 60 compressed grains
+// mixed: one step between host buffers 381 -> 319 us; a batch of 8 samples of 100 grains 429 -> 380 us a step.
 __device__ void contact_scatter(const mel_dev& d, int b, int n0, double2* acc, int lane)
 {
     const int mb = d.b_mat[b];
@@ -881,10 +882,11 @@ __device__ __forceinline__ float2 row_of(const float4& v, int r) { return r ? ma
 // them into registers, asked for while the tile before is finished, and half by a bulk copy; the
 // next tile's pairs are brought to L2 a tile ahead.  Shared memory carries the displacement gathers,
 // the contributions (each written and read once, without bank conflicts) and what the copies bring.
-// Measured on B200, 700 grains of 384 nodes: FP64 272 -> 183 us a launch, mixed 193 -> 146 us, against
+// Measured on B200 (body kernel, with its tail), 700 grains of 384 nodes: FP64 272 -> 182 us a launch,
+// mixed 193 -> 143 us; 2000 discs of 404 nodes: 0.664 -> 0.461 ms and 0.484 -> 0.347 ms, against
 // whole chunk images in two shared-memory buffers (each pair read three times there, both gathers
 // meeting banks twice on average, 134 points a chunk for 7 warps); 50 grains of 192 to 576 nodes,
-// one body an SM, FP64 122 -> 69 us.
+// one body an SM, FP64 122 -> 66 us.
 template <bool MX>
 __device__ __forceinline__ void tile_forces(const mel_dev& d, int b, const typename tile_rows_t<MX>::pair* s_u, double2* s_f,
                                             char* region, uint64_t* s_bar, volatile int* s_abort, int tid, int lane, int warp)
@@ -1771,8 +1773,9 @@ __device__ __forceinline__ void wide_body_cta(const mel_dev& d, int bb, double T
 // need its results: the body kernel starts beside it and waits (grid_wait) where it reads contact
 // forces, and before any CTA writes the positions and velocities that the contact pass reads.  The
 // contact pass waits for the body kernel before it, and only then lets the next one start, so that
-// no two body kernels ever run together.  Measured on B200, a step: 4x4 lattice 68 -> 61 us, 50 grains
-// FP64 127 -> 116 us, 700 grains FP64 251 -> 235 us, mixed 215 -> 200 us.
+// no two body kernels ever run together.  Measured on B200, a step with nothing else changed: 4x4
+// lattice 68 -> 61 us, 50 grains FP64 127 -> 116 us, 700 grains FP64 251 -> 235 us, mixed 215 -> 200 us
+// (with the proximity update as it is now the steps take 32, 78, 192 and 157 us).
 __global__ void __launch_bounds__(128) contact_kernel(const __grid_constant__ mel_dev d, double law_dt_scale, int czm_init)
 {
     grid_wait();

@@ -698,18 +698,14 @@ static mel_status build(mel_handle* h, const mel_model_desc* d, const mel_option
     h->H.b_per.assign(d->body_periodic, d->body_periodic + nb);
     h->H.b_bd0.assign(d->body_border_ptr, d->body_border_ptr + nb + 1);
     h->H.bd_e0.assign(d->border_node_ptr, d->border_node_ptr + nbd + 1);
-    // Gauss points: chunk images of <= gpcap points (one point thread each) and <= ecap support
-    // entries.  The entry cap is the largest that lets two body CTAs, each with its ring of
-    // MEL_STAGES images, share an SM; a body too large for that runs one CTA per SM.
-    // Bodies above MEL_MAX_BODY_NODES nodes keep their node arrays in global memory (gscr), so
-    // shared memory is sized by the others (max_def_nodes); max_all_nodes bounds the touched nodes
-    // of a chunk.
-    int max_def_nodes = 1, max_all_nodes = 1;
+    // Gauss points: tiles, and chunk images for the bodies above MEL_MAX_BODY_NODES nodes, which keep
+    // their node arrays in global memory (gscr), so that shared memory is sized by the others
+    // (max_def_nodes).
+    int max_def_nodes = 1;
     bool any_wide = false;
     for (int b = 0; b < nb; b++)
         if (d->body_type[b] == MEL_BODY_DEFORMABLE) {
             const int nnb = d->body_node_ptr[b + 1] - d->body_node_ptr[b];
-            max_all_nodes = std::max(max_all_nodes, nnb);
             if (nnb > MEL_MAX_BODY_NODES) any_wide = true;
             else max_def_nodes = std::max(max_def_nodes, nnb);
         }
