@@ -16,7 +16,7 @@
 #define MEL_CHUNK_GP_FP64 224     // Gauss points per chunk of a wide body: one point thread each
 #define MEL_PULL_WARPS 7          // warps 0-6 of the chunk loop: point pass, then pull
 #define MEL_PIECE 8               // entries of one node a lane of the mixed pull sums before the warp combines
-#define MEL_BAR_BYTES 128         // mbarriers, the abort flag and the tail's ticket (at byte 64)
+#define MEL_BAR_BYTES 128         // mbarriers, the flags of lost waits and the tail's ticket (at byte 64)
 #define MEL_PLACES(mixed) ((mixed) ? 16 : 8)      // slots of one shared-memory wavefront (8 or 16 bytes each)
 // head rows: derivative pairs of a point that its thread holds in registers (the rest are tail rows).
 // Measured on B200, body kernel of 700 grains of 384 nodes: FP64 with 16 / 12 / 8 / 4 head rows 237 /
@@ -27,6 +27,7 @@
 #define MEL_TILE_SLOTS_MAX 8192   // largest the tuning table may name
 #define MEL_CHUNK_E_MAX 2048      // support entries per chunk of a wide body, upper bound
 #define MEL_WAIT_NS 1000000000ull // bound of every device-side wait (1 s)
+#define MEL_WAIT_NOT (~0ull)      // a wait with this bound gives up without a look (tests)
 #define MEL_NBR_CAP_DEFAULT 64    // neighbour slots per body (grown on overflow)
 #define MEL_MAX_BODY_NODES 4096   // nodes per deformable body held in shared memory
 #define MEL_MAX_WIDE_NODES 65535  // larger bodies keep their node arrays in global memory (16-bit indices)
@@ -217,9 +218,10 @@ struct mel_dev {
     // gathered (contact << 2 | role, at most MEL_PRESSURE_CAP) and the pressures
     int* cp_cnt; int* cp_item;
     double *cpx, *cpy;
-    // bound of the body kernel's pipeline waits (MEL_WAIT_NS; the environment variable
-    // MELGPU_WAIT_NS read by mel_create shortens it so that tests can make a wait give up)
-    unsigned long long wait_ns;
+    // bounds of the body kernel's waits (MEL_WAIT_NS; the environment variables MELGPU_WAIT_NS, all of
+    // them, and MELGPU_TILE_WAIT_NS read by mel_create shorten them so that tests can make a wait
+    // give up): wait_tile_ns those for a tile's index words and for its pull sections
+    unsigned long long wait_ns, wait_tile_ns[2];
     // error words
     unsigned int* err;
 };

@@ -449,9 +449,9 @@ __device__ __forceinline__ unsigned long long global_ns()
     asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
     return t;
 }
-// wait for phase `parity` of `bar` to complete; gives up after `limit_ns` (the pipeline's waits use
-// mel_dev::wait_ns, MEL_WAIT_NS unless a test shortens it; the final wait for copies in flight
-// always allows MEL_WAIT_NS)
+// wait for phase `parity` of `bar` to complete; gives up after `limit_ns`, at once when that is MEL_WAIT_NOT
+// (the waits use mel_dev::wait_ns and wait_tile_ns, MEL_WAIT_NS unless a test shortens them; the
+// final wait for copies in flight always allows MEL_WAIT_NS)
 __device__ __forceinline__ bool mbar_test_wait(uint64_t* bar, unsigned parity)
 {
     unsigned ok;
@@ -462,6 +462,7 @@ __device__ __forceinline__ bool mbar_test_wait(uint64_t* bar, unsigned parity)
 __device__ bool mbar_wait_bounded(uint64_t* bar, unsigned parity, unsigned long long limit_ns = MEL_WAIT_NS)
 {
     if (limit_ns == 0) return mbar_test_wait(bar, parity);     // no waiting at all (tests)
+    if (limit_ns == MEL_WAIT_NOT) return false;
     if (mbar_try_wait(bar, parity)) return true;
     const unsigned long long t0 = global_ns();
     while (true) {
@@ -876,7 +877,13 @@ __device__ __forceinline__ float2 row_of(const float4& v, int r) { return r ? ma
 // subtracts its contributions.  Strain sums run in support order and every node's in ascending
 // point order, tile after tile, as the reference adds them.  The mixed form keeps derivative pairs,
 // strain, stress and contributions in FP32 (displacements relative to the body's first node) and the
-// nodes' sums in FP64.  Sets *s_abort when a wait gives up.
+// nodes' sums in FP64.
+//
+// A wait that gives up sets its own flag, s_lost[1] for the index words and s_lost[2] for the pull
+// sections ([0] is the displacements'), which every thread tests behind the next barrier, so that all
+// seven warps leave together.  A flag is set again only behind the barrier that follows its test: with
+// one flag for both waits a warp that had passed a barrier but not yet tested could find the
+// flag of the next wait, leave alone, and the others would stay in the barrier for good.
 //
 // What bounds it: latency.  The derivative pairs are read once (16 of the 20 bytes an entry), half of
 // them into registers, asked for while the tile before is finished, and half by a bulk copy; the
@@ -889,7 +896,7 @@ __device__ __forceinline__ float2 row_of(const float4& v, int r) { return r ? ma
 // one body an SM, FP64 122 -> 66 us.
 template <bool MX>
 __device__ __forceinline__ void tile_forces(const mel_dev& d, int b, const typename tile_rows_t<MX>::pair* s_u, double2* s_f,
-                                            char* region, uint64_t* s_bar, volatile int* s_abort, int tid, int lane, int warp)
+                                            char* region, uint64_t* s_bar, volatile int* s_lost, int tid, int lane, int warp)
 {
     typedef tile_rows_t<MX> rows_t;
     typedef typename rows_t::load load_t;
@@ -964,8 +971,8 @@ __device__ __forceinline__ void tile_forces(const mel_dev& d, int b, const typen
         if (more && tid == 0) l2_prefetch(d.timg + mel_tile_base(Tn.x), (unsigned)mel_tile_o_idx(Tn.y, Tn.z));
         const uint4 rn = point(more ? Tn : T);
         lane_t N = L;
-        bool ok = mbar_wait_bounded(bar_i, phase_i, d.wait_ns);
-        if (!ok) { atomicOr(&d.err[MEL_E_WAIT], 1u); *s_abort = 1; }
+        bool ok = mbar_wait_bounded(bar_i, phase_i, d.wait_tile_ns[0]);
+        if (!ok) { atomicOr(&d.err[MEL_E_WAIT], 1u); s_lost[1] = 1; }
         if (ok && L.K > 0) {
             const int lw = min(lane, L.w - 1);
             const load_t* const tail = reinterpret_cast<const load_t*>(s_idx) + L.t0 / PER + lw;
@@ -1101,13 +1108,13 @@ __device__ __forceinline__ void tile_forces(const mel_dev& d, int b, const typen
             for (int k = 0; k < HEAD; k += PER) fetch(g[k / PER], N, k);
         }
         compute_sync();
-        if (*s_abort) break;
+        if (s_lost[1]) break;
         if (more) {
             phase_i ^= 1u;
             if (tid == 0) { fence_proxy_async(); issue_idx(Tn); }
         }
-        ok = mbar_wait_bounded(bar_p, phase, d.wait_ns);
-        if (!ok) { atomicOr(&d.err[MEL_E_WAIT], 1u); *s_abort = 1; }
+        ok = mbar_wait_bounded(bar_p, phase, d.wait_tile_ns[1]);
+        if (!ok) { atomicOr(&d.err[MEL_E_WAIT], 1u); s_lost[2] = 1; }
         else {
             // pull: slot s is lane s & 31 of group s >> 5, groups sorted by entry count; warp w takes
             // groups w, 13 - w, 14 + w, ... so that the heavy ones are spread over the warps
@@ -1149,14 +1156,14 @@ __device__ __forceinline__ void tile_forces(const mel_dev& d, int b, const typen
             }
         }
         compute_sync();
-        if (*s_abort) break;
+        if (s_lost[2]) break;
         if (tid == 0 && more) { fence_proxy_async(); issue_pull(Tn); }
         L = N;
         T = Tn;
         Tn = Tnn;
         phase ^= 1u;
     }
-    if (*s_abort && tid == 0) {       // give the copies still in flight a bounded time to land
+    if (t < t1 && tid == 0) {         // a wait gave up: give the copies still in flight a bounded time to land
         mbar_wait_bounded(bar_i, phase_i);
         mbar_wait_bounded(bar_p, phase);
     }
@@ -1166,7 +1173,7 @@ __device__ __forceinline__ void tile_forces(const mel_dev& d, int b, const typen
 //   s_up                   n + 1 double2       displacements (and a zero that padded rows name)
 //   s_f, s_fc              2 x n double2       internal forces, contact forces
 //   s_upf (mixed only)     n2 x float2         displacements relative to node 0 (n2 = n + 1 rounded to 2)
-//   mbarriers, abort flag, ticket              MEL_BAR_BYTES
+//   mbarriers, flags of lost waits, ticket     MEL_BAR_BYTES
 //   region                 a tile's contributions, index words and pull slots during the Gauss-point
 //                          pass, then s_fn, s_fd, s_vp, s_ap (n double2 each), the six work terms per
 //                          node (6 x n double) and, in the first half-step of Solver_step, the
@@ -1196,14 +1203,14 @@ __device__ void deformable_body(const mel_dev& d, int b, double T, double T0, ch
         if (!chunk_forces<MX>(d, b, smem, s_up, s_f, s_fc, s_upf)) return;
     } else {
         uint64_t* s_bar = reinterpret_cast<uint64_t*>(s_after);
-        volatile int* s_abort = reinterpret_cast<volatile int*>(s_bar + 3);
+        volatile int* s_lost = reinterpret_cast<volatile int*>(s_bar + 3);
         // warp 0 has the displacement parameters brought by one bulk copy and waits for it; the others
         // clear the force sums.  s_bar[1] and s_bar[2] serve the tiles
         if (warp == 0) {
             if (lane == 0) {
                 for (int i = 0; i < 3; i++) mbar_init(s_bar + i, 1);
                 mbar_init_fence();
-                *s_abort = 0;
+                for (int i = 0; i < 3; i++) s_lost[i] = 0;
                 mbar_arrive_expect_tx(s_bar, (unsigned)(sizeof(double2) * n));
                 bulk_load(s_up, d.up + n0, (unsigned)(sizeof(double2) * n), s_bar);
                 // what padded rows and positions name: a zero displacement and a zero contribution
@@ -1212,7 +1219,7 @@ __device__ void deformable_body(const mel_dev& d, int b, double T, double T0, ch
                 else reinterpret_cast<double2*>(region)[d.tile_cap] = make_double2(0., 0.);
             }
             __syncwarp();
-            if (!mbar_wait_bounded(s_bar, 0u, d.wait_ns)) { atomicOr(&d.err[MEL_E_WAIT], 1u); *s_abort = 1; }
+            if (!mbar_wait_bounded(s_bar, 0u, d.wait_ns)) { atomicOr(&d.err[MEL_E_WAIT], 1u); s_lost[0] = 1; }
         } else {
             for (int i = tid - 32; i < n; i += blockDim.x - 32) {
                 s_f[i] = make_double2(0., 0.);
@@ -1220,7 +1227,7 @@ __device__ void deformable_body(const mel_dev& d, int b, double T, double T0, ch
             }
         }
         __syncthreads();
-        if (*s_abort) {
+        if (s_lost[0]) {
             if (tid == 0) mbar_wait_bounded(s_bar, 0u);   // give the copy in flight a bounded time to land
             return;
         }
@@ -1241,8 +1248,8 @@ __device__ void deformable_body(const mel_dev& d, int b, double T, double T0, ch
             if (k1 > k0) { l2_prefetch(d.ks_idx + k0, 2u * (k1 - k0)); l2_prefetch(d.ks_N + k0, 8u * (k1 - k0)); }
         }
         if (warp < MEL_BODY_CTHREADS / 32) {
-            if constexpr (MX) tile_forces<true>(d, b, s_upf, s_f, region, s_bar, s_abort, tid, lane, warp);
-            else tile_forces<false>(d, b, s_up, s_f, region, s_bar, s_abort, tid, lane, warp);
+            if constexpr (MX) tile_forces<true>(d, b, s_upf, s_f, region, s_bar, s_lost, tid, lane, warp);
+            else tile_forces<false>(d, b, s_up, s_f, region, s_bar, s_lost, tid, lane, warp);
         } else {                                           // warp 7, meanwhile
             grid_wait();
             contact_scatter(d, b, n0, s_fc, lane);
@@ -1256,7 +1263,10 @@ __device__ void deformable_body(const mel_dev& d, int b, double T, double T0, ch
     unsigned krec = d.ks_rec[ks + ki0];
     int kbase = d.kg_base[(ks + ki0) >> 5];
     __syncthreads();
-    if (!wide && *reinterpret_cast<volatile int*>(reinterpret_cast<uint64_t*>(s_after) + 3)) return;
+    if (!wide) {
+        const volatile int* s_lost = reinterpret_cast<volatile int*>(reinterpret_cast<uint64_t*>(s_after) + 3);
+        if (s_lost[1] | s_lost[2]) return;
+    }
     double2* s_fn = reinterpret_cast<double2*>(wide ? d.gscr + go + mel_wide_pre_bytes(n) : region);
     double2* s_fd = s_fn + n;
     double2* s_vp = s_fd + n;

@@ -305,6 +305,13 @@ static mel_status build(mel_handle* h, const mel_model_desc* d, const mel_option
         const unsigned long long v = strtoull(w, &end, 10);
         if (end && *end == 0 && v < MEL_WAIT_NS) D.wait_ns = v;
     }
+    D.wait_tile_ns[0] = D.wait_tile_ns[1] = D.wait_ns;
+    if (const char* w = getenv("MELGPU_TILE_WAIT_NS")) {  // test knob: "index,pull", -1 for a wait that gives up at once
+        long long v[2];
+        if (sscanf(w, "%lld,%lld", &v[0], &v[1]) == 2)
+            for (int k = 0; k < 2; k++)
+                if (v[k] < (long long)MEL_WAIT_NS) D.wait_tile_ns[k] = v[k] < 0 ? MEL_WAIT_NOT : (unsigned long long)v[k];
+    }
     // time
     double t2[2] = { d->time, d->time };
     D.time2 = dupload(h, t2, 2);
