@@ -26,8 +26,8 @@
 #define MEL_TILE_SLOTS 3840       // slots of a tile: 224 points of 15 supports on average, groups padded
 #define MEL_TILE_SLOTS_MAX 8192   // largest the tuning table may name
 #define MEL_CHUNK_E_MAX 2048      // support entries per chunk of a wide body, upper bound
-#define MEL_WAIT_NS 1000000000ull // bound of every device-side wait (1 s)
-#define MEL_WAIT_NOT (~0ull)      // a wait with this bound gives up without a look (tests)
+#define MEL_WAIT_NS 1000000000u   // bound of every device-side wait (1 s)
+#define MEL_WAIT_NOT 1u           // a wait with this bound gives up without a look (tests)
 #define MEL_NBR_CAP_DEFAULT 64    // neighbour slots per body (grown on overflow)
 #define MEL_MAX_BODY_NODES 4096   // nodes per deformable body held in shared memory
 #define MEL_MAX_WIDE_NODES 65535  // larger bodies keep their node arrays in global memory (16-bit indices)
@@ -177,7 +177,6 @@ struct mel_dev {
                                               // whose conditions are both none)
     int nblk;                                 // segment blocks (MEL_SEGB segments of one border)
     const int* bd_blk0;                       // [nbd+1] first block of each border
-    const int* blk_border;                    // border of each block
     double4* seg_blk;                         // block boxes of the current proximity update
     int nsblk;                                // superblocks (MEL_SEGB2 consecutive blocks of one border)
     const int* bd_sblk0;                      // [nbd+1] first superblock of each border
@@ -221,7 +220,7 @@ struct mel_dev {
     // bounds of the body kernel's waits (MEL_WAIT_NS; the environment variables MELGPU_WAIT_NS, all of
     // them, and MELGPU_TILE_WAIT_NS read by mel_create shorten them so that tests can make a wait
     // give up): wait_tile_ns those for a tile's index words and for its pull sections
-    unsigned long long wait_ns, wait_tile_ns[2];
+    unsigned wait_ns, wait_tile_ns[2];
     // error words
     unsigned int* err;
 };

@@ -459,10 +459,9 @@ __device__ __forceinline__ bool mbar_test_wait(uint64_t* bar, unsigned parity)
                  : "=r"(ok) : "r"(smem_u32(bar)), "r"(parity) : "memory");
     return ok != 0;
 }
-__device__ bool mbar_wait_bounded(uint64_t* bar, unsigned parity, unsigned long long limit_ns = MEL_WAIT_NS)
+__device__ bool mbar_wait_bounded(uint64_t* bar, unsigned parity, unsigned limit_ns = MEL_WAIT_NS)
 {
-    if (limit_ns == 0) return mbar_test_wait(bar, parity);     // no waiting at all (tests)
-    if (limit_ns == MEL_WAIT_NOT) return false;
+    if (limit_ns <= MEL_WAIT_NOT) return limit_ns == 0 && mbar_test_wait(bar, parity);     // no waiting at all (tests)
     if (mbar_try_wait(bar, parity)) return true;
     const unsigned long long t0 = global_ns();
     while (true) {

@@ -303,14 +303,14 @@ static mel_status build(mel_handle* h, const mel_model_desc* d, const mel_option
     if (const char* w = getenv("MELGPU_WAIT_NS")) {       // test knob: shorter pipeline waits
         char* end = nullptr;
         const unsigned long long v = strtoull(w, &end, 10);
-        if (end && *end == 0 && v < MEL_WAIT_NS) D.wait_ns = v;
+        if (end && *end == 0 && v < MEL_WAIT_NS) D.wait_ns = (unsigned)v;
     }
     D.wait_tile_ns[0] = D.wait_tile_ns[1] = D.wait_ns;
     if (const char* w = getenv("MELGPU_TILE_WAIT_NS")) {  // test knob: "index,pull", -1 for a wait that gives up at once
         long long v[2];
         if (sscanf(w, "%lld,%lld", &v[0], &v[1]) == 2)
             for (int k = 0; k < 2; k++)
-                if (v[k] < (long long)MEL_WAIT_NS) D.wait_tile_ns[k] = v[k] < 0 ? MEL_WAIT_NOT : (unsigned long long)v[k];
+                if (v[k] < (long long)MEL_WAIT_NS) D.wait_tile_ns[k] = v[k] < 0 ? MEL_WAIT_NOT : (unsigned)v[k];
     }
     // time
     double t2[2] = { d->time, d->time };
@@ -679,16 +679,14 @@ static mel_status build(mel_handle* h, const mel_model_desc* d, const mel_option
     D.cpx = dalloc<double>(h, (size_t)ne + 1);
     D.cpy = dalloc<double>(h, (size_t)ne + 1);
     {
-        std::vector<int> blk0(nbd + 1, 0), blk_border;
+        std::vector<int> blk0(nbd + 1, 0);
         for (int g = 0; g < nbd; g++) {
             int nseg = d->border_node_ptr[g + 1] - d->border_node_ptr[g] - 1;
             int nbk = (nseg + MEL_SEGB - 1) / MEL_SEGB;
             blk0[g + 1] = blk0[g] + nbk;
-            for (int k = 0; k < nbk; k++) blk_border.push_back(g);
         }
         D.nblk = blk0[nbd];
         D.bd_blk0 = dupload(h, blk0);
-        D.blk_border = dupload(h, blk_border);
         D.seg_blk = (double4*)dalloc<double>(h, 4 * (size_t)(D.nblk + 1));
         std::vector<int> sblk0(nbd + 1, 0), sblk_border;
         for (int g = 0; g < nbd; g++) {
@@ -908,7 +906,7 @@ static mel_status check_errors(mel_handle* h, const unsigned* words = nullptr)
     if (words) memcpy(w, words, sizeof w);
     else if (cudaMemcpy(w, h->d.err, sizeof w, cudaMemcpyDeviceToHost) != cudaSuccess) { mel_set_cuda_error(cudaGetLastError(), "err", __FILE__, __LINE__); return MEL_ERR_CUDA; }
     if (w[MEL_E_BOUNDS]) { mel_set_error("device index check failed (code %u)", w[MEL_E_BOUNDS]); return MEL_ERR_BOUNDS; }
-    if (w[MEL_E_WAIT]) { mel_set_error("a wait of the body kernel's pipeline gave up after %llu ns", h->d.wait_ns); return MEL_ERR_TIMEOUT; }
+    if (w[MEL_E_WAIT]) { mel_set_error("a wait of the body kernel's pipeline gave up after %u ns", h->d.wait_ns); return MEL_ERR_TIMEOUT; }
     if (w[MEL_E_DEACT]) {
         mel_set_error("body %u turned inactive while one of its contact elements carried a force: the reference keeps "
                       "sending that force to the other bodies for the rest of the run (its send list is no longer cleared, "
