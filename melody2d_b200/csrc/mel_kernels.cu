@@ -1188,7 +1188,7 @@ __device__ void deformable_body(const mel_dev& d, int b, double T, double T0, ch
     const int n0 = d.b_node0[b];
     const int n = d.b_node0[b + 1] - n0;
     if (n == 0) return;
-    const double dt = d.dt[0];
+    const double dt = ld_l2(d.dt);
     constexpr bool wide = WIDE;
     const long long go = WIDE ? d.b_gscr[b] : 0LL;
     double2* s_up = wide ? d.up + n0 : reinterpret_cast<double2*>(smem);
@@ -1255,12 +1255,14 @@ __device__ void deformable_body(const mel_dev& d, int b, double T, double T0, ch
         }
     }
     // the first node's masses and velocity parameters and the first kinematics slot, asked for before
-    // the barrier
+    // the barrier.  Every thread has waited for the contact pass here: the state is read plainly from now on
     const int i0 = min(tid, n - 1), ki0 = tid >= 32 ? min(tid - 32, n - 1) : 0;
     const int ks = d.b_ks0[b];
-    double2 m0 = d.mass[n0 + i0], im0 = d.minv[n0 + i0], vp0 = d.vp[n0 + i0];
+    double2 m0 = d.mass[n0 + i0], im0 = d.minv[n0 + i0];
     unsigned krec = d.ks_rec[ks + ki0];
     int kbase = d.kg_base[(ks + ki0) >> 5];
+    grid_wait();
+    double2 vp0 = d.vp[n0 + i0];
     __syncthreads();
     if (!wide) {
         const volatile int* s_lost = reinterpret_cast<volatile int*>(reinterpret_cast<uint64_t*>(s_after) + 3);
@@ -1521,12 +1523,12 @@ __device__ void rigid_body(const mel_dev& d, int b, double T, double T0, char* s
     const int tid = threadIdx.x;
     const int n0 = d.b_node0[b];
     const int n = d.b_node0[b + 1] - n0;
-    const double dt = d.dt[0];
+    const double dt = ld_l2(d.dt);
     double* rg = d.rg + MEL_RIGID_NF * b;
     double* rf = d.rf + 15 * b;
     double* sh = reinterpret_cast<double*>(smem);   // [0..14] forces, [16..23] drivendof, [24..32] sums
     double* sT = sh + 64;                            // staged border terms, 6 x MEL_RIGID_BATCH
-    const double xcs = rg[MEL_RG_XC], ycs = rg[MEL_RG_YC];   // centre at the start of the step
+    const double xcs = ld_l2(rg + MEL_RG_XC), ycs = ld_l2(rg + MEL_RG_YC);   // centre at the start of the step
     // ---- Update_bc_forces, rigid (Code/Body.h:800-899): terms of every border entry computed in
     // parallel, then each of the six sums (Neumann x, y, moment; Dirichlet x, y, moment) added
     // in entry order by one lane.  Borders whose conditions are all none or driven add only zero
@@ -1547,7 +1549,7 @@ __device__ void rigid_body(const mel_dev& d, int b, double T, double T0, char* s
                 int gn = n0 + d.e_node[e];
                 double length = d.e_len0[e];
                 double fxn = 0., fyn = 0., fxd = 0., fyd = 0.;
-                double2 ub = d.u[gn], vb = d.v[gn], xb = d.x[gn];
+                double2 ub = ld_l2(d.u + gn), vb = ld_l2(d.v + gn), xb = ld_l2(d.x + gn);
                 double px = 0., py = 0.;                  // Border::x_bc_pressure, y_bc_pressure
                 if (tx == MEL_BC_ORIENTED || tx == MEL_BC_FOLLOWING) { px = xv; fxn = px * length; }
                 else if (tx == MEL_BC_SOFT) { px = d.bd_bcp[4 * g] * (xv - ub.x) + d.bd_bcp[4 * g + 1] * (xvel - vb.x); fxd = px * length; }
@@ -1759,7 +1761,7 @@ template <bool MX, bool AD = false>
 __device__ __forceinline__ void body_cta(const mel_dev& d, int bb, double T, char* smem, double T0 = 0.)
 {
     int b = d.b_order[bb];
-    if (d.b_status[b] == MEL_STATUS_INACTIVE) return;
+    if (ld_l2(d.b_status + b) == MEL_STATUS_INACTIVE) return;
     if (d.any_damped && threadIdx.x == 32) { grid_wait(); contact_work(d, b); }
     if (d.b_type[b] == MEL_BODY_RIGID) rigid_body<AD>(d, b, T, T0, smem);
     else deformable_body<MX, AD, false>(d, b, T, T0, smem);
@@ -1782,7 +1784,10 @@ __device__ __forceinline__ void wide_body_cta(const mel_dev& d, int bb, double T
 // need its results: the body kernel starts beside it and waits (grid_wait) where it reads contact
 // forces, and before any CTA writes the positions and velocities that the contact pass reads.  The
 // contact pass waits for the body kernel before it, and only then lets the next one start, so that
-// no two body kernels ever run together.  Measured on B200, a step with nothing else changed: 4x4
+// no two body kernels ever run together; what the body kernel reads before its own wait (time, step,
+// status, displacement parameters, a rigid body's state) it reads from L2 (mel_dependent.cuh).  With a
+// damped law one thread of a body waits first, for the contact work it adds up, and its warp holds the
+// Gauss-point warps at their first barrier: such models run the two passes one after the other.  Measured on B200, a step with nothing else changed: 4x4
 // lattice 68 -> 61 us, 50 grains FP64 127 -> 116 us, 700 grains FP64 251 -> 235 us, mixed 215 -> 200 us
 // (with the proximity update as it is now the steps take 32, 78, 192 and 157 us).
 __global__ void __launch_bounds__(128) contact_kernel(const __grid_constant__ mel_dev d, double law_dt_scale, int czm_init)
@@ -1799,7 +1804,7 @@ __global__ void __launch_bounds__(MEL_BODY_THREADS, 2) body_kernel(const __grid_
 {
     extern __shared__ __align__(16) char smem[];
     grid_release();
-    const double T = d.time2[parity];
+    const double T = ld_l2(d.time2 + parity);
     body_cta<MX>(d, blockIdx.x, T, smem);
     grid_wait();          // a CTA that had nothing to wait for ends no earlier than the contact pass
     if (blockIdx.x == 0 && threadIdx.x == 0) d.time2[parity ^ 1] = T + d.dt[0];
@@ -1905,14 +1910,14 @@ __global__ void __launch_bounds__(MEL_BODY_THREADS, 2) body_kernel_batch(const m
 {
     extern __shared__ __align__(16) char smem[];
     __shared__ mel_dev sd;                   // the sample's descriptor, read once per CTA
-    const int2 c = cta[(int)blockIdx.x + cta_base];
+    const int2 c = ld_l2(cta + blockIdx.x + cta_base);
     {
         const int* src = reinterpret_cast<const int*>(devs + c.x);
         int* dst = reinterpret_cast<int*>(&sd);
-        for (int k = threadIdx.x; k < (int)(sizeof(mel_dev) / sizeof(int)); k += blockDim.x) dst[k] = src[k];
+        for (int k = threadIdx.x; k < (int)(sizeof(mel_dev) / sizeof(int)); k += blockDim.x) dst[k] = ld_l2(src + k);
     }
     __syncthreads();
-    body_cta<MX>(sd, c.y, sd.time2[0], smem);
+    body_cta<MX>(sd, c.y, ld_l2(sd.time2), smem);
     grid_wait();
 }
 
