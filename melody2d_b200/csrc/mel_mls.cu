@@ -25,6 +25,7 @@
 // conditioning, and they satisfy the linear reproducing conditions to round-off.
 #include <algorithm>
 #include <cstdio>
+#include <new>
 #include <vector>
 #include "mel_internal.h"
 
@@ -240,7 +241,7 @@ mel_status mel_mls_shapes(int n_bodies, const int* body_node_ptr, const double* 
                           const int* body_point_ptr, const double* points, long long* sup_ptr, int* sup_idx,
                           double* N, double* dNdx, double* dNdy, long long capacity, long long* n_entries, int device,
                           double* kernel_ms)
-{
+try {
     if (n_bodies <= 0 || !body_node_ptr || !nodes || !radii || !body_point_ptr || !points || !sup_ptr || !n_entries) {
         mel_set_error("invalid arguments");
         return MEL_ERR_INVALID;
@@ -317,4 +318,7 @@ mel_status mel_mls_shapes(int n_bodies, const int* body_node_ptr, const double* 
     MEL_CUDA_OK(cudaMemcpy(dNdx, d_Nx.p, sizeof(double) * ne, cudaMemcpyDeviceToHost));
     MEL_CUDA_OK(cudaMemcpy(dNdy, d_Ny.p, sizeof(double) * ne, cudaMemcpyDeviceToHost));
     return MEL_OK;
+} catch (const std::bad_alloc&) {                    // the list of slices
+    mel_set_error("no host memory for the slices of %d points", body_point_ptr[n_bodies]);
+    return MEL_ERR_OOM;
 }

@@ -3,6 +3,7 @@
 #include <atomic>
 #include <cstdlib>
 #include <cstring>
+#include <new>
 #include <numeric>
 #include <thread>
 #include "mel_tiles.h"
@@ -253,18 +254,24 @@ bool fill_tile(const mel_model_desc* d, const mel_tile& T, int g, int nnb, bool 
 
 }  // namespace
 
-// f(body, scratch) for every tiled body, on a few host threads (bodies are independent)
+// f(body, scratch) for every tiled body, on a few host threads (bodies are independent); false when memory
+// ran out in one of them (an exception must not leave a thread, nor this one while others run)
 template <class F>
-static void over_bodies(const mel_model_desc* d, F&& f)
+static bool over_bodies(const mel_model_desc* d, F&& f)
 {
     const int nb = d->n_bodies, hw = (int)std::thread::hardware_concurrency();
     const long long work = d->gp_sup_ptr[d->n_gauss];
     const int nthr = std::max(1, std::min({ hw > 0 ? hw : 1, 16, nb, (int)(work / 200000) + 1 }));
     std::atomic<int> next{ 0 };
+    std::atomic<bool> good{ true };
     auto run = [&]() {
-        scratch S;
-        for (int b; (b = next++) < nb;)
-            if (d->body_type[b] == MEL_BODY_DEFORMABLE && d->body_node_ptr[b + 1] - d->body_node_ptr[b] <= MEL_MAX_BODY_NODES) f(b, S);
+        try {
+            scratch S;
+            for (int b; good && (b = next++) < nb;)
+                if (d->body_type[b] == MEL_BODY_DEFORMABLE && d->body_node_ptr[b + 1] - d->body_node_ptr[b] <= MEL_MAX_BODY_NODES) f(b, S);
+        } catch (const std::bad_alloc&) {
+            good = false;
+        }
     };
     std::vector<std::thread> th;
     for (int i = 1; i < nthr; i++) {
@@ -272,15 +279,22 @@ static void over_bodies(const mel_model_desc* d, F&& f)
     }
     run();
     for (auto& t : th) t.join();
+    return good;
+}
+
+static mel_status no_memory()
+{
+    mel_set_error("no host memory for the Gauss-point tiles");
+    return MEL_ERR_OOM;
 }
 
 mel_status mel_plan_tiles(const mel_model_desc* d, int cap, bool mixed, mel_tile_set& out)
-{
+try {
     const int nb = d->n_bodies;
     if (cap < 256 * MEL_PLACES(mixed) || cap > 16384) { mel_set_error("tile cap %d out of range", cap); return MEL_ERR_INVALID; }
     std::vector<body_plan> plan(nb);
     std::vector<std::pair<mel_status, int>> rc(nb, { MEL_OK, 0 });
-    over_bodies(d, [&](int b, scratch& S) { rc[b] = plan_body(d, b, cap, mixed, plan[b], S); });
+    if (!over_bodies(d, [&](int b, scratch& S) { rc[b] = plan_body(d, b, cap, mixed, plan[b], S); })) return no_memory();
     for (int b = 0; b < nb; b++) {
         if (rc[b].first == MEL_OK) continue;
         if (rc[b].first == MEL_ERR_INVALID) mel_set_error("Gauss support index out of range");
@@ -312,19 +326,24 @@ mel_status mel_plan_tiles(const mel_model_desc* d, int cap, bool mixed, mel_tile
     out.b_tile0[nb] = (int)out.tiles.size();
     out.bytes = total;
     return MEL_OK;
+} catch (const std::bad_alloc&) {
+    return no_memory();
 }
 
 mel_status mel_fill_tiles(const mel_model_desc* d, mel_tile_set& out)
-{
+try {
     free(out.data);
     out.data = static_cast<uint8_t*>(calloc(std::max<size_t>(out.bytes, 16), 1));
     if (!out.data) { mel_set_error("host memory for the Gauss-point tiles (%zu bytes)", out.bytes); return MEL_ERR_OOM; }
     std::atomic<bool> good{ true };
-    over_bodies(d, [&](int b, scratch& S) {
+    const bool room = over_bodies(d, [&](int b, scratch& S) {
         const int nnb = d->body_node_ptr[b + 1] - d->body_node_ptr[b];
         for (int i = out.b_tile0[b]; i < out.b_tile0[b + 1]; i++)
             if (!fill_tile(d, out.tiles[i], out.gp0[i], nnb, out.mixed, out.cap, out.data + mel_tile_base(out.tiles[i].base), S)) good = false;
     });
+    if (!room) return no_memory();
     if (!good) { mel_set_error("the Gauss-point tiles do not hold their points"); return MEL_ERR_INVALID; }
     return MEL_OK;
+} catch (const std::bad_alloc&) {
+    return no_memory();
 }
