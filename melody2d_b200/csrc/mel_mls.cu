@@ -135,7 +135,8 @@ __global__ void __launch_bounds__(MLS_THREADS) mls_kernel(const int4* slice, int
     }
     __syncthreads();
     const double s = s_scale, is = 1.0 / s;
-    for (int p = sl.y + warp; p < sl.z; p += MLS_THREADS / 32) {
+    for (int k = warp; k < sl.z - sl.y; k += MLS_THREADS / 32) {
+        const int p = sl.y + k;
         const double2 xp = pts[p];
         if (PASS == 0) {
             const int c = supports_of(xp, nn, sx, sr, lane, nullptr, 0);
@@ -206,8 +207,8 @@ __global__ void __launch_bounds__(1024) mls_scan_kernel(const int* cnt, long lon
     __shared__ long long s_w[32];
     const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
     long long run = 0;
-    for (int base = 0; base <= n; base += 8192) {
-        const int i0 = base + 8 * t;
+    for (long long base = 0; base <= n; base += 8192) {      // 64 bits: n may be near the largest int
+        const long long i0 = base + 8 * t;
         int v[8];
         long long sum = 0;
 #pragma unroll
