@@ -8,8 +8,8 @@
 //   neighbour_kernel or cl_*   (body, border) overlap with periodic shifts and de-duplication
 //                      (Code/Proximity.h:112-169), one warp per body
 //   tasks_kernel       tasks and slots per body and their offsets: one task per (slave body, slave
-//                      border, neighbour) in the reference's loop order, then one self task per (slave
-//                      body, border); a slot per (task, slave border node)
+//                      border, neighbour, piece of the border) in the reference's loop order, then
+//                      self tasks per (slave body, border, piece); a slot per (task, slave border node)
 //   [host read-back]   task and slot totals of every member
 //   find_kernel        accepted candidates: a thread per slot tests the master's boxes, then a warp per
 //                      slot that is near one tests the segments; candidates are listed in any order
@@ -619,9 +619,17 @@ __device__ __forceinline__ double near_margin(const mel_dev& d, double2 xs, doub
 
 // ---------------------------------------------------------------------------------------------
 // tasks and slots.  A body's tasks are contiguous: (border, neighbour) pairs in the reference's loop
-// order (Code/Proximity.h:207-212), then one self task per border (Code/Proximity.h:346-356); its
-// slots likewise, a slot per slave border node of each task.
+// order (Code/Proximity.h:207-212), then self tasks per border (Code/Proximity.h:346-356); its
+// slots likewise, a slot per slave border node of each task.  A pair, or a border with itself, is cut
+// into pieces of TASK_NODES slave border nodes, a task each: a candidate finds its place by looking
+// through all of its task (write_item), which over a border of thousands of nodes is quadratic.
+// Measured on B200, two blocks of 10,000 contacts each: write_kernel 1,129 us with a task for the whole
+// border, 596 with pieces.  A grain's
+// border, 33 to 97 nodes, is one piece.
 // ---------------------------------------------------------------------------------------------
+#define TASK_NODES 128
+__device__ __forceinline__ int task_pieces(int nS) { return (nS + TASK_NODES - 1) / TASK_NODES; }
+
 __device__ __forceinline__ bool has_self(const mel_dev& d, int b)
 {
     return d.self_contact && d.b_type[b] == MEL_BODY_DEFORMABLE && !d.b_per[b];
@@ -638,22 +646,24 @@ __device__ __forceinline__ slot_ref slot_of(const mel_prox_job& j, int s)
     r.b = lo;
     int at = s - j.bslot0[lo];
     const int n = j.nbn[lo], g0 = d.b_bd0[lo], g1 = d.b_bd0[lo + 1];
-    int g = g0;
+    int g = g0, before = 0;                  // tasks before the border's (for the first of its neighbours)
     r.q = -1;
     for (; g < g1; g++) {                    // regular tasks
         const int nS = d.bd_e0[g + 1] - d.bd_e0[g];
-        if (at < n * nS) { r.q = at / nS; at -= r.q * nS; break; }
+        if (at < n * nS) { r.q = at / nS; at -= r.q * nS; before += r.q * task_pieces(nS); break; }
         at -= n * nS;
+        before += n * task_pieces(nS);
     }
     if (g == g1)                             // self tasks
         for (g = g0; g < g1 - 1; g++) {
             const int nS = d.bd_e0[g + 1] - d.bd_e0[g];
             if (at < nS) break;
             at -= nS;
+            before += task_pieces(nS);
         }
     r.g = g;
     r.kS = at;
-    r.t = j.btask0[lo] + (r.q >= 0 ? (g - g0) * n + r.q : (g1 - g0) * n + (g - g0));
+    r.t = j.btask0[lo] + before + at / TASK_NODES;
     return r;
 }
 
@@ -962,7 +972,8 @@ __global__ void __launch_bounds__(1024) tasks_kernel(const mel_prox_job* J, int 
         int tc = 0, sc = 0;
         if (b < d.nb) {
             const int g0 = d.b_bd0[b], g1 = d.b_bd0[b + 1], per = j.nbn[b] + (has_self(d, b) ? 1 : 0);
-            tc = (g1 - g0) * per;
+            for (int g = g0; g < g1; g++) tc += task_pieces(d.bd_e0[g + 1] - d.bd_e0[g]);
+            tc *= per;
             sc = (d.bd_e0[g1] - d.bd_e0[g0]) * per;
         }
         int tt, st;
