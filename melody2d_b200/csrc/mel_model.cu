@@ -850,6 +850,7 @@ static mel_status build(mel_handle* h, const mel_model_desc* d, const mel_option
     P.ncand = dalloc<int>(h, 1);
     P.bslot0 = dalloc<int>(h, nb + 2);
     P.b_cont0 = dalloc<int>(h, nb + 1);
+    P.e_head = dalloc<unsigned long long>(h, ne);
     size_t cb = sizeof(mel_contact) * 1024;
     if (cudaMalloc(&D.cont, cb) != cudaSuccess) return MEL_ERR_OOM;
     P.cont_bytes = cb;
@@ -1266,7 +1267,7 @@ mel_status mel_destroy(mel_handle* h)
     for (void* p : h->allocs) cudaFree(p);
     mel_prox_state& P = h->P;
     for (void* p : { (void*)P.nbr, (void*)P.cand, (void*)P.tcand, (void*)P.toff, (void*)P.tkey, (void*)P.bucket, (void*)P.inc_task,
-                     (void*)P.inc_rng, (void*)P.scan_ws, (void*)P.cont_alt, (void*)P.cont_w, (void*)P.cont_rt, (void*)h->d.cont })
+                     (void*)P.inc_rng, (void*)P.c_next, (void*)P.scan_ws, (void*)P.cont_alt, (void*)P.cont_w, (void*)P.cont_rt, (void*)h->d.cont })
         if (p) cudaFree(p);
     mel_prox_stage_free(P.stage);
     if (h->ck.side) { cudaStreamSynchronize(h->ck.side); cudaStreamDestroy(h->ck.side); }

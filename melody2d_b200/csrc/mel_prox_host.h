@@ -24,6 +24,9 @@ struct mel_prox_state {
     int* inc_cnt = nullptr;                                 // per master body
     int2* inc_rng = nullptr; size_t inc_rng_bytes = 0;
     int* b_inc0 = nullptr; int* b_cont0 = nullptr;
+    unsigned long long* e_head = nullptr;                   // per border entry: its chain of old contacts (LONG_LIST)
+    int* c_next = nullptr; size_t c_next_bytes = 0;
+    unsigned stamp = 0;                                     // of the run that made the chains
     size_t cont_bytes = 0;
     mel_contact* cont_alt = nullptr; size_t cont_alt_bytes = 0;
     double* cont_w = nullptr; size_t cont_w_bytes = 0;
@@ -56,6 +59,7 @@ struct mel_prox_job {
     int *tcand, *toff, *tkey, *bucket, *inc_task, *inc_cnt; int tcand_n;
     int2* inc_rng; int* b_inc0; int* b_cont0;
     mel_contact* cont_new;        // the list being written (write stage)
+    unsigned long long* e_head; int* c_next; unsigned stamp; int link;
     int* readback;                // this member's words of the run's read-back array (host memory)
     int cl_on, cl_T, cl_ncx;      // cell-list broad phase (mel_prox_state)
     double cl_h, cl_hx;

@@ -24,3 +24,30 @@ def test_contact_lists(gpu_lib, oracle_built, n, superblocks):
     assert_contacts_equal(s.contacts(), o.contacts())
     assert (s.contacts()["fx"] != 0).sum() > n
     s.close()
+
+
+@pytest.mark.parametrize("n", [40, 126, 127, 128, 252, 254, 256, 900])
+def test_history_of_long_lists(gpu_lib, oracle_built, n):
+    """Lists handed in by the caller, each contact twice with different history and in any order within its
+    slave body: on both sides of 256 elements a body, an update inherits from the first in the list."""
+    from melody2d_b200.solver import Solver
+    from oracle.pyoracle import Oracle
+    flat = blocks_flat(n)
+    s = Solver.from_flat(flat)
+    o = Oracle(flat, correctly_rounded=True)
+    c = s.contacts()
+    rng = np.random.default_rng(n)
+    twice = np.concatenate([c, c])
+    twice["gapt"] = rng.standard_normal(len(twice))
+    twice["vgapt"] = rng.standard_normal(len(twice))
+    twice = twice[np.lexsort((rng.random(len(twice)), twice["bodyS"]))]
+    for x in (s, o):
+        x.set_contacts(twice)
+        x.update_proximity()
+    assert_contacts_equal(s.contacts(), o.contacts())
+    assert len(np.unique(s.contacts()["gapt"])) > n // 2
+    # and from the list that this left
+    for x in (s, o):
+        x.step(11)
+    assert_contacts_equal(s.contacts(), o.contacts())
+    s.close()
