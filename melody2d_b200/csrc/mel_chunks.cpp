@@ -294,3 +294,14 @@ mel_status mel_build_chunks(const mel_model_desc* d, int ecap, mel_chunk_set& ou
     out.b_chunk0[nb] = (int)out.chunks.size();
     return MEL_OK;
 }
+
+mel_status mel_build_wide_chunks(const mel_model_desc* d, size_t room, mel_chunk_set& out, bool mixed)
+{
+    for (int ecap : { MEL_CHUNK_E_MAX(mixed), 3072, 2560, 2048, 1792, 1536, 1280, 1024, 768, 512, 256 }) {
+        if (ecap > MEL_CHUNK_E_MAX(mixed)) continue;
+        const mel_status rc = mel_build_chunks(d, ecap, out, mixed, 0, MEL_MAX_BODY_NODES);
+        if (rc) return rc;
+        if (MEL_BAR_BYTES + 2 * (size_t)out.img_max <= room) break;
+    }
+    return MEL_OK;
+}

@@ -21,3 +21,6 @@ struct mel_chunk_set {
 // error code with the message set.
 mel_status mel_build_chunks(const mel_model_desc* d, int ecap, mel_chunk_set& out, bool mixed = false, long long = 0,
                             int min_nodes = 0);
+// The images of the bodies above MEL_MAX_BODY_NODES nodes, with the most entries a chunk (up to
+// MEL_CHUNK_E_MAX) whose two buffers and mbarriers take at most `room` bytes of shared memory.
+mel_status mel_build_wide_chunks(const mel_model_desc* d, size_t room, mel_chunk_set& out, bool mixed);

@@ -771,13 +771,9 @@ static mel_status build(mel_handle* h, const mel_model_desc* d, const mel_option
         D.tile_pad = (unsigned long long)TS.cap * 0x0001000100010001ull;
     }
     if (any_wide) {
-        // chunk images of the wide bodies: the largest entry cap whose two buffers leave room for two
-        // CTAs per SM (FP32 images hold 12 bytes an entry instead of 20)
-        for (int ecap : { MEL_CHUNK_E_MAX, 1792, 1536, 1280, 1024, 768, 512, 256 }) {
-            mel_status rc = mel_build_chunks(d, ecap, CS, mixed, 0, MEL_MAX_BODY_NODES);
-            if (rc) return rc;
-            if (MEL_BAR_BYTES + 2 * (size_t)CS.img_max <= two_per_sm + sizeof(mel_dev)) break;    // (not in batches)
-        }
+        // chunk images of the wide bodies, which leave room for two CTAs per SM (they are not in batches)
+        mel_status rc = mel_build_wide_chunks(d, two_per_sm + sizeof(mel_dev), CS, mixed);
+        if (rc) return rc;
         h->body_smem = std::max(h->body_smem, MEL_BAR_BYTES + 2 * (size_t)CS.img_max);
     }
     h->nge = (int)(TS.n_entries + CS.n_entries);
