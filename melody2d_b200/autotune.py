@@ -57,10 +57,10 @@ def tune(out: str, discs: int, steps: int, workers: int) -> dict:
                            "body_ms": {str(k): round(v, 5) for k, v in times.items()}, "generate_s": round(gen_s, 1)})
             print(json.dumps(report[-1]), flush=True)
     with open(out, "w") as fh:
-        fh.write("# slots per tile (precision 0 fp64 / 1 mixed, largest deformable body in nodes), written by\n"
+        fh.write("# \"tile\", precision (0 fp64 / 1 mixed), largest deformable body in nodes, slots per tile; written by\n"
                  "# python -m melody2d_b200.autotune (body-kernel time on a %d-disc sample of each class)\n" % discs)
         for p, n, c in rows:
-            fh.write("%d %d %d\n" % (p, n, c))
+            fh.write("tile %d %d %d\n" % (p, n, c))
     return {"table": out, "classes": report}
 
 

@@ -250,10 +250,11 @@ static mel_status validate(const mel_model_desc* d)
     return MEL_OK;
 }
 
-// Chunk entry cap for a model of this precision whose largest deformable body has max_nodes
+// Slots per tile for a model of this precision whose largest deformable body has max_nodes
 // nodes: MELGPU_CHUNK_CAP if set, else the first line of the tuning table (the file named by
-// MELGPU_TUNE_FILE; lines "precision max_body_nodes cap", '#' comments) whose precision matches and
-// whose node bound covers max_nodes; 0 when neither applies.
+// MELGPU_TUNE_FILE; lines "tile precision max_body_nodes slots", '#' comments) whose precision matches
+// and whose node bound covers max_nodes; 0 when neither applies.  Lines of three numbers, as earlier
+// tables have them, count another thing, the entries of a chunk, and are passed over.
 static int tuned_chunk_cap(int precision, int max_nodes)
 {
     if (const char* c = getenv("MELGPU_CHUNK_CAP")) {
@@ -267,9 +268,8 @@ static int tuned_chunk_cap(int precision, int max_nodes)
     char line[256];
     int cap = 0;
     while (fgets(line, sizeof line, f)) {
-        if (line[0] == '#') continue;
         int p = -1, mn = 0, c = 0;
-        if (sscanf(line, "%d %d %d", &p, &mn, &c) == 3 && p == precision && max_nodes <= mn && c >= 64 && c <= MEL_TILE_SLOTS_MAX) {
+        if (sscanf(line, "tile %d %d %d", &p, &mn, &c) == 3 && p == precision && max_nodes <= mn && c >= 64 && c <= MEL_TILE_SLOTS_MAX) {
             cap = (c + 127) & ~127;
             break;
         }

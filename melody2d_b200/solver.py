@@ -111,7 +111,7 @@ def lib():
     if _lib is None:
         if not os.path.exists(LIB_PATH):
             raise RuntimeError(f"{LIB_PATH} is missing: build it with `python -m melody2d_b200.build`")
-        # the chunk-size tuning table written by melody2d_b200.autotune, unless the caller names one
+        # the tile-size tuning table written by melody2d_b200.autotune, unless the caller names one
         table = os.path.join(_HERE, "tuning.txt")
         if "MELGPU_TUNE_FILE" not in os.environ and os.path.exists(table):
             os.environ["MELGPU_TUNE_FILE"] = table
@@ -372,7 +372,7 @@ class Solver:
                     n_deformable_nodes=n[0].value, n_contacts=n[1].value)
 
     def kernel_config(self) -> dict:
-        """Body-kernel launch configuration: chunk entry cap, shared memory per CTA, CTAs."""
+        """Body-kernel launch configuration: slots per tile (chunk_cap), shared memory per CTA, CTAs."""
         cap, ctas = C.c_int(), C.c_int()
         smem = C.c_longlong()
         _check(lib().mel_get_kernel_config(self.h, C.byref(cap), C.byref(smem), C.byref(ctas)))
