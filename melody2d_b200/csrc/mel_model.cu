@@ -734,7 +734,9 @@ static mel_status build(mel_handle* h, const mel_model_desc* d, const mel_option
     cudaDeviceGetAttribute(&smem_sm, cudaDevAttrMaxSharedMemoryPerMultiprocessor, h->device);
     cudaDeviceGetAttribute(&smem_blk, cudaDevAttrMaxSharedMemoryPerBlockOptin, h->device);
     cudaDeviceGetAttribute(&smem_res, cudaDevAttrReservedSharedMemoryPerBlock, h->device);
-    // (a batch's CTAs hold a member's descriptor beside it)
+    // room of a body CTA when one or two share an SM (a batch's CTAs hold a member's descriptor beside it, and
+    // a model must fit them too: it may join a batch any time)
+    const size_t one_per_sm = (size_t)smem_blk - sizeof(mel_dev);
     const size_t two_per_sm = (size_t)(smem_sm / 2 - smem_res) - sizeof(mel_dev);
     const bool mixed = h->precision == MEL_PREC_MIXED;
     {
@@ -750,15 +752,15 @@ static mel_status build(mel_handle* h, const mel_model_desc* d, const mel_option
         mel_status rc = MEL_OK;
         int cap = tuned_chunk_cap(h->precision, max_def_nodes);
         if (cap > 0 && (rc = plan(std::max(cap, least))) != MEL_OK) return rc;
-        if (cap == 0 || need() > (size_t)smem_blk)
-            for (size_t room : { two_per_sm, (size_t)smem_blk }) {
+        if (cap == 0 || need() > one_per_sm)
+            for (size_t room : { two_per_sm, one_per_sm }) {
                 for (cap = std::max(MEL_TILE_SLOTS, least); ; cap = std::max(cap - 256, least)) {
                     if ((rc = plan(cap)) != MEL_OK) return rc;
                     if (need() <= room || cap == least) break;
                 }
                 if (need() <= room) break;
             }
-        if (need() > (size_t)smem_blk) {
+        if (need() > one_per_sm) {
             mel_set_error("deformable body of %d nodes does not fit the body kernel's shared memory", max_def_nodes);
             return MEL_ERR_UNSUPPORTED;
         }
