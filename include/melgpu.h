@@ -445,7 +445,7 @@ mel_status  mel_get_kernel_times(mel_handle* h, double* ms_contact, double* ms_b
  * sizes of the resident layout), deformable node count and current contact count. */
 mel_status  mel_get_step_stats(mel_handle* h, double* ms_total, double* bytes_body, double* bytes_contact,
                                int* n_deformable_nodes, int* n_contacts);
-/* Launch configuration of the body kernel chosen at mel_create: support entries per chunk image,
+/* Launch configuration of the body kernel chosen at mel_create: slots per Gauss-point tile,
  * dynamic shared memory per CTA (bytes) and CTAs per launch (one per body). */
 mel_status  mel_get_kernel_config(mel_handle* h, int* chunk_cap, long long* body_smem, int* body_ctas);
 /* Sizes of the resident model. */

@@ -33,7 +33,9 @@
 #define MEL_WAIT_NS 1000000000u   // bound of every device-side wait (1 s)
 #define MEL_WAIT_NOT 1u           // a wait with this bound gives up without a look (tests)
 #define MEL_NBR_CAP_DEFAULT 64    // neighbour slots per body (grown on overflow)
-#define MEL_MAX_BODY_NODES 4096   // nodes per deformable body held in shared memory
+// largest deformable body that keeps its node arrays in shared memory.  What a CTA has room for is less (176 or
+// 184 bytes a node): 1,313 nodes in FP64, 1,256 in the mixed form; larger ones up to here are refused
+#define MEL_MAX_BODY_NODES 4096
 #define MEL_MAX_WIDE_NODES 65535  // larger bodies keep their node arrays in global memory (16-bit indices)
 // bytes of a wide body's node arrays in global memory (mel_dev::gscr): s_f, s_fc, s_upf, then the
 // post-loop arrays s_fn, s_fd, s_vp, s_ap, the six work terms and the temporary parameters

@@ -4,7 +4,8 @@
 // A tile is up to MEL_TILE_GP consecutive points, sorted by (support count descending, index) into
 // groups of up to 32, one warp each.  The pass keeps a point's first derivative pairs in registers,
 // loaded straight from global memory, and holds in shared memory the points' contributions, one slot
-// an entry, and what bulk copies bring: the other pairs (an eighth of them) and the indices.  Sections of a tile (byte offsets from mel_tile::base, each 16-byte aligned):
+// an entry, and what bulk copies bring: the other pairs (about half of them in FP64, a quarter in the
+// mixed form) and the indices.  Sections of a tile (byte offsets from mel_tile::base, each 16-byte aligned):
 //   head    pairs dN/dx, dN/dy of the rows k < MEL_TILE_HEAD, read straight into registers: entry k of
 //           lane l of a group at h0 + k w + l, h0 the pairs of the groups before and w the group's
 //           width (its points rounded up to the slots of one shared-memory wavefront).  FP64 pairs;

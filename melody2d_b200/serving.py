@@ -82,8 +82,9 @@ def _build(seed: int):
 
 
 def estimate_device_bytes(flat: dict) -> float:
-    """Device memory of a solver created from `flat`: its arrays plus the chunk images, contact and
-    proximity buffers (about 1.6x the description's arrays for these samples)."""
+    """Device memory of a solver created from `flat`: its arrays plus the Gauss-point
+    tiles, contact and proximity buffers (1.6x the description's arrays, more than these samples take: a sample
+    of 1800 grains takes 1,911 MB in FP64, 1,424 MB mixed, where this gives 3,098)."""
     host = sum(np.asarray(v).nbytes for k, v in flat.items() if k != "material_names")
     return 1.6 * host
 
